@@ -129,10 +129,11 @@ def _experts(E, n, k, quant, gen):
     return q, torch.stack(scales)
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """Activations, quantised weights in row-major order and router logits, from the seed alone."""
     gen = torch.Generator(device="cuda").manual_seed(seed)
     kind = case["kind"]
-    state = dict(case)
+    d = {}
 
     def normal(*shape):
         return torch.randn(*shape, generator=gen, device="cuda")
@@ -140,47 +141,57 @@ def prepare(case, seed):
     if kind in ("dense", "pertoken"):
         M, N, K = case["M"], case["N"], case["K"]
         w = normal(N, K) * 0.02
-        x = normal(M, K).to(torch.bfloat16)
-        shape = dict(M=M, N=N, K=K, tile_m=64, tile_n=128, tile_k=128, out_dtype=case["out"])
-        if kind == "dense":
-            q, state["w_scale"] = _block_quant(w)
-            state["gemm"] = compile_blockscale_preshuffle_gemm(**shape)
-        else:
-            q, state["w_scale"] = _channel_quant(w)
-            state["gemm"] = compile_preshuffle_gemm_a8(**shape)
-        state["w"] = shuffle_weight(q.contiguous())
-        state["c"] = torch.empty((M, N), dtype=DTYPES[case["out"]], device="cuda")
-        if case["quantise"]:
-            state["x"] = x
-        else:
-            state["x_q"], state["x_scale"] = (quant_1x128 if kind == "dense" else quant_pertoken)(x)
-        return state
+        d["x"] = normal(M, K).to(torch.bfloat16)
+        d["w"], d["w_scale"] = (_block_quant if kind == "dense" else _channel_quant)(w)
+        return d
     if kind == "int4":
         M, N, K = case["M"], case["N"], case["K"]
         g = (normal(N, K) * 0.02).view(N, K // 128, 128)
         s = (g.abs().amax(dim=-1) / 7.0).to(torch.bfloat16)
         s[s == 0] = 1
-        q = torch.round(g / s.float().unsqueeze(-1)).clamp_(-8, 7).to(torch.int8).view(N, K)
-        state["w"], state["w_scale"] = pack_int4_weight(q, s)
-        state["gemm"] = compile_int4_weight_only_gemm(N=N, K=K)
-        state["x"] = normal(M, K).to(torch.bfloat16)
-        state["c"] = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
-        return state
+        d["w"] = torch.round(g / s.float().unsqueeze(-1)).clamp_(-8, 7).to(torch.int8).view(N, K)
+        d["w_scale"] = s
+        d["x"] = normal(M, K).to(torch.bfloat16)
+        return d
     T, H, I, E = case["T"], case["H"], case["I"], case["E"]
     quant = _block_quant if kind == "moe" else _channel_quant
-    w1, w1_scale = _experts(E, 2 * I, H, quant, gen)
-    w1 = shuffle_weight(w1)
-    w2, w2_scale = _experts(E, H, I, quant, gen)
-    w2 = shuffle_weight(w2)
+    d["w1"], d["w1_scale"] = _experts(E, 2 * I, H, quant, gen)
+    d["w2"], d["w2_scale"] = _experts(E, H, I, quant, gen)
+    d["x"] = normal(T, H).to(torch.bfloat16)
+    d["logits"] = normal(T, E)
+    d["logits"][:, :case["hot"]] += 2.0
+    return d
+
+
+def prepare(case, seed):
+    kind = case["kind"]
+    d = _inputs(case, seed)
+    state = {**case, **d}
+    if kind in ("dense", "pertoken"):
+        M, N, K = case["M"], case["N"], case["K"]
+        shape = dict(M=M, N=N, K=K, tile_m=64, tile_n=128, tile_k=128, out_dtype=case["out"])
+        compile_gemm = compile_blockscale_preshuffle_gemm if kind == "dense" else compile_preshuffle_gemm_a8
+        state["gemm"] = compile_gemm(**shape)
+        state["w"] = shuffle_weight(d["w"].contiguous())
+        state["c"] = torch.empty((M, N), dtype=DTYPES[case["out"]], device="cuda")
+        if not case["quantise"]:
+            state["x_q"], state["x_scale"] = (quant_1x128 if kind == "dense" else quant_pertoken)(state.pop("x"))
+        return state
+    if kind == "int4":
+        M, N, K = case["M"], case["N"], case["K"]
+        state["w"], state["w_scale"] = pack_int4_weight(d["w"], d["w_scale"])
+        state["gemm"] = compile_int4_weight_only_gemm(N=N, K=K)
+        state["c"] = torch.empty((M, N), dtype=torch.bfloat16, device="cuda")
+        return state
+    for name in ("w1", "w2"):
+        d[name] = None
+        state[name] = shuffle_weight(state[name])
+    weights = [state.pop(name) for name in ("w1", "w1_scale", "w2", "w2_scale")]
     if kind == "moe":
-        state["layer"] = BlockscaleMoE(w1, w1_scale, w2, w2_scale, topk=case["topk"], tile_m=_tile_m(T),
-                                       mode=case["mode"])
+        state["layer"] = BlockscaleMoE(*weights, topk=case["topk"], tile_m=_tile_m(case["T"]), mode=case["mode"])
     else:
-        state["layer"] = PertokenMoE(w1, w1_scale, w2, w2_scale, topk=case["topk"], tile_m=_tile_m(T))
-    state["x"] = normal(T, H).to(torch.bfloat16)
-    state["logits"] = normal(T, E)
-    state["logits"][:, :case["hot"]] += 2.0
-    state["out"] = torch.empty((T, H), dtype=torch.bfloat16, device="cuda")
+        state["layer"] = PertokenMoE(*weights, topk=case["topk"], tile_m=_tile_m(case["T"]))
+    state["out"] = torch.empty((case["T"], case["H"]), dtype=torch.bfloat16, device="cuda")
     return state
 
 
@@ -239,3 +250,51 @@ def tolerance(case):
     if case["kind"] in ("moe", "ptmoe"):
         return {"rel": 2e-2, "max": 0.2} if case.get("mode") == "atomic" else {"rel": 1e-2, "max": 0.17}
     return {"rel": 8.5e-4, "max": 2e-3} if case.get("out") == "fp16" else {"rel": 6.6e-3, "max": 1.6e-2}
+
+
+def _quantised(x, group, dtype=torch.float64):
+    """The values, in 64 bits, that rows quantised in groups of ``group`` stand for; scale and code
+    are computed in ``dtype``, by division (torch multiplies by the reciprocal of a Python number,
+    which moves values that lie halfway between two codes)."""
+    g = x.to(dtype).view(x.shape[0], -1, group)
+    s = g.abs().amax(dim=-1, keepdim=True)
+    s = s / torch.full_like(s, 448.0)
+    s[s == 0] = 1
+    return ((g / s).to(FP8).double() * s.double()).view(x.shape)
+
+
+def _weight(w, scale, kind):
+    """The values, in 64 bits, that one quantised weight ``[N, K]`` stands for."""
+    n, k = w.shape
+    if kind in ("pertoken", "ptmoe"):
+        return w.double() * scale.double().view(n, 1)
+    s = scale.double().view(-1, k // 128).repeat_interleave(128, dim=0)[:n]
+    return (w.double().view(n, -1, 128) * s.unsqueeze(-1)).view(n, k)
+
+
+def exact(case, seed):
+    """``run``'s results by dequantised products in 64 bits. What a layer's formats define stays: the
+    fp8 codes and 32-bit scales of its activations, and the fp8 grid of its intermediate."""
+    kind = case["kind"]
+    d = _inputs(case, seed)
+    x = d["x"]
+    if kind == "int4":
+        n, k = d["w"].shape
+        w = (d["w"].double().view(n, -1, 128) * d["w_scale"].double().unsqueeze(-1)).view(n, k)
+        return x.double() @ w.t()
+    x = _quantised(x, 128 if kind in ("dense", "moe") else x.shape[1], torch.float32)
+    if kind in ("dense", "pertoken"):
+        return x @ _weight(d["w"], d["w_scale"], kind).t()
+    I = case["I"]
+    values, ids = torch.topk(d["logits"], case["topk"], dim=-1)
+    weights = torch.softmax(values.double(), dim=-1)
+    out = torch.zeros_like(x)
+    for e in range(case["E"]):
+        token, slot = (ids == e).nonzero(as_tuple=True)
+        if token.numel() == 0:
+            continue
+        y = x[token] @ _weight(d["w1"][e], d["w1_scale"][e], kind).t()
+        act = _quantised(torch.nn.functional.silu(y[:, :I]) * y[:, I:], 128 if kind == "moe" else I)
+        y = act @ _weight(d["w2"][e], d["w2_scale"][e], kind).t()
+        out.index_add_(0, token, y * weights[token, slot].unsqueeze(-1))
+    return out
