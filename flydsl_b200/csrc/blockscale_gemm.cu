@@ -409,12 +409,20 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           }
         }
       }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1) {
       // ---------------- MMA issuer ----------------
-      // One thread issues every MMA of the CTA. (Per K block it spends ~60-100 cycles in each barrier
-      // wait, ~64 per tcgen05.mma and ~50-100 in the commit, less than the 512 cycles the tensor core
-      // needs; a second issuing thread taking alternate K blocks was measured to change nothing,
-      // the epilogue being the slower side.)
+      // One elected lane issues every MMA of the CTA; the whole warp runs the loop, which keeps the
+      // descriptors in uniform registers.
+      const bool leader = elect_one();
+      const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+      // operands of the stage and the accumulator buffer, asked for together (a query costs about a
+      // hundred cycles, and normally both are ready); the whole warp observes both
+      auto wait_both = [&](uint32_t full, uint32_t fph, uint32_t empty, uint32_t eph) -> bool {
+        if (__all_sync(0xffffffffu, mbar_test_both(full, fph, empty, eph))) return true;
+        const bool ok = mbar_wait(full, fph, abort_flag, p.err, kErrWaitSmemFull) &&
+                        mbar_wait(empty, eph, abort_flag, p.err, kErrWaitTmemEmpty);
+        return __all_sync(0xffffffffu, ok);
+      };
       constexpr uint32_t idesc = umma_idesc_e4m3_f32(BM, BN);
       uint32_t it = 0;
       uint32_t tiles_issued = 0;   // kDensePT
@@ -428,29 +436,35 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           // one accumulator buffer per TILE: wait for it once, accumulate every K block into it,
           // then tell the epilogue; the per-K-block commits only hand the stages back
           const int buf = static_cast<int>(tiles_issued % kAccBufs);
-          if (!mbar_wait(tempty_bar(buf), ((tiles_issued / kAccBufs) & 1) ^ 1, abort_flag, p.err,
-                         kErrWaitTmemEmpty)) {
+          const bool free_ok = mbar_wait(tempty_bar(buf), ((tiles_issued / kAccBufs) & 1) ^ 1, abort_flag, p.err,
+                                         kErrWaitTmemEmpty);
+          if (!__all_sync(0xffffffffu, free_ok)) {
             alive = false;
             break;
           }
-          const uint32_t d = tmem_base + buf * BN;
+          const uint32_t d = tmem_u + buf * BN;
           for (int kb = 0; kb < KB; ++kb, ++it) {
             const int s = it % kStages;
             const uint32_t sa = smem_base + s * C::kStageBytes;
             const uint64_t adesc = umma_desc_sw128(sa);
             const uint64_t bdesc = umma_desc_sw128(sa + kATileBytes);
-            if (!mbar_wait(full_bar(s), (it / kStages) & 1, abort_flag, p.err, kErrWaitSmemFull)) {
+            const bool full_ok = mbar_wait(full_bar(s), (it / kStages) & 1, abort_flag, p.err, kErrWaitSmemFull);
+            if (!__all_sync(0xffffffffu, full_ok)) {
               alive = false;
               break;
             }
             tc_fence_after();
+            if (leader) {
 #pragma unroll
-            for (int k = 0; k < BK / 32; ++k)
-              tc_mma_f8(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) ? 1u : 0u);
-            tc_commit(done_bar(it % kDone));
+              for (int k = 0; k < BK / 32; ++k)
+                tc_mma_f8(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) ? 1u : 0u);
+              tc_commit(done_bar(it % kDone));
+            }
+            __syncwarp();
           }
           if (!alive) break;
-          tc_commit(tfull_bar(buf));
+          if (leader) tc_commit(tfull_bar(buf));
+          __syncwarp();
           ++tiles_issued;
           continue;
         }
@@ -462,20 +476,22 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const uint32_t sa = smem_base + s * C::kStageBytes;
           const uint64_t adesc = umma_desc_sw128(sa);
           const uint64_t bdesc = umma_desc_sw128(sa + kATileBytes);
-          const uint32_t d = tmem_base + buf * BN;
+          const uint32_t d = tmem_u + buf * BN;
           // The operands normally landed long ago; the accumulator buffer is what the issuer really
           // waits for, so that wait comes last and nothing but the fence separates it from the MMAs.
-          if (!mbar_wait(full_bar(s), ph, abort_flag, p.err, kErrWaitSmemFull) ||
-              !mbar_wait(tempty_bar(buf), tph ^ 1, abort_flag, p.err, kErrWaitTmemEmpty)) {
+          if (!wait_both(full_bar(s), ph, tempty_bar(buf), tph ^ 1)) {
             alive = false;
             break;
           }
           tc_fence_after();
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < BK / 32; ++k)
-            tc_mma_f8(d, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
-          // the MMAs of the K block are done: partial sums in TMEM, operands consumed
-          tc_commit(done_bar(it % kDone));
+            for (int k = 0; k < BK / 32; ++k)
+              tc_mma_f8(d, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
+            // the MMAs of the K block are done: partial sums in TMEM, operands consumed
+            tc_commit(done_bar(it % kDone));
+          }
+          __syncwarp();
         }
       }
     } else if (is_dense(MODE) && C::kStaged && warp == 2 && lane == 0) {
@@ -796,7 +812,11 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
     // Scales are prefetched kRing K blocks ahead into a register ring; the ring of the NEXT tile is
     // loaded before the current tile's store phase so that its latency hides behind the stores.
-    constexpr int kRing = 2;
+    //
+    // Distance: at least a cold (HBM) latency, ~1 us. A 256-wide tile's K block takes ~0.5 us; the
+    // narrower ones take 0.25-0.28 us and have registers to spare (same shape, two -> four K blocks at
+    // 64 columns: 21 -> 18.8 us, two -> eight at 128 columns: 22.7 -> 21.2 us).
+    constexpr int kRing = BN == 256 ? 2 : BN == 128 ? 8 : 4;
     ScaleCtx cur;
     float ring_a[kRing], ring_b0[kRing], ring_b1[kRing];
     TilePos pos = walk.start();
@@ -860,6 +880,11 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             const int buf = it % kAccBufs;
             const float s0 = ring_a[j] * ring_b0[j];
             const float s1 = ring_a[j] * ring_b1[j];
+            // Both products exist before the ring slots are loaded again. Left to itself the compiler
+            // forms them where they are used, loads into other registers and moves the values over at
+            // the end of the trip, which waits there for loads issued in this very trip: a memory
+            // latency in every K block (M = 256, N = 4096, K = 7168, 64-wide tiles: 28.6 -> 21 us).
+            asm volatile("" ::"f"(s0), "f"(s1));
             if (kb + kRing < KB) {
               ring_a[j] = __ldg(pf_a);
               ring_b0[j] = __ldg(pf_b0);

@@ -73,6 +73,37 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
+// Both phases complete? Never suspends; the two queries are in flight together.
+__device__ __forceinline__ bool mbar_test_both(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+      "and.pred p, p, q;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok)
+      : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1)
+      : "memory");
+  return ok != 0;
+}
+// One lane of a converged warp. Code that a whole warp runs and only the elected lane's tcgen05
+// instructions leave keeps their operands in uniform registers; the same code under `lane == 0` does
+// not, and every instruction then pays for moving them.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}"
+      : "=r"(ok));
+  return ok != 0;
+}
+
 // Every wait in these kernels is bounded. A role that runs out of patience raises the CTA-wide
 // abort flag (shared memory) and records why in the device error word; every other role sees the
 // flag on its next wait and leaves its loop, so the CTA reaches its teardown (TMEM release) and the
