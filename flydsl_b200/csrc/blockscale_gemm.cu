@@ -23,6 +23,7 @@
 // kernels/moe_blockscale_2stage.py (:206-1161, :1386-2387); none of its AMD data movement is kept.
 #include <cuda_fp8.h>
 
+#include "cluster.cuh"
 #include "common.cuh"
 
 namespace flyb200 {
@@ -84,13 +85,16 @@ struct GemmParams {
   // output): fp8 rows [a_rows, N] and their scales [N/128, a_rows] instead of the 16-bit `out`.
   uint8_t* out_q;
   float* out_scale_t;
+  // Split-K (kSplit kernels, dense modes): CTAs of a cluster that share a tile, K blocks of each
+  int splits;
+  int kbps;
 };
 
-template <int BN, int MODE, typename OutT>
+template <int BN, int MODE, typename OutT, bool SPLIT = false>
 struct Cfg {
   static constexpr int kOutCols = (is_moe1(MODE)) ? BN / 2 : BN;   // output columns per tile
   // 16-bit outputs of tiles at least 64 wide go through a shared-memory staging tile.
-  static constexpr bool kStaged = (sizeof(OutT) == 2) && (kOutCols >= 32) && (BN >= 64);
+  static constexpr bool kStaged = (sizeof(OutT) == 2) && (kOutCols >= 32) && (BN >= 64) && !SPLIT;
   static constexpr int kRegions = (kOutCols + 63) / 64;
   // The per-token mode is bound by its operand feed, and its epilogue has a whole tile's K loop to
   // get the previous tile out: it stages and stores a tile in two halves of 128 columns, which leaves
@@ -110,7 +114,14 @@ struct Cfg {
   static constexpr int kAccBufs = (512 / BN) > 8 ? 8 : (512 / BN);
   static constexpr int kTmemCols = BN * kAccBufs;
   static constexpr int kCH = BN / 4;  // columns per epilogue thread per column group
-  static constexpr int kSmemBytes = kStages * kStageBytes + kCBytes + kMiscBytes + 1024;
+  // Split-K: no staging tile. The exchange lies over the ring: this CTA's partial tile (fp32, BM rows)
+  // and behind it one slice of rows from every other CTA of the cluster; kSplitMax CTAs fit.
+  static constexpr int kSplitMax = BN == 256 ? 4 : 8;
+  __host__ __device__ static constexpr int split_rows(int rows, int splits) { return (rows + splits - 1) / splits; }
+  static_assert(!SPLIT || BM * BN * 4 + (kSplitMax - 1) * split_rows(BM, kSplitMax) * BN * 4 <= kAvail,
+                "split-K exchange does not fit");
+  static constexpr int kRingBytes = SPLIT ? kAvail : kStages * kStageBytes;
+  static constexpr int kSmemBytes = kRingBytes + kCBytes + kMiscBytes + 1024;
   static_assert(kStages >= 3, "pipeline too shallow");
 };
 
@@ -175,10 +186,11 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 struct TilePos {
   int tile, m_blk, n_tile;
 };
-template <int BN, int MODE>
+template <int BN, int MODE, bool SPLIT = false>
 struct TileWalker {
   int num_m, num_n, total;
   int step_major, step_minor;  // gridDim.x split by the minor dimension's extent
+  int p_splits;                // split-K: consecutive CTAs of one tile
   // Dense with many row blocks: they are taken in groups of group_m; inside a group the order is the
   // usual one (row blocks fastest, then column tiles), so a group's slice of A (group_m x 128 x K
   // bytes) stays in L2 while all column tiles pass over it, instead of the whole of A streaming
@@ -193,6 +205,7 @@ struct TileWalker {
   static constexpr bool kRowBlockMajor = (!is_dense(MODE));
   __device__ __forceinline__ TileWalker(const GemmParams& p) {
     group_m = 0;
+    p_splits = SPLIT ? p.splits : 1;
     if constexpr (is_dense(MODE)) {
       num_m = (p.M + BM - 1) / BM;
       num_n = (p.N + BN - 1) / BN;
@@ -206,6 +219,7 @@ struct TileWalker {
       num_n = (p.N + kColsPerTile - 1) / kColsPerTile;
     }
     total = num_m * num_n;
+    if constexpr (SPLIT) group_m = 0;   // one tile per cluster
     const int minor = kRowBlockMajor ? num_n : num_m;
     const int g = static_cast<int>(gridDim.x);
     step_major = minor > 0 ? g / minor : 0;
@@ -223,6 +237,7 @@ struct TileWalker {
   __device__ __forceinline__ TilePos start() const {
     TilePos t;
     t.tile = static_cast<int>(blockIdx.x);
+    if constexpr (SPLIT) t.tile /= p_splits;
     if (is_dense(MODE) && group_m > 0) {
       if (t.tile < total) decode_grouped(t);
       else t.m_blk = t.n_tile = 0;
@@ -254,11 +269,16 @@ struct TileWalker {
   }
 };
 
-template <int BN, int MODE, typename OutT>
+// SPLIT (dense modes): the CTAs of a cluster share one tile, each takes a range of its K blocks, and
+// the fp32 partial tiles are added through distributed shared memory (see the end of the epilogue).
+// For problems with far fewer tiles than SMs and a long K, which are one serial chain of K blocks per
+// tile otherwise: M = 256, N = 4096, K = 7168 has 64 tiles of 128 columns and 56 K blocks each.
+template <int BN, int MODE, typename OutT, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_c,
                const GemmParams p) {
-  using C = Cfg<BN, MODE, OutT>;
+  static_assert(!SPLIT || is_dense(MODE), "split-K is built for the dense modes");
+  using C = Cfg<BN, MODE, OutT, SPLIT>;
   constexpr int kStages = C::kStages;
   constexpr int CH = C::kCH;
   extern __shared__ uint8_t smem_raw[];
@@ -268,9 +288,9 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_al = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t cstage_base = smem_base + kStages * C::kStageBytes;       // 1024-aligned
+  const uint32_t cstage_base = smem_base + C::kRingBytes;       // 1024-aligned
   const uint32_t misc_base = cstage_base + C::kCBytes;
-  uint8_t* misc = smem_al + kStages * C::kStageBytes + C::kCBytes;
+  uint8_t* misc = smem_al + C::kRingBytes + C::kCBytes;
   long long* row_off = reinterpret_cast<long long*>(misc);                 // [128], MoE staged output
   const uint32_t bar_base = misc_base + 1024;
   // Barriers. full[s]: operands of stage s have landed. done[i]: the MMAs of K-block iteration i
@@ -287,8 +307,9 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   auto done_bar = [&](uint32_t i) { return bar_base + 8u * (kStages + i); };
   auto tempty_bar = [&](int b) { return bar_base + 8u * (kStages + kDone + b); };
   auto tfull_bar = [&](int b) { return bar_base + 8u * (kStages + kDone + kAccBufs + b); };   // kDensePT
-  constexpr int kNumBars = kStages + kDone + 2 * kAccBufs + 3;
+  constexpr int kNumBars = kStages + kDone + 2 * kAccBufs + 4;
   static_assert(8 * kNumBars + 8 <= 1024, "barrier area overflows the misc block");
+  const uint32_t recv_bar = bar_base + 8u * (kNumBars - 4);   // split-K: the other CTAs' slices have landed
   const uint32_t epi_bar = bar_base + 8u * (kNumBars - 3);
   const uint32_t cfull_bar = bar_base + 8u * (kNumBars - 2);
   const uint32_t cfree_bar = bar_base + 8u * (kNumBars - 1);
@@ -315,6 +336,7 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     mbar_init(epi_bar, kEpiWarps);
     mbar_init(cfull_bar, kEpiWarps);
     mbar_init(cfree_bar, is_dense(MODE) ? 1 : 2);
+    mbar_init(recv_bar, 1);
     *abort_flag = 0;
     fence_proxy_async_smem();
     fence_barrier_init();
@@ -329,6 +351,7 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if constexpr (SPLIT) cluster_sync_all();   // every receive barrier exists before anybody signals one
 
   // Everything above touched no global memory, so it may overlap the tail of the previous kernel in
   // the stream (programmatic dependent launch); nothing below starts before that kernel's results
@@ -336,8 +359,12 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  const TileWalker<BN, MODE> walk(p);
-  const int KB = p.K / BK;
+  const TileWalker<BN, MODE, SPLIT> walk(p);
+  // K blocks [kb_first, kb_first + KB) of the tile are this CTA's
+  const int split = SPLIT ? static_cast<int>(cluster_ctarank()) : 0;
+  const int kb_first = SPLIT ? split * p.kbps : 0;
+  const int KBt = p.K / BK;
+  const int KB = SPLIT ? min(p.kbps, KBt - kb_first) : KBt;
 
   // Register re-balancing. setmaxnreg.inc blocks until the CTA's own pool (registers per thread at
   // launch x 384 threads = 168 x 384) can satisfy it, so the totals after the exchange must fit in
@@ -391,10 +418,10 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           }
           const uint32_t sa = smem_base + s * C::kStageBytes;
           const uint32_t sb = sa + kATileBytes;
-          const uint8_t* src = wbase + kb * row_stride_kb + static_cast<size_t>(n0) * BK;
+          const uint8_t* src = wbase + (kb_first + kb) * row_stride_kb + static_cast<size_t>(n0) * BK;
           if constexpr (is_dense(MODE)) {
             mbar_arrive_expect_tx(full_bar(s), p.a_box_rows * BK + rows_b * BK);
-            tma_load_2d(sa, &tmap_a, kb * BK, m_blk * BM, full_bar(s));
+            tma_load_2d(sa, &tmap_a, (kb_first + kb) * BK, m_blk * BM, full_bar(s));
             bulk_load(sb, src, rows_b * BK, full_bar(s));
           } else if constexpr (is_moe1(MODE)) {
             mbar_arrive_expect_tx(full_bar(s), 2 * rows_b * BK + (p.a_sorted ? p.a_box_rows * BK : 0));
@@ -544,7 +571,7 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           const int n0 = pos.n_tile * C::kOutCols;
           if (MODE == kMoe1 && BN == 256 && p.out_q) {
             // re-quantised tile: 128 rows x 128 fp8 bytes in region 0, the rows' scales in region 1
-            const float* scale_s = reinterpret_cast<const float*>(smem_al + kStages * C::kStageBytes +
+            const float* scale_s = reinterpret_cast<const float*>(smem_al + C::kRingBytes +
                                                                   kRegionBytes) + 2 * BM;
             const int c8 = lane & 7;   // 8 chunks of 16 bytes per row
             if (n0 + 128 <= p.N) {
@@ -723,8 +750,8 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         c.sa_step = p.M;
         const int n0 = n_tile * BN;
         const int nblk_max = (p.N + 127) / 128 - 1;
-        sb_idx0 = static_cast<long long>(min((n0 + half * CH) / 128, nblk_max)) * KB;
-        sb_idx1 = static_cast<long long>(min((n0 + BN / 2 + half * CH) / 128, nblk_max)) * KB;
+        sb_idx0 = static_cast<long long>(min((n0 + half * CH) / 128, nblk_max)) * KBt;
+        sb_idx1 = static_cast<long long>(min((n0 + BN / 2 + half * CH) / 128, nblk_max)) * KBt;
       } else {
         const int e = p.expert_ids[m_blk];
         if (e < 0 || e >= p.experts) return false;
@@ -774,6 +801,11 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       c.sa = p.scale_a + sa_idx;
       c.sb0 = p.scale_b + sb_idx0;
       c.sb1 = p.scale_b + sb_idx1;
+      if constexpr (SPLIT && !is_pt(MODE)) {
+        c.sa += kb_first * c.sa_step;
+        c.sb0 += kb_first;
+        c.sb1 += kb_first;
+      }
       return true;
     };
     auto setup_output = [&](const TilePos& pos, OutCtx& c) {
@@ -839,6 +871,7 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     constexpr int LDW = (CH > 32) ? 16 : CH;
     constexpr int NSUB = CH / LDW;            // loads per column group
     constexpr int NQ = 2 * NSUB;              // loads per K block (two column groups)
+    bool exchanged = false;                   // split-K: this warp has passed the exchange barrier
     uint32_t tiles_done = 0;                  // dense: tiles (per-token mode: half tiles) staged so far
     uint32_t pt_tiles = 0;                    // per-token mode: tiles drained so far
     uint32_t dn_i = 0, dn_ph = 0;             // it % kDone and (it / kDone) & 1, kept as counters
@@ -1025,7 +1058,92 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const float route_w = oc.route_w;
       const float* accf = reinterpret_cast<const float*>(acc);  // [0,CH) group 0, [CH,2CH) group 1
       // ---- output ----
-      if constexpr (C::kStaged) {
+      if constexpr (SPLIT) {
+        // Split-K exchange. The tile's valid rows are dealt out to the CTAs of the cluster in slices.
+        // Every CTA lays its fp32 partial tile down row by row in shared memory (over the ring: all of
+        // its MMAs have completed), one bulk copy per owner moves that owner's slice into its receive
+        // area, and the owner adds the slices in rank order: deterministic, no workspace. No copy may
+        // start before every CTA of the cluster has consumed its last stage: the cluster barrier.
+        // Rows are 4 BN bytes, 16-byte chunks swizzled by the row so that the eight rows that a store
+        // phase touches fall on different banks.
+        const int mrows = min(BM, p.M - m_blk * BM);
+        const int rps = C::split_rows(mrows, p.splits);
+        constexpr int kRowBytes = BN * 4;
+        if (threadIdx.x == kEpiWarp0 * 32) {
+          const int own = max(0, min(mrows, (split + 1) * rps) - split * rps);
+          if (own > 0) mbar_arrive_expect_tx(recv_bar, static_cast<uint32_t>((p.splits - 1) * own * kRowBytes));
+        }
+        __syncwarp();
+        cluster_arrive();
+        if (row_ok) {
+#pragma unroll
+          for (int grp = 0; grp < 2; ++grp) {
+#pragma unroll
+            for (int j = 0; j < CH; j += 4) {
+              const int chunk = ((grp ? col1 : col0) + j) >> 2;
+              const uint32_t addr = smem_base + r * kRowBytes + ((chunk ^ (r & 7)) << 4);
+              asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(accf[grp * CH + j]),
+                           "f"(accf[grp * CH + j + 1]), "f"(accf[grp * CH + j + 2]), "f"(accf[grp * CH + j + 3])
+                           : "memory");
+            }
+          }
+        }
+        cluster_wait();
+        exchanged = true;
+        fence_proxy_async_smem();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        constexpr uint32_t kRecvOff = BM * kRowBytes;   // receive area: [sender, own rank left out][row of the slice]
+        if (ew < p.splits && ew != split && lane == 0) {   // one copy per owner, each from a warp of its own
+          const int lo = ew * rps;
+          const int rows = min(mrows, lo + rps) - lo;
+          if (rows > 0) {
+            const int slot = split < ew ? split : split - 1;
+            bulk_copy_to_cta(map_to_cta(smem_base + kRecvOff + static_cast<uint32_t>(slot * rps * kRowBytes), ew),
+                             smem_base + static_cast<uint32_t>(lo * kRowBytes),
+                             static_cast<uint32_t>(rows * kRowBytes), map_to_cta(recv_bar, ew));
+          }
+        }
+        __syncwarp();
+        const int lo = split * rps;
+        const int own = min(mrows, lo + rps) - lo;
+        if (own > 0) {
+          const bool got = mbar_wait(recv_bar, 0, abort_flag, p.err, kErrWaitExchange);
+          if (!__all_sync(0xffffffffu, got)) { alive = false; break; }
+          constexpr int kChunks = BN / 4;                          // 16-byte chunks of a row
+          constexpr int kLanes = kChunks < 32 ? kChunks : 32;      // lanes on a row
+          constexpr int kRowsPerStep = 32 / kLanes;
+          for (int i0 = ew * kRowsPerStep; i0 < own; i0 += kEpiWarps * kRowsPerStep) {
+            const int i = i0 + lane / kLanes;
+            if (i < own) {
+              const int rr = lo + i;   // row of the tile
+#pragma unroll
+              for (int u = 0; u < kChunks / kLanes; ++u) {
+                const int chunk = (lane % kLanes) + u * kLanes;
+                const uint32_t sw = static_cast<uint32_t>((chunk ^ (rr & 7)) << 4);
+                float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int c = 0; c < p.splits; ++c) {   // fixed rank order
+                  const uint32_t addr =
+                      c == split ? smem_base + rr * kRowBytes + sw
+                                 : smem_base + kRecvOff + ((c < split ? c : c - 1) * rps + i) * kRowBytes + sw;
+                  float4 v;
+                  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                               : "r"(addr)
+                               : "memory");
+                  sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+                }
+                const int col = n0 + chunk * 4;
+                if (col < p.N) {   // N % 16 == 0: a chunk is all in or all out
+                  uint2 q;
+                  q.x = pack2(sum.x, sum.y, OutT());
+                  q.y = pack2(sum.z, sum.w, OutT());
+                  *reinterpret_cast<uint2*>(out + static_cast<size_t>(m_blk * BM + rr) * p.N + col) = q;
+                }
+              }
+            }
+          }
+        }
+      } else if constexpr (C::kStaged) {
         // (1) the staging tile must be free. Dense: the store warp's TMA store of the previous tile
         //     has read it (cfree; 16 K blocks have passed, so this wait is normally over at once).
         //     MoE: the previous tile's cooperative row stores are done (every thread passes this
@@ -1061,7 +1179,7 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             // stores them; the row's two threads (64 columns each) exchange their amax through
             // shared memory. fp8 tile: 128 rows x 128 bytes in staging region 0 (16-byte chunks
             // swizzled by row); amax/scale scratch in region 1.
-            float* amax_s = reinterpret_cast<float*>(smem_al + kStages * C::kStageBytes + kRegionBytes);
+            float* amax_s = reinterpret_cast<float*>(smem_al + C::kRingBytes + kRegionBytes);
             float* scale_s = amax_s + 2 * BM;
             float* yq = const_cast<float*>(accf);   // y overwrites the gate half of the accumulators
             float vmax = -3.4e38f, vmin = 3.4e38f;
@@ -1285,6 +1403,17 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       }
       pos = npos;
     }
+    if constexpr (SPLIT) {
+      __syncwarp();
+      if (!exchanged) cluster_sync_all();   // a warp that gave up: the cluster's barriers still count it
+    }
+  }
+  if constexpr (SPLIT) {
+    __syncwarp();
+    if (warp < kEpiWarp0) cluster_sync_all();   // (exchange barrier, see the epilogue)
+    // nobody leaves before every copy that reads its shared memory has landed: owners arrive after
+    // their receive barrier
+    cluster_sync_all();
   }
 
   // ---------------- teardown ----------------
@@ -1346,7 +1475,7 @@ template <int BN, int MODE, typename OutT>
 static int launch(const CUtensorMap& tmap_a, const CUtensorMap& tmap_c, const GemmParams& p,
                   int grid, cudaStream_t stream) {
   using C = Cfg<BN, MODE, OutT>;
-  auto kern = bs_gemm_kernel<BN, MODE, OutT>;
+  auto kern = bs_gemm_kernel<BN, MODE, OutT, false>;
   static thread_local int configured_dev = -1;
   int dev = 0;
   FLYB200_CUDA_CHECK(cudaGetDevice(&dev));
@@ -1369,6 +1498,45 @@ static int launch(const CUtensorMap& tmap_a, const CUtensorMap& tmap_c, const Ge
   return FLYB200_OK;
 }
 
+// Split-K launch: clusters of p.splits CTAs, one tile per cluster.
+template <int BN, int MODE, typename OutT>
+static int launch_split(const CUtensorMap& tmap_a, const GemmParams& p, int tiles, cudaStream_t stream) {
+  using C = Cfg<BN, MODE, OutT, true>;
+  auto kern = bs_gemm_kernel<BN, MODE, OutT, true>;
+  static thread_local int configured_dev = -1;
+  int dev = 0;
+  FLYB200_CUDA_CHECK(cudaGetDevice(&dev));
+  if (configured_dev != dev) {
+    FLYB200_CUDA_CHECK(
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+    configured_dev = dev;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * p.splits), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attrs[2];
+  attrs[0].id = cudaLaunchAttributeClusterDimension;
+  attrs[0].val.clusterDim.x = static_cast<unsigned>(p.splits);
+  attrs[0].val.clusterDim.y = 1;
+  attrs[0].val.clusterDim.z = 1;
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attrs;
+  cfg.numAttrs = 2;
+  FLYB200_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, tmap_a, tmap_a, p));
+  return FLYB200_OK;
+}
+template <int MODE, typename OutT>
+static int launch_split_bn(int bn, const CUtensorMap& tmap_a, const GemmParams& p, int tiles, cudaStream_t stream) {
+  switch (bn) {
+    case 64: return launch_split<64, MODE, OutT>(tmap_a, p, tiles, stream);
+    case 128: return launch_split<128, MODE, OutT>(tmap_a, p, tiles, stream);
+    default: return launch_split<256, MODE, OutT>(tmap_a, p, tiles, stream);
+  }
+}
+
 template <int MODE, typename OutT>
 static int launch_bn(int bn, const CUtensorMap& tmap_a, const CUtensorMap& tmap_c,
                      const GemmParams& p, int grid, cudaStream_t stream) {
@@ -1386,11 +1554,15 @@ static int launch_bn(int bn, const CUtensorMap& tmap_a, const CUtensorMap& tmap_
 
 static inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
+// Time of one K block of a tile (ns), measured on B200: the slope over K of graph replays with cold
+// operands (M = 256, N = 4096: 32 columns 0.25, 64 0.21-0.25, 128 0.27, 256 0.46 us) and of full waves
+// (M = N = 4096, K = 7168: 128 columns 0.36, 256 0.50 us).
+static double tile_kb_ns(int bn) { return bn == 256 ? 490.0 : bn == 128 ? 330.0 : bn == 64 ? 250.0 : 245.0; }
+
 // Tile-width heuristic (role of select_tile_config in the reference's test). Cost model per K block
-// of one tile, fitted to measurements on B200: the tensor-core side costs a fixed ~360 ns (MMA
-// issue, TMEM round trip of the promotion) plus ~0.9 ns per output column; the memory side costs
-// the tile's weight bytes at one SM's share of HBM bandwidth when few row blocks share them. The
-// persistent loop runs ceil(tiles / SMs) rounds; pick the width with the smallest total.
+// of one tile: tile_kb_ns on the tensor-core side; the memory side costs the tile's weight bytes at one
+// SM's share of HBM bandwidth when few row blocks share them. The persistent loop runs
+// ceil(tiles / SMs) rounds; pick the width with the smallest total.
 static int pick_block_n(int m_blocks, int n_cols, int sms, bool moe1) {
   const int cands[4] = {256, 128, 64, 32};
   int best = 128;
@@ -1401,7 +1573,7 @@ static int pick_block_n(int m_blocks, int n_cols, int sms, bool moe1) {
     const int cols = moe1 ? bn / 2 : bn;
     const long tiles = static_cast<long>(m_blocks) * cdiv(n_cols, cols);
     const long rounds = (tiles + sms - 1) / sms;
-    const double compute_ns = 360.0 + 0.9 * bn;
+    const double compute_ns = tile_kb_ns(bn);
     // weight tile bytes per K block over ~44 GB/s per SM; row blocks that run concurrently on the
     // same weight tile share one HBM read through L2
     const int sharing = m_blocks < 8 ? (m_blocks < 1 ? 1 : m_blocks) : 8;
@@ -1411,6 +1583,91 @@ static int pick_block_n(int m_blocks, int n_cols, int sms, bool moe1) {
     if (cost < best_cost - 1e-9) {
       best_cost = cost;
       best = bn;
+    }
+  }
+  return best;
+}
+
+// Clusters of `splits` CTAs of the split-K kernel that the GPU holds at once: 148 SMs are not a
+// multiple of every cluster size, and a cluster stays inside one of the GPU's SM groups.
+template <int BN>
+static int query_clusters(int splits) {
+  using C = Cfg<BN, kDense, __nv_bfloat16, true>;
+  auto kern = bs_gemm_kernel<BN, kDense, __nv_bfloat16, true>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(splits), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = C::kSmemBytes;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = static_cast<unsigned>(splits);
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+// Every width's kernel takes a whole SM, so one width answers for all. Asked once per device and thread.
+static int max_clusters(int splits) {
+  static thread_local int dev_of = -1;
+  static thread_local int known[9];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (dev != dev_of) {
+    for (int i = 0; i < 9; ++i) known[i] = -1;
+    dev_of = dev;
+  }
+  if (known[splits] < 0) known[splits] = query_clusters<128>(splits);
+  return known[splits];
+}
+
+// Split-K plan of a dense problem: the tile width and cluster size with the smallest estimated time, or
+// splits = 1 where the plain tiled kernel is estimated to be as fast. All clusters have to be resident
+// at once (a second wave doubles the time: M = 256, N = 1024, K = 8192 with 16 clusters of eight 18.2
+// us, with 32 of four 10.7). The exchange costs ~3 us and ~50 ns per KB that leaves a CTA. Measured, 56 K
+// blocks, 1 / 2 / 4 CTAs per tile: 12 tiles of 128 columns 20.2 / 15.6 / 11.5 us, 6 tiles of 256 28.0 /
+// 21.2 / 16.1 us, 64 tiles of 128 (two per tile) 16.8 against 17.7 us for 128 unsplit tiles of 64.
+struct SplitPlan {
+  int bn, splits, kbps;
+};
+static SplitPlan pick_split(int M, int N, int K, int sms, bool pertoken, int force_bn, int force_splits) {
+  const int m_blocks = cdiv(M, BM), kbt = K / BK;
+  const int rows = M < BM ? M : BM;
+  // per-token scales: no promotion per K block, 256-wide tiles at the tensor core's pace
+  auto kb_ns = [&](int bn) { return pertoken ? 330.0 : tile_kb_ns(bn); };
+  SplitPlan best{force_bn, 1, kbt};
+  double best_cost = 1e30;
+  if (!force_splits) {
+    const int bn = pertoken ? 256 : pick_block_n(m_blocks, N, sms, false);
+    const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
+    best = SplitPlan{bn, 1, kbt};
+    best_cost = ((tiles + sms - 1) / sms) * kbt * kb_ns(bn);
+  }
+  const int widths[3] = {256, 128, 64};
+  for (int w = 0; w < 3; ++w) {
+    const int bn = widths[w];
+    if ((force_bn && bn != force_bn) || (pertoken && bn != 256)) continue;
+    const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
+    for (int sp = 2; sp <= (bn == 256 ? 4 : 8); ++sp) {
+      if (force_splits && sp != force_splits) continue;
+      const int kbps = cdiv(kbt, sp);
+      if (cdiv(kbt, kbps) != sp) continue;           // some CTA would have no K block
+      if (!force_splits && (tiles * sp > sms || tiles > max_clusters(sp))) continue;
+      const double exchange = 3000.0 + rows * bn * 4.0 * (sp - 1) / sp / 20.0;
+      const double cost = kbps * kb_ns(bn) + exchange;
+      if (cost < best_cost - 1e-9) {
+        best_cost = cost;
+        best = SplitPlan{bn, sp, kbps};
+      }
     }
   }
   return best;
@@ -1478,7 +1735,12 @@ extern "C" int flyb200_blockscale_gemm(void* c, const void* a, const void* b_rep
   const int sms = sm_count();
   if (sms <= 0) return FLYB200_ERR_CUDA;
   const int m_blocks = cdiv(M, BM);
-  int bn = (cfg && cfg->block_n) ? cfg->block_n : pick_block_n(m_blocks, N, sms, false);
+  SplitPlan plan{0, 1, K / BK};
+  if (path == 1 && cfg->split_k > 1 && cfg->block_n != 32)   // asked for: split if the plan exists
+    plan = pick_split(M, N, K, sms, false, cfg->block_n, cfg->split_k);
+  else if (path == 0 && !(cfg && (cfg->block_n || cfg->max_ctas || cfg->split_k)))
+    plan = pick_split(M, N, K, sms, false, 0, 0);
+  int bn = (cfg && cfg->block_n) ? cfg->block_n : plan.splits > 1 ? plan.bn : pick_block_n(m_blocks, N, sms, false);
   int grid = sms;
   if (cfg && cfg->max_ctas > 0 && cfg->max_ctas < grid) grid = cfg->max_ctas;
   const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
@@ -1501,6 +1763,13 @@ extern "C" int flyb200_blockscale_gemm(void* c, const void* a, const void* b_rep
   if ((rc = make_tensor_map_2d(&tmap_a, a, M, K, 1, p.a_box_rows))) return rc;
   if ((rc = make_tensor_map_2d(&tmap_c, c, M, N, 2, p.a_box_rows))) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  p.splits = plan.splits;
+  p.kbps = plan.kbps;
+  if (plan.splits > 1) {
+    if (out_dtype == FLYB200_BF16)
+      return launch_split_bn<kDense, __nv_bfloat16>(bn, tmap_a, p, static_cast<int>(tiles), st);
+    return launch_split_bn<kDense, __half>(bn, tmap_a, p, static_cast<int>(tiles), st);
+  }
   if (out_dtype == FLYB200_BF16)
     return launch_bn<kDense, __nv_bfloat16>(bn, tmap_a, tmap_c, p, grid, st);
   return launch_bn<kDense, __half>(bn, tmap_a, tmap_c, p, grid, st);
@@ -1545,6 +1814,11 @@ extern "C" int flyb200_pertoken_gemm(void* c, const void* a, const void* b_repac
   const int sms = sm_count();
   if (sms <= 0) return FLYB200_ERR_CUDA;
   const int m_blocks = cdiv(M, BM);
+  SplitPlan plan{256, 1, K / BK};
+  if (path == 1 && cfg->split_k > 1)
+    plan = pick_split(M, N, K, sms, true, 256, cfg->split_k);
+  else if (path == 0 && !(cfg && (cfg->block_n || cfg->max_ctas || cfg->split_k)))
+    plan = pick_split(M, N, K, sms, true, 256, 0);
   int grid = sms;
   if (cfg && cfg->max_ctas > 0 && cfg->max_ctas < grid) grid = cfg->max_ctas;
   const long tiles = static_cast<long>(m_blocks) * cdiv(N, 256);
@@ -1565,6 +1839,13 @@ extern "C" int flyb200_pertoken_gemm(void* c, const void* a, const void* b_repac
   if ((rc = make_tensor_map_2d(&tmap_a, a, M, K, 1, p.a_box_rows))) return rc;
   if ((rc = make_tensor_map_2d(&tmap_c, c, M, N, 2, p.a_box_rows))) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  p.splits = plan.splits;
+  p.kbps = plan.kbps;
+  if (plan.splits > 1) {
+    if (out_dtype == FLYB200_BF16)
+      return launch_split<256, kDensePT, __nv_bfloat16>(tmap_a, p, static_cast<int>(tiles), st);
+    return launch_split<256, kDensePT, __half>(tmap_a, p, static_cast<int>(tiles), st);
+  }
   if (out_dtype == FLYB200_BF16) return launch<256, kDensePT, __nv_bfloat16>(tmap_a, tmap_c, p, grid, st);
   return launch<256, kDensePT, __half>(tmap_a, tmap_c, p, grid, st);
 }
