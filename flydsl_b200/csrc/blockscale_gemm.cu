@@ -175,11 +175,6 @@ __device__ __forceinline__ float round_through(float v, __nv_bfloat16) {
 }
 __device__ __forceinline__ float round_through(float v, float) { return v; }
 
-__device__ __forceinline__ float silu_mul(float g, float u) {
-  // silu(g) * u with the fast exp, as the reference does (moe_blockscale_2stage.py:239-251).
-  return __fdividef(g, 1.0f + __expf(-g)) * u;
-}
-
 // Tile bookkeeping shared by every role so that all of them walk the same sequence: tile
 // blockIdx.x, then one grid further, and so on. A position carries (m block, n tile) and is advanced
 // with additions only (the integer division happens once, in start()).
@@ -1685,6 +1680,12 @@ int launch_decode_gemm(void* c, const void* a, const void* b_repacked, const flo
                        const float* scale_b, int M, int N, int K, int out_dtype, int force_splits,
                        cudaStream_t stream, bool pertoken);
 bool decode_path_pays_off(int M, int N, int K);
+// moe_swap.cu
+int launch_moe_swap(int stage, bool pertoken, void* out, const void* act, const void* w_repacked,
+                    const float* scale_x, const float* scale_w, const int32_t* sorted_ids, const int32_t* expert_ids,
+                    const float* sorted_weights, const int32_t* num_valid_ids, int T, int n, int kdim, int num_blocks,
+                    int E, int k, int tile_m, int doweight, int accumulate, int out_sorted, int a_rows, int out_dtype,
+                    int max_ctas, cudaStream_t stream);
 // pt_pair_gemm.cu
 int launch_pertoken_pair_gemm(void* c, const void* a, const void* b_repacked, const float* scale_a,
                               const float* scale_b, int M, int N, int K, int out_dtype, int max_ctas, int group_m,
@@ -1896,6 +1897,12 @@ static int moe_sorted_layout(const flyb200_gemm_cfg* cfg, int T, int E, int k, i
   return make_tensor_map_2d(tmap, act, p->a_rows, kdim, 1, tile_m);
 }
 
+// Small routing blocks take the kernel with the weights on the MMA's M side (moe_swap.cu), unless a tile
+// width was asked for: up to 32 tokens per block, where the tiled kernel's 128 rows are mostly padding.
+static bool moe_swap_pays_off(const flyb200_gemm_cfg* cfg, const GemmParams& p) {
+  return p.a_sorted && p.tile_m <= 32 && !cfg->block_n;
+}
+
 static int moe_gemm1_impl(void* out, void* out_q, float* out_scale_t, const void* x, const void* w_repacked,
                           const float* scale_x, const float* scale_w, const int32_t* sorted_ids,
                           const int32_t* expert_ids, const float* sorted_weights,
@@ -1947,6 +1954,10 @@ static int moe_gemm1_impl(void* out, void* out_q, float* out_scale_t, const void
   CUtensorMap tmap{};
   if ((rc = moe_sorted_layout(cfg, T, E, k, tile_m, H, x, &p, &tmap))) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (!out_q && moe_swap_pays_off(cfg, p))
+    return launch_moe_swap(1, pertoken, out, x, w_repacked, scale_x, scale_w, sorted_ids, expert_ids, sorted_weights,
+                           num_valid_ids, T, I, H, num_blocks, E, k, tile_m, doweight, 0, p.out_sorted, p.a_rows,
+                           out_dtype, cfg->max_ctas, st);
   if (pertoken) {
     if (out_dtype == FLYB200_BF16) return launch<256, kMoe1PT, __nv_bfloat16>(tmap, tmap, p, grid, st);
     return launch<256, kMoe1PT, __half>(tmap, tmap, p, grid, st);
@@ -2021,6 +2032,10 @@ static int moe_gemm2_impl(void* out, const void* a2, const void* w_repacked,
   if (p.out_sorted)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "stage 2 has no sorted output layout (cfg.path bit 1)");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (moe_swap_pays_off(cfg, p))
+    return launch_moe_swap(2, pertoken, out, a2, w_repacked, scale_x, scale_w, sorted_ids, expert_ids, sorted_weights,
+                           num_valid_ids, T, H, I, num_blocks, E, k, tile_m, doweight, accumulate, 0, p.a_rows,
+                           out_dtype, cfg->max_ctas, st);
   if (pertoken) {
     if (out_dtype == FLYB200_BF16) return launch<256, kMoe2PT, __nv_bfloat16>(tmap, tmap, p, grid, st);
     if (out_dtype == FLYB200_F16) return launch<256, kMoe2PT, __half>(tmap, tmap, p, grid, st);

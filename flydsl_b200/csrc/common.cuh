@@ -328,6 +328,11 @@ __device__ __forceinline__ void reg_alloc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R));
 }
 
+__device__ __forceinline__ float silu_mul(float g, float u) {
+  // silu(g) * u with the fast exp, as the reference does (moe_blockscale_2stage.py:239-251).
+  return __fdividef(g, 1.0f + __expf(-g)) * u;
+}
+
 // ---- output packing ----------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t pack2(float a, float b, __nv_bfloat16) {
   __nv_bfloat162 v = __floats2bfloat162_rn(a, b);

@@ -59,6 +59,8 @@ class BlockscaleMoE:
         # the stage-1 output and its re-quantisation stay in routing order as well.
         # Measured on the 256-expert layer: 4.31 -> 3.76 ms at 128-token blocks, but slightly slower
         # for decode-size batches (one more launch, nothing to hide), hence the default by block size.
+        # Blocks of at most 32 rows take these layouts all the same where forward() does the routing
+        # itself: the stages are then the kernel with the weights on the MMA's M side.
         self.sorted_layout = (self.tile_m >= 64 and self.tile_m % 8 == 0) if sorted_layout is None \
             else bool(sorted_layout)
         # Optional: re-quantisation between the stages fused into the stage-1 epilogue (routing-order
@@ -71,12 +73,17 @@ class BlockscaleMoE:
             raise ValueError("fused_quant needs sorted_layout and block_n1 in (None, 256)")
         common = dict(model_dim=self.H, inter_dim=self.I, experts=self.E, topk=self.topk,
                       tile_m=self.tile_m, tile_n=256, tile_k=128)
-        self.gemm1 = compile_moe_blockscale_gemm1(doweight_stage1=False, out_dtype=_DT_NAME[mid_dtype],
-                                                  block_n=block_n1, a_sorted=self.sorted_layout,
-                                                  out_sorted=self.sorted_layout, **common)
-        self.gemm2 = compile_moe_blockscale_gemm2(doweight_stage2=True, out_dtype=_DT_NAME[out_dtype],
-                                                  accumulate=(mode == "atomic"), block_n=block_n2,
-                                                  a_sorted=self.sorted_layout, **common)
+
+        def stages(in_order):
+            return (compile_moe_blockscale_gemm1(doweight_stage1=False, out_dtype=_DT_NAME[mid_dtype],
+                                                 block_n=block_n1, a_sorted=in_order, out_sorted=in_order, **common),
+                    compile_moe_blockscale_gemm2(doweight_stage2=True, out_dtype=_DT_NAME[out_dtype],
+                                                 accumulate=(mode == "atomic"), block_n=block_n2, a_sorted=in_order,
+                                                 **common))
+
+        self.gemm1, self.gemm2 = stages(self.sorted_layout)
+        small = sorted_layout is None and self.tile_m <= 32 and self.tile_m % 8 == 0 and not (block_n1 or block_n2)
+        self._small_stages = stages(True) if small else None
         self.reduce = compile_moe_reduction(topk=self.topk, model_dim=self.H,
                                             dtype_str=_DT_NAME[out_dtype]) if mode == "reduce" else None
         self._buf = {}
@@ -86,21 +93,25 @@ class BlockscaleMoE:
         """Build from plain row-major fp8 weights (repacks them on the GPU)."""
         return cls(shuffle_weight(w1_q), w1_scale, shuffle_weight(w2_q), w2_scale, **kw)
 
-    def _buffers(self, T: int, dev):
-        key = (T, dev)
+    def _buffers(self, T: int, dev, in_order: Optional[bool] = None):
+        in_order = self.sorted_layout if in_order is None else in_order
+        key = (T, dev, in_order)
         b = self._buf.get(key)
         if b is None:
+            # rows of padding positions are never written and never looked at, whatever they hold; the
+            # layouts that a caller's routing can meet start out as zeros all the same
+            new = torch.empty if in_order and not self.sorted_layout else torch.zeros
             # rows of the stage-1 output / stage-2 input: routes, or sorted positions incl. padding
-            L = (T * self.topk + self.E * self.tile_m - self.topk) if self.sorted_layout else T * self.topk
+            L = (T * self.topk + self.E * self.tile_m - self.topk) if in_order else T * self.topk
             b = {
                 "rows": L,
                 "x_sorted": torch.empty((L, self.H), dtype=torch.float8_e4m3fn, device=dev)
-                if self.sorted_layout else None,
+                if in_order else None,
                 "xs_sorted": torch.empty((self.H // 128, L), dtype=torch.float32, device=dev)
-                if self.sorted_layout else None,
-                "out1": None if self.fused_quant else torch.zeros((L, self.I), dtype=self.mid_dtype, device=dev),
-                "a2_q": torch.zeros((L, self.I), dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn),
-                "a2_s": torch.zeros((self.I // 128, L), dtype=torch.float32, device=dev),
+                if in_order else None,
+                "out1": None if self.fused_quant else new((L, self.I), dtype=self.mid_dtype, device=dev),
+                "a2_q": new((L, self.I), dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn),
+                "a2_s": new((self.I // 128, L), dtype=torch.float32, device=dev),
                 "routes": torch.empty((T * self.topk, self.H), dtype=self.out_dtype, device=dev)
                 if self.mode == "reduce" else None,
             }
@@ -119,11 +130,15 @@ class BlockscaleMoE:
         # every launch below goes to torch's current stream (stream=None)
         T = x_q.shape[0]
         dev = x_q.device
-        b = self._buffers(T, dev)
+        dense_in = x_q.is_contiguous() and x_scale_t.is_contiguous()
+        small = self._small_stages is not None and routing is None and dense_in
+        gemm1, gemm2 = self._small_stages if small else (self.gemm1, self.gemm2)
+        in_order = self.sorted_layout or small
+        b = self._buffers(T, dev, in_order)
         permuted = False
         if routing is None:
             # routing-order layouts: the sort kernel also permutes the activations (one launch)
-            fuse = self.sorted_layout and x_q.is_contiguous() and x_scale_t.is_contiguous()
+            fuse = in_order and dense_in
             sid, sw, seid, npp = moe_sorting(
                 topk_ids, topk_weights, num_experts=self.E, block_size=self.tile_m,
                 permute=(x_q, x_scale_t, b["x_sorted"], b["xs_sorted"]) if fuse else None)
@@ -132,24 +147,24 @@ class BlockscaleMoE:
             sid, sw, seid, npp = routing
         nblk = seid.numel()
         mid_code = {torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}[self.mid_dtype]
-        if self.sorted_layout:
+        if in_order:
             if sid.numel() != b["rows"]:
                 raise ValueError("routing buffers do not match this layer's experts/tile_m/topk")
             if not permuted:
                 moe_gather_rows(x_q, x_scale_t, sid, npp, topk=self.topk, out=b["x_sorted"],
                                 scale_out=b["xs_sorted"])
             if self.fused_quant:
-                self.gemm1.quantized(b["a2_q"], b["a2_s"], b["x_sorted"], self.w1, b["xs_sorted"],
-                                     self.w1_scale, sid, seid, sw, npp, T, nblk, None)
+                gemm1.quantized(b["a2_q"], b["a2_s"], b["x_sorted"], self.w1, b["xs_sorted"],
+                                self.w1_scale, sid, seid, sw, npp, T, nblk, None)
             else:
-                self.gemm1(b["out1"], b["x_sorted"], self.w1, b["xs_sorted"], self.w1_scale, sid, seid, sw,
-                           npp, T, self.I, self.H, nblk, None)
+                gemm1(b["out1"], b["x_sorted"], self.w1, b["xs_sorted"], self.w1_scale, sid, seid, sw,
+                      npp, T, self.I, self.H, nblk, None)
                 _lib.check(_lib.load().flyb200_quant_1x128_devrows(
                     b["out1"].data_ptr(), b["a2_q"].data_ptr(), b["a2_s"].data_ptr(), npp.data_ptr(),
                     b["rows"], self.I, mid_code, _lib.stream_handle(None)))
         else:
-            self.gemm1(b["out1"], x_q, self.w1, x_scale_t, self.w1_scale, sid, seid, sw, npp, T, self.I,
-                       self.H, nblk, None)
+            gemm1(b["out1"], x_q, self.w1, x_scale_t, self.w1_scale, sid, seid, sw, npp, T, self.I,
+                  self.H, nblk, None)
             _lib.check(_lib.load().flyb200_quant_1x128(
                 b["out1"].data_ptr(), b["a2_q"].data_ptr(), b["a2_s"].data_ptr(), T * self.topk, self.I,
                 mid_code, _lib.stream_handle(None)))
@@ -157,16 +172,16 @@ class BlockscaleMoE:
             out = torch.empty((T, self.H), dtype=self.out_dtype, device=dev)
         if self.mode == "atomic":
             out.zero_()
-            self.gemm2(out, b["a2_q"], self.w2, b["a2_s"], self.w2_scale, sid, seid, sw, npp, T,
-                       self.H, self.I, nblk, None)
+            gemm2(out, b["a2_q"], self.w2, b["a2_s"], self.w2_scale, sid, seid, sw, npp, T,
+                  self.H, self.I, nblk, None)
         else:
             if routing is not None:
                 # A caller's routing may drop routes (expert_mask, ids outside the local experts):
                 # their rows are never written by stage 2, so they must read as zero in the sum
                 # (the reference wrapper zero-fills its intermediate, :2714-2715).
                 b["routes"].zero_()
-            self.gemm2(b["routes"], b["a2_q"], self.w2, b["a2_s"], self.w2_scale, sid, seid, sw, npp,
-                       T, self.H, self.I, nblk, None)
+            gemm2(b["routes"], b["a2_q"], self.w2, b["a2_s"], self.w2_scale, sid, seid, sw, npp,
+                  T, self.H, self.I, nblk, None)
             self.reduce(b["routes"], out, None, T, None)
         return out
 
