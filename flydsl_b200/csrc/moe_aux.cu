@@ -58,6 +58,56 @@ moe_reduce_kernel(const T* __restrict__ x, T* __restrict__ y, const uint8_t* __r
   }
 }
 
+// Four quotients to four fp8 bytes.
+__device__ __forceinline__ uint32_t fp8x4(float a, float b, float c, float d) {
+  return static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3)) |
+         (static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(c, d), __NV_SATFINITE, __NV_E4M3)) << 16);
+}
+// Largest |v| of eight packed 16-bit values as a bit pattern: |v| as unsigned 16-bit integers order like
+// the values, and anything at or above the pattern of +Inf is an Inf/NaN.
+__device__ __forceinline__ uint32_t amax_bits8(const uint4& raw) {
+  const uint32_t m2 = __vmaxu2(__vmaxu2(raw.x & 0x7fff7fffu, raw.y & 0x7fff7fffu),
+                               __vmaxu2(raw.z & 0x7fff7fffu, raw.w & 0x7fff7fffu));
+  return max(m2 & 0xffffu, m2 >> 16);
+}
+template <typename T>
+__device__ __forceinline__ constexpr uint32_t inf_bits() {
+  return std::is_same<T, __half>::value ? 0x7c00u : 0x7f80u;
+}
+template <typename T>
+__device__ __forceinline__ float from_bits16(uint32_t bits) {
+  if constexpr (std::is_same<T, __half>::value) return __half2float(__ushort_as_half(static_cast<unsigned short>(bits)));
+  else return __uint_as_float(bits << 16);
+}
+// Eight packed 16-bit values over `scale`, as fp8. `rare`: some value of the group is an Inf or a NaN
+// (NaN -> 0, +-Inf -> +-448 first), the scale's mantissa is all ones, or something may be subnormal: the
+// true division. Otherwise the quotients come from one reciprocal: q0 = v*rc, q =
+// fma(fma(-d, q0, v), rc, q0) is the IEEE quotient v/d when rc is the correctly rounded reciprocal of d
+// (Markstein). The correction step loses the sign of -0 / scale = -0: the inputs' signs are put back.
+template <typename T>
+__device__ __forceinline__ uint2 quant8(const uint4& raw, float scale, float rc, bool rare) {
+  const T* e = reinterpret_cast<const T*>(&raw);
+  float v[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) v[j] = to_f32<T>(e[j]);
+  if (rare) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (v[j] != v[j]) v[j] = 0.f;
+      else if (isinf(v[j])) v[j] = v[j] > 0 ? 448.f : -448.f;
+      v[j] = __fdiv_rn(v[j], scale);
+    }
+    return make_uint2(fp8x4(v[0], v[1], v[2], v[3]), fp8x4(v[4], v[5], v[6], v[7]));
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float q0 = v[j] * rc;
+    v[j] = __fmaf_rn(__fmaf_rn(-scale, q0, v[j]), rc, q0);
+  }
+  return make_uint2(fp8x4(v[0], v[1], v[2], v[3]) | (__byte_perm(raw.x, raw.y, 0x7531) & 0x80808080u),
+                    fp8x4(v[4], v[5], v[6], v[7]) | (__byte_perm(raw.z, raw.w, 0x7531) & 0x80808080u));
+}
+
 // 16-bit inputs: half a warp per 128-wide group (16 lanes x 16 bytes), so a warp moves 512 bytes per
 // load instruction; the amax reduction stays inside the half-warp. `raw` holds the lane's 8 values
 // (zeros for a lane without work). The kernel is bound by its instruction count, so the group's amax
@@ -68,37 +118,27 @@ moe_reduce_kernel(const T* __restrict__ x, T* __restrict__ y, const uint8_t* __r
 template <typename T>
 __device__ __forceinline__ void quant_group16(const uint4& raw, uint8_t* __restrict__ q_dst,
                                               float* __restrict__ scale_dst, bool active, int sub) {
-  constexpr uint32_t kInfBits = (sizeof(T) == 2 && std::is_same<T, __half>::value) ? 0x7c00u : 0x7f80u;
-  const uint32_t m2 = __vmaxu2(__vmaxu2(raw.x & 0x7fff7fffu, raw.y & 0x7fff7fffu),
-                               __vmaxu2(raw.z & 0x7fff7fffu, raw.w & 0x7fff7fffu));
-  uint32_t amax_bits = max(m2 & 0xffffu, m2 >> 16);
+  uint32_t amax_bits = amax_bits8(raw);
 #pragma unroll
   for (int o = 8; o > 0; o >>= 1)  // xor distances < 16 stay inside the half-warp
     amax_bits = max(amax_bits, __shfl_xor_sync(0xffffffffu, amax_bits, o));
-  float v[8];
-  const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) v[j] = to_f32<T>(e[j]);
   float amax;
-  if (__any_sync(0xffffffffu, amax_bits >= kInfBits)) {
+  const bool special = __any_sync(0xffffffffu, amax_bits >= inf_bits<T>());
+  if (special) {
+    const T* e = reinterpret_cast<const T*>(&raw);
     float vmax = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      if (v[j] != v[j]) v[j] = 0.f;
-      else if (isinf(v[j])) v[j] = v[j] > 0 ? 448.f : -448.f;
-      vmax = fmaxf(vmax, fabsf(v[j]));
+      const float v = fabsf(to_f32<T>(e[j]));
+      vmax = fmaxf(vmax, v != v ? 0.f : isinf(v) ? 448.f : v);
     }
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
     amax = vmax;
-  } else if constexpr (std::is_same<T, __half>::value) {
-    amax = __half2float(__ushort_as_half(static_cast<unsigned short>(amax_bits)));
   } else {
-    amax = __uint_as_float(amax_bits << 16);
+    amax = from_bits16<T>(amax_bits);
   }
-  // Quotients from one reciprocal: q0 = y*rc, q = fma(fma(-d, q0, y), rc, q0) is the IEEE quotient
-  // y/d when rc is the correctly rounded reciprocal of d, the mantissa of d is not all ones and
-  // nothing is subnormal (Markstein); the rare other cases take the true division.
+  // amax / 448 the same way (see quant8)
   float scale;
   {
     constexpr float kRc448 = 1.0f / 448.0f;   // correctly rounded by the compiler
@@ -109,60 +149,49 @@ __device__ __forceinline__ void quant_group16(const uint4& raw, uint8_t* __restr
   if (__any_sync(0xffffffffu, tiny)) scale = __fdiv_rn(amax, 448.f);
   if (scale == 0.f) scale = 1.f;
   if (active) {
-    float qv[8];
-    if (((__float_as_uint(scale) & 0x7fffffu) == 0x7fffffu) || tiny) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) qv[j] = __fdiv_rn(v[j], scale);
-    } else {
-      const float rc = __frcp_rn(scale);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float q0 = v[j] * rc;
-        const float qc = __fmaf_rn(__fmaf_rn(-scale, q0, v[j]), rc, q0);
-        // the sign of the input, for the one case the correction step loses it: -0 / scale = -0
-        qv[j] = __uint_as_float(__float_as_uint(qc) | (__float_as_uint(v[j]) & 0x80000000u));
-      }
-    }
-    const uint32_t lo = static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(qv[0], qv[1]), __NV_SATFINITE, __NV_E4M3)) |
-                        (static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(qv[2], qv[3]), __NV_SATFINITE, __NV_E4M3)) << 16);
-    const uint32_t hi = static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(qv[4], qv[5]), __NV_SATFINITE, __NV_E4M3)) |
-                        (static_cast<uint32_t>(__nv_cvt_float2_to_fp8x2(make_float2(qv[6], qv[7]), __NV_SATFINITE, __NV_E4M3)) << 16);
-    *reinterpret_cast<uint2*>(q_dst) = make_uint2(lo, hi);
+    const bool rare = special || tiny || (__float_as_uint(scale) & 0x7fffffu) == 0x7fffffu;
+    *reinterpret_cast<uint2*>(q_dst) = quant8<T>(raw, scale, __frcp_rn(scale), rare);
     if (sub == 0) *scale_dst = scale;
   }
 }
 
-// A warp takes whole rows (the input streams sequentially, no index arithmetic beyond additions),
-// two groups per step (one per half-warp), four steps' loads in flight at once: a dependent load ->
-// reduce -> divide -> store chain per group is latency-bound with one.
+// A warp takes whole rows (the input streams sequentially, no index arithmetic beyond additions), or,
+// where there are too few rows to fill the GPU, one of `parts` equal parts of a row (eight groups at
+// least); two groups per step (one per half-warp), four steps' loads in flight at once: a dependent load
+// -> reduce -> divide -> store chain per group is latency-bound with one. (32 rows of 7168: seven such
+// steps one after the other took 13 us.)
 template <typename T>
 __device__ __forceinline__ void quant_rows16(const T* __restrict__ x, uint8_t* __restrict__ q,
                                              float* __restrict__ scale_t, int64_t rows,
-                                             int64_t scale_stride, int cols) {
+                                             int64_t scale_stride, int cols, int parts) {
   constexpr int kInFlight = 4;
   const int groups = cols / 128;
+  const int per_part = ((groups + parts - 1) / parts + 7) / 8 * 8;
   const int lane = threadIdx.x & 31;
   const int sub = lane & 15;
   const int hw = lane >> 4;
   const int64_t warp0 = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
   const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t row = warp0; row < rows; row += nwarps) {
+  for (int64_t item = warp0; item < rows * parts; item += nwarps) {
+    const int64_t row = parts == 1 ? item : item / parts;
+    const int g_first = static_cast<int>(item - row * parts) * per_part;
+    const int g_last = min(groups, g_first + per_part);
     const T* xrow = x + row * cols + sub * 8;
     uint8_t* qrow = q + row * cols + sub * 8;
     float* srow = scale_t + row;
-    for (int g0 = 0; g0 < groups; g0 += 2 * kInFlight) {
+    for (int g0 = g_first; g0 < g_last; g0 += 2 * kInFlight) {
       uint4 raw[kInFlight];
 #pragma unroll
       for (int u = 0; u < kInFlight; ++u) {
         const int g = g0 + 2 * u + hw;
         raw[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (g < groups) raw[u] = *reinterpret_cast<const uint4*>(xrow + g * 128);
+        if (g < g_last) raw[u] = *reinterpret_cast<const uint4*>(xrow + g * 128);
       }
 #pragma unroll
       for (int u = 0; u < kInFlight; ++u) {
         const int g = g0 + 2 * u + hw;
-        if (g0 + 2 * u < groups)   // warp-uniform: the shuffles inside need the whole warp
-          quant_group16<T>(raw[u], qrow + g * 128, srow + static_cast<int64_t>(g) * scale_stride, g < groups, sub);
+        if (g0 + 2 * u < g_last)   // warp-uniform: the shuffles inside need the whole warp
+          quant_group16<T>(raw[u], qrow + g * 128, srow + static_cast<int64_t>(g) * scale_stride, g < g_last, sub);
       }
     }
   }
@@ -171,8 +200,14 @@ __device__ __forceinline__ void quant_rows16(const T* __restrict__ x, uint8_t* _
 template <typename T>
 __global__ void __launch_bounds__(256)
 quant_1x128_kernel16(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale_t,
-                     int64_t rows, int cols) {
-  quant_rows16<T>(x, q, scale_t, rows, rows, cols);
+                     int64_t rows, int cols, int parts) {
+  quant_rows16<T>(x, q, scale_t, rows, rows, cols, parts);
+}
+// Parts per row (see quant_rows16): enough for the GPU's 64 warps per SM, at least eight groups each.
+static int quant_parts(int64_t rows, int cols, int sms) {
+  const int64_t want = (static_cast<int64_t>(sms) * 64 + rows - 1) / rows;
+  const int most = (cols / 128 + 7) / 8;
+  return static_cast<int>(want < most ? want : most);
 }
 
 // One warp per (row, 128-wide group): lane owns 4 consecutive elements.
@@ -284,15 +319,20 @@ extern "C" int flyb200_quant_1x128(const void* x, void* q, float* scale_t, int64
   if (blocks > static_cast<int64_t>(sms) * 16) blocks = static_cast<int64_t>(sms) * 16;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const int g = static_cast<int>(blocks);
+  // 16-bit inputs: a warp per part of a row; few of them go out in small blocks, over more SMs
+  const int parts = quant_parts(rows, cols, sms);
+  const int threads16 = rows * parts < static_cast<int64_t>(sms) * 8 ? 64 : 256;
+  const int64_t need16 = (rows * parts * 32 + threads16 - 1) / threads16;
+  const int g16 = static_cast<int>(need16 < static_cast<int64_t>(sms) * 16 ? need16 : static_cast<int64_t>(sms) * 16);
   uint8_t* qo = static_cast<uint8_t*>(q);
   switch (in_dtype) {
     case FLYB200_BF16:
-      quant_1x128_kernel16<__nv_bfloat16><<<g, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(x), qo,
-                                                             scale_t, rows, cols);
+      quant_1x128_kernel16<__nv_bfloat16><<<g16, threads16, 0, st>>>(static_cast<const __nv_bfloat16*>(x), qo,
+                                                                     scale_t, rows, cols, parts);
       break;
     case FLYB200_F16:
-      quant_1x128_kernel16<__half><<<g, 256, 0, st>>>(static_cast<const __half*>(x), qo, scale_t,
-                                                      rows, cols);
+      quant_1x128_kernel16<__half><<<g16, threads16, 0, st>>>(static_cast<const __half*>(x), qo, scale_t,
+                                                              rows, cols, parts);
       break;
     case FLYB200_F32:
       quant_1x128_kernel<float><<<g, 256, 0, st>>>(static_cast<const float*>(x), qo, scale_t, rows,
@@ -409,6 +449,81 @@ extern "C" int flyb200_moe_gather_rows_pertoken(const void* x, const float* scal
 // row, two passes over the row (the second finds it in L1/L2). Used between the stages of the
 // per-token-scale MoE, where the reference test calls the torch function on the host side.
 namespace flyb200 {
+// One pass for rows of up to 16384 values: TPR threads hold a row in registers (eight 16-byte chunks
+// each at most), so that it is read once with all its loads in flight; a block of 256 threads takes
+// 256 / TPR rows at a time. (A warp per row in two passes, 1000 rows of 7168: 28 us for 22 MB.)
+template <typename T, int TPR>
+__global__ void __launch_bounds__(256)
+quant_pertoken_row_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale,
+                          const int* __restrict__ num_rows_dev, int64_t rows_alloc, int cols) {
+  constexpr int kRows = 256 / TPR;      // rows of a block
+  constexpr int kWarps = TPR / 32;      // warps of a row
+  __shared__ uint32_t warp_bits[8];
+  __shared__ float warp_max[8];
+  const int64_t rows = num_rows_dev ? min(static_cast<int64_t>(num_rows_dev[0]), rows_alloc) : rows_alloc;
+  const int chunks = cols / 8;
+  const int tid = threadIdx.x % TPR, sub = threadIdx.x / TPR;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int first_warp = sub * kWarps;
+  for (int64_t row0 = blockIdx.x * static_cast<int64_t>(kRows); row0 < rows; row0 += gridDim.x * static_cast<int64_t>(kRows)) {
+    const int64_t row = row0 + sub;
+    const bool on = row < rows;
+    const uint4* xrow = reinterpret_cast<const uint4*>(x + (on ? row : 0) * cols);
+    uint4 raw[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int c = tid + u * TPR;
+      raw[u] = on && c < chunks ? xrow[c] : make_uint4(0u, 0u, 0u, 0u);
+    }
+    uint32_t bits = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) bits = max(bits, amax_bits8(raw[u]));
+    bits = __reduce_max_sync(0xffffffffu, bits);
+    if constexpr (kWarps > 1) {
+      if (lane == 0) warp_bits[warp] = bits;
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) bits = max(bits, warp_bits[first_warp + w]);
+    }
+    const bool special = bits >= inf_bits<T>();   // the same for all threads of a row
+    float amax = 0.f;
+    if (special) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const T* e = reinterpret_cast<const T*>(&raw[u]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float v = fabsf(to_f32<T>(e[j]));
+          amax = fmaxf(amax, v != v ? 0.f : isinf(v) ? 448.f : v);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    } else {
+      amax = from_bits16<T>(bits);
+    }
+    if constexpr (kWarps > 1) {
+      if (lane == 0) warp_max[warp] = amax;   // every row of the block passes here: the barrier is the block's
+      __syncthreads();
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) amax = fmaxf(amax, warp_max[first_warp + w]);
+    }
+    float sc = __fdiv_rn(amax, 448.f);
+    if (sc == 0.f) sc = 1.f;
+    const bool rare = special || ((__float_as_uint(sc) & 0x7fffffu) == 0x7fffffu) || amax < 1e-20f;
+    const float rc = __frcp_rn(sc);
+    if (on) {
+      uint2* qrow = reinterpret_cast<uint2*>(q + row * cols);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int c = tid + u * TPR;
+        if (c < chunks) qrow[c] = quant8<T>(raw[u], sc, rc, rare);
+      }
+      if (tid == 0) scale[row] = sc;
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 quant_pertoken_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale,
@@ -475,6 +590,30 @@ quant_pertoken_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* _
     if (lane == 0) scale[row] = sc;
   }
 }
+
+// Threads per row: the fewest that hold it, then more while the rows alone leave SMs without warps and
+// every thread keeps two chunks; rows of more than 16384 values take the two-pass kernel.
+template <typename T>
+static void launch_quant_pertoken(const T* x, uint8_t* q, float* scale, const int* num_rows_dev, int64_t rows, int cols,
+                                  int sms, cudaStream_t st) {
+  const int chunks = cols / 8;
+  auto grid = [&](int rows_per_block) {
+    const int64_t need = (rows + rows_per_block - 1) / rows_per_block;
+    return static_cast<int>(need < static_cast<int64_t>(sms) * 16 ? need : static_cast<int64_t>(sms) * 16);
+  };
+  int tpr = 32;
+  while (tpr < 256 && (chunks > 8 * tpr || (rows * tpr < static_cast<int64_t>(sms) * 1024 && chunks >= 4 * tpr))) tpr *= 2;
+  if (chunks > 8 * tpr)
+    quant_pertoken_kernel<T><<<grid(8), 256, 0, st>>>(x, q, scale, num_rows_dev, rows, cols);
+  else if (tpr == 32)
+    quant_pertoken_row_kernel<T, 32><<<grid(8), 256, 0, st>>>(x, q, scale, num_rows_dev, rows, cols);
+  else if (tpr == 64)
+    quant_pertoken_row_kernel<T, 64><<<grid(4), 256, 0, st>>>(x, q, scale, num_rows_dev, rows, cols);
+  else if (tpr == 128)
+    quant_pertoken_row_kernel<T, 128><<<grid(2), 256, 0, st>>>(x, q, scale, num_rows_dev, rows, cols);
+  else
+    quant_pertoken_row_kernel<T, 256><<<grid(1), 256, 0, st>>>(x, q, scale, num_rows_dev, rows, cols);
+}
 }  // namespace flyb200
 
 extern "C" int flyb200_quant_pertoken(const void* x, void* q, float* scale, const int32_t* num_rows_dev,
@@ -489,16 +628,12 @@ extern "C" int flyb200_quant_pertoken(const void* x, void* q, float* scale, cons
   if (rows == 0) return FLYB200_OK;
   const int sms = sm_count();
   if (sms <= 0) return FLYB200_ERR_CUDA;
-  int64_t blocks = (rows + 7) / 8;
-  if (blocks > static_cast<int64_t>(sms) * 16) blocks = static_cast<int64_t>(sms) * 16;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   uint8_t* qo = static_cast<uint8_t*>(q);
   if (in_dtype == FLYB200_BF16)
-    quant_pertoken_kernel<__nv_bfloat16><<<static_cast<int>(blocks), 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(x), qo, scale, num_rows_dev, rows, cols);
+    launch_quant_pertoken(static_cast<const __nv_bfloat16*>(x), qo, scale, num_rows_dev, rows, cols, sms, st);
   else
-    quant_pertoken_kernel<__half><<<static_cast<int>(blocks), 256, 0, st>>>(static_cast<const __half*>(x), qo,
-                                                                            scale, num_rows_dev, rows, cols);
+    launch_quant_pertoken(static_cast<const __half*>(x), qo, scale, num_rows_dev, rows, cols, sms, st);
   FLYB200_CUDA_CHECK(cudaGetLastError());
   return FLYB200_OK;
 }
@@ -509,9 +644,9 @@ namespace flyb200 {
 template <typename T>
 __global__ void __launch_bounds__(256)
 quant_1x128_devrows_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale_t,
-                           const int* __restrict__ num_rows_dev, int64_t rows_alloc, int cols) {
+                           const int* __restrict__ num_rows_dev, int64_t rows_alloc, int cols, int parts) {
   const int64_t rows = min(static_cast<int64_t>(num_rows_dev[0]), rows_alloc);
-  quant_rows16<T>(x, q, scale_t, rows, rows_alloc, cols);
+  quant_rows16<T>(x, q, scale_t, rows, rows_alloc, cols, parts);
 }
 }  // namespace flyb200
 
@@ -530,12 +665,13 @@ extern "C" int flyb200_quant_1x128_devrows(const void* x, void* q, float* scale_
   if (sms <= 0) return FLYB200_ERR_CUDA;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   uint8_t* qo = static_cast<uint8_t*>(q);
+  const int parts = quant_parts(rows_alloc, cols, sms);
   if (in_dtype == FLYB200_BF16)
     quant_1x128_devrows_kernel<__nv_bfloat16><<<sms * 16, 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(x), qo, scale_t, num_rows_dev, rows_alloc, cols);
+        static_cast<const __nv_bfloat16*>(x), qo, scale_t, num_rows_dev, rows_alloc, cols, parts);
   else
-    quant_1x128_devrows_kernel<__half><<<sms * 16, 256, 0, st>>>(static_cast<const __half*>(x), qo,
-                                                                 scale_t, num_rows_dev, rows_alloc, cols);
+    quant_1x128_devrows_kernel<__half><<<sms * 16, 256, 0, st>>>(
+        static_cast<const __half*>(x), qo, scale_t, num_rows_dev, rows_alloc, cols, parts);
   FLYB200_CUDA_CHECK(cudaGetLastError());
   return FLYB200_OK;
 }
