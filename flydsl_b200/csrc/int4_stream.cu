@@ -17,15 +17,15 @@
 //   * warp 8 (one thread): ring of slots, each = one packed 128 x 128 group (8 KB, one bulk copy)
 //     + the tokens' 128 K columns (two TMA tiles of 64 K, 128-byte swizzle); group scales of the whole
 //     K range in one go.
-//   * warps 0-7: warp w owns weight rows [16w, 16w+16) = two n-blocks of mma.m16n8k16 (tokens are
+//   * warps 0-15 (0-7 beyond 32 tokens): warp w owns weight rows [16 (w % 8), +16) = two n-blocks of mma.m16n8k16 (tokens are
 //     the M=16 side). Per group: 8 x 16-byte loads of its rows' packed words (the four threads of a
 //     quad read the same row: a broadcast), per K step one ldmatrix.x4 of the token fragment and two
 //     MMAs into a per-group accumulator, then acc += group_sum * scale[n][group] in fp32 -- the same
 //     promotion structure as the block-scale kernels: equals dequantise-then-matmul with the products
-//     q*a summed in fp32 before scaling. (The template also builds with four n-blocks per warp and
-//     with the K steps of a group dealt out to two or four warps; neither was faster.)
+//     q*a summed in fp32 before scaling. Warps 8-15 take every other group; their sums are added
+//     once, before the exchange.
 //
-// Where the time goes (ncu, M=16, N=K=8192): the schedulers issue on 43 % of the cycles, the integer
+// Where the time goes with eight warps (ncu, M=16, N=K=8192): the schedulers issue on 43 % of the cycles, the integer
 // ALU pipe is the busiest at 41 %, the legacy tensor pipe 22 %, DRAM 17 %: the unpack instructions
 // (three per two weights) bound the kernel at ~960 cycles per 8 KB group against ~330 for the SM's
 // share of HBM bandwidth.
@@ -41,8 +41,8 @@
 
 namespace flyb200 {
 
-// consumer warps: 16 / NB row groups (NB n-blocks of 8 weight rows each) x KS parts of each group's
-// K steps; + one producer warp
+// consumer warps: KS sets, each taking every KS-th group, of 16 / NB row groups (NB n-blocks of 8 weight
+// rows each); + one producer warp
 constexpr int s4_threads(int nb, int ks) { return 32 * ((16 / nb) * ks + 1); }
 constexpr int kS4MaxSlots = 16;
 constexpr int kS4PackedBytes = 128 * 64;
@@ -97,8 +97,8 @@ int4_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const Int4StreamP
   using C = S4Cfg<MB>;
   constexpr int kRowGroups = 16 / NB;
   constexpr int kConsumers = kRowGroups * KS;
-  constexpr int kSteps = 8 / KS;      // K steps of a group per consumer warp
-  constexpr int kWords = 16 / KS;     // packed words of a row per consumer warp
+  constexpr int kSteps = 8;           // K steps of a group
+  constexpr int kWords = 16;          // packed words of a row
   extern __shared__ uint8_t smem_raw[];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -132,7 +132,7 @@ int4_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const Int4StreamP
   if (warp == 0) {
     if (lane < slots) {
       mbar_init(full_bar(lane), 1);
-      mbar_init(empty_bar(lane), kConsumers);
+      mbar_init(empty_bar(lane), kRowGroups);   // a group is consumed by one warp of each row group
     }
     if (lane == 0) {
       mbar_init(recv_bar, 1);
@@ -197,7 +197,7 @@ int4_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const Int4StreamP
     const int gid = lane >> 2, tig = lane & 3;
     const uint32_t sh = 4u * tig;
     const int wr = warp % kRowGroups;   // row group: weight rows [8 NB wr, 8 NB (wr + 1))
-    const int kh = warp / kRowGroups;   // which part of every group's K steps
+    const int kh = warp / kRowGroups;   // this warp takes every KS-th group, from group kh on
     float acc[MB][NB][4];
 #pragma unroll
     for (int mb = 0; mb < MB; ++mb)
@@ -220,7 +220,7 @@ int4_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const Int4StreamP
 #pragma unroll
     for (int a = 0; a < 4; ++a)
       lm_off[a] = static_cast<uint32_t>(lm_row * 128 + (((2 * a + lm_chunk) ^ (lane & 7)) << 4));
-    for (int i = 0; i < count && alive; ++i) {
+    for (int i = kh; i < count && alive; i += KS) {
       const int s = i % slots;
       const bool got = mbar_wait(full_bar(s), (i / slots) & 1, abort_flag, p.err, kErrWaitSmemFull);
       if (!__all_sync(0xffffffffu, got)) {
@@ -239,7 +239,7 @@ int4_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const Int4StreamP
         for (int v = 0; v < kWords / 4; ++v)
           asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(w[nb][4 * v]), "=r"(w[nb][4 * v + 1]), "=r"(w[nb][4 * v + 2]), "=r"(w[nb][4 * v + 3])
-                       : "r"(blk + 128u * (kh * (kWords / 4) + v)));
+                       : "r"(blk + 128u * v));
       }
       float tmp[MB][NB][4];
 #pragma unroll
@@ -250,8 +250,7 @@ int4_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const Int4StreamP
           for (int e = 0; e < 4; ++e) tmp[mb][nb][e] = 0.f;
       const uint32_t xs = base + kS4PackedBytes;
 #pragma unroll
-      for (int kl = 0; kl < kSteps; ++kl) {
-        const int ks = kh * kSteps + kl;
+      for (int ks = 0; ks < kSteps; ++ks) {
         uint32_t a[MB][4];
 #pragma unroll
         for (int mb = 0; mb < MB; ++mb) {
@@ -259,8 +258,8 @@ int4_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const Int4StreamP
         }
 #pragma unroll
         for (int nb = 0; nb < NB; ++nb) {
-          const uint32_t b0 = dq_pair(w[nb][2 * kl] >> sh);
-          const uint32_t b1 = dq_pair(w[nb][2 * kl + 1] >> sh);
+          const uint32_t b0 = dq_pair(w[nb][2 * ks] >> sh);
+          const uint32_t b1 = dq_pair(w[nb][2 * ks + 1] >> sh);
 #pragma unroll
           for (int mb = 0; mb < MB; ++mb) mma_bf16_16816(tmp[mb][nb], a[mb], b0, b1);
         }
@@ -292,7 +291,7 @@ int4_stream_kernel(const __grid_constant__ CUtensorMap tmap_x, const Int4StreamP
     consumer_sync();
     float* send = reinterpret_cast<float*>(smem_al);
 #pragma unroll
-    for (int part = 0; part < KS; ++part) {   // the warps of K part 0 write, those of part 1 add
+    for (int part = 0; part < KS; ++part) {   // the first set writes, the second adds
       if (kh == part) {
 #pragma unroll
         for (int mb = 0; mb < MB; ++mb)
@@ -450,11 +449,13 @@ int launch_int4_stream(void* c, const void* a, const void* wq, const void* scale
   const int rc = make_tensor_map_2d(&tmap, a, M, K, 2, 16 * plan.mb);
   if (rc) return rc;
   switch (plan.mb) {
-    // Eight consumer warps of two n-blocks each, every warp all K steps of a group: measured at
-    // M=16, N=K=8192 against 16 warps taking half the K steps each (21.5 / 23.5 us) and against four
-    // n-blocks per warp with two or four K parts (22.8 / 24.5 us).
-    case 1: return launch_int4_stream_mb<1, 2, 1>(tmap, p, stream);
-    case 2: return launch_int4_stream_mb<2, 2, 1>(tmap, p, stream);
+    // Two sets of eight consumer warps, each taking every other group: a group is a chain of shared
+    // loads, unpacking and MMAs that leaves a scheduler with two warps idle more than half of the time.
+    // M=16, N=K=8192: 21.0 -> 19.6 us a call (24.6 -> 22.5 us with cold caches). Sharing the K steps of
+    // a group out instead repeats the promotion and was slower than one set (23.5 against 21.5 us), as
+    // were four n-blocks per warp (22.8 / 24.5 us). 33 to 64 tokens: accumulators for one set only.
+    case 1: return launch_int4_stream_mb<1, 2, 2>(tmap, p, stream);
+    case 2: return launch_int4_stream_mb<2, 2, 2>(tmap, p, stream);
     default: return launch_int4_stream_mb<4, 2, 1>(tmap, p, stream);
   }
 }
