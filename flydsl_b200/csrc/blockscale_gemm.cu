@@ -1645,6 +1645,7 @@ static SplitPlan pick_split(int M, int N, int K, int sms, bool pertoken, int for
     const int bn = pertoken ? 256 : pick_block_n(m_blocks, N, sms, false);
     const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
     best = SplitPlan{bn, 1, kbt};
+    if (static_cast<long>(m_blocks) * cdiv(N, 256) * 2 > sms) return best;   // no room even for the widest tiles
     best_cost = ((tiles + sms - 1) / sms) * kbt * kb_ns(bn);
   }
   const int widths[3] = {256, 128, 64};

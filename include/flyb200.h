@@ -55,7 +55,9 @@ typedef struct flyb200_gemm_cfg {
                      * int4 GEMM: see flyb200_int4_gemm.
                      * MoE stages: bit 0 = activations already in routing order (TMA-fed),
                      *             bit 1 = stage-1 output in routing order                   */
-  int32_t split_k;  /* decode kernel: K splits per weight tile (cluster size, 1..8); 0 = auto    */
+  int32_t split_k;  /* decode kernel: K splits per weight tile (cluster size, 1..8); 0 = auto.
+                     * Dense GEMM with path 1: CTAs that share a tile's K range (0, 1 = none; up to 4
+                     * with 256-wide, 8 with narrower tiles; not with 32); path 0 chooses by size  */
 } flyb200_gemm_cfg;
 
 /* Weight repack [batch, N, K] (row-major fp8 bytes) -> per batch [K/128][N/8][8 rows][128 B], the
