@@ -1707,6 +1707,17 @@ static int dense_group_m(int M, int K) {
   return cdiv(M, BM) >= 2 * gm ? gm : 0;
 }
 
+// Wide decode shapes on the tiled kernel: with this many weight tiles it fills the GPU without split-K,
+// and a narrow tile's K block takes 0.25 us. Measured, decode against tiled kernel (us, graph replay, cold
+// weights): M = 16, N = 10240 (80 tiles of 128) K = 2048 9.1 / 9.4, K = 4096 13.7 / 14.3; N = 12288 (96)
+// 9.9 / 9.5, 15.0 / 14.3; N = 16384 11.0 / 10.1, 19.9 / 15.1. M = 32, N = 7168 (56) K = 1024 6.4 / 5.3, K =
+// 2048 8.7 / 7.7, K = 4096 11.9 / 11.6, K = 7168 16.9 / 17.2; N = 16384, K = 2048 12.5 / 10.3. (Block scales
+// only: the per-token tiles are 256 wide and lose to the decode kernel on such shapes.)
+static bool tiled_beats_decode(int M, int N, int K) {
+  const int n_tiles = cdiv(N, 128);
+  return n_tiles >= 96 || (M > 16 && M <= 32 && n_tiles >= 56 && K <= 4096);
+}
+
 extern "C" int flyb200_blockscale_gemm(void* c, const void* a, const void* b_repacked,
                                        const float* scale_a_t, const float* scale_b, int32_t M,
                                        int32_t N, int32_t K, int32_t out_dtype,
@@ -1730,7 +1741,8 @@ extern "C" int flyb200_blockscale_gemm(void* c, const void* a, const void* b_rep
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "cfg.path must be 0 (auto), 1 (tiled) or 2 (decode)");
   if (path == 2 && M > 64)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "the decode path takes M <= 64 (got %d)", M);
-  if (path == 2 || (path == 0 && M <= 64 && !(cfg && cfg->block_n) && decode_path_pays_off(M, N, K)))
+  if (path == 2 || (path == 0 && M <= 64 && !(cfg && cfg->block_n) && !tiled_beats_decode(M, N, K) &&
+                    decode_path_pays_off(M, N, K)))
     return launch_decode_gemm(c, a, b_repacked, scale_a_t, scale_b, M, N, K, out_dtype,
                               cfg ? cfg->split_k : 0, reinterpret_cast<cudaStream_t>(stream), false);
 

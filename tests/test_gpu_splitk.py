@@ -62,3 +62,26 @@ def test_split_k_pertoken(M, N, K):
     bound = _bound(out[0], a_q.float() * sa.view(M, 1), w.float() * sb.view(N, 1), K // 32 + 4)
     assert ((out[1] - out[0]).abs() <= bound).all()
     assert torch.equal(out[1], out[2])
+
+
+# Decode-size M on both sides of the line between the decode and the tiled kernel
+@pytest.mark.parametrize("M,N,K", [(1, 12288, 256), (16, 12272, 256), (16, 12160, 256), (17, 7168, 512), (32, 7056, 512),
+                                   (17, 7040, 512), (32, 7168, 4224)])
+def test_decode_or_tiled(M, N, K):
+    from flydsl_b200 import _lib
+    from flydsl_b200.kernels import compile_blockscale_preshuffle_gemm
+    from flydsl_b200.utils import shuffle_weight
+
+    case = O.make_dense_case(M, N, K, seed=M + N)
+    b = shuffle_weight(case["b_q"].cuda())
+    sa, sb = case["a_scale"].cuda().t().contiguous(), case["b_scale"].cuda().contiguous()
+    out = []
+    for path in ("auto", "tiled"):
+        fn = compile_blockscale_preshuffle_gemm(M=M, N=N, K=K, tile_m=64, tile_n=128, tile_k=128, out_dtype="fp16", path=path)
+        c = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+        fn(c, case["a_q"].cuda(), b, sa, sb, M, N, None)
+        assert _lib.query_device_error() == 0
+        out.append(c.float())
+    a = (case["a_q"].cuda().float().view(M, -1, 128) * case["a_scale"].cuda().unsqueeze(-1)).view(M, K)
+    w = case["b_q"].cuda().float() * O.expand_weight_scale(case["b_scale"].cuda(), N, K)
+    assert ((out[0] - out[1]).abs() <= _bound(out[1], a, w, K // 128 + 8)).all()
