@@ -361,13 +361,28 @@ struct S4Plan {
   int mb, ks, splits, kbps, slots;
 };
 
+// Sets of consumer warps (KS of the kernel) with `mb` blocks of 16 tokens: accumulators of 33 to 64 tokens
+// leave registers for one set only.
+static constexpr int s4_sets(int mb) { return mb <= 2 ? 2 : 1; }
+
+// Groups a ring may hold. A ring that wraps is a multiple of the sets deep, so that a slot's groups all
+// belong to one set: a warp then waits for every fill of the slots that it reads. With an odd ring and
+// two sets it waited for every other fill only, and a parity wait cannot tell a fill that has not landed
+// yet from the one two later.
+static int s4_ring(int slots, int kbps, int ks) {
+  if (slots > kS4MaxSlots) slots = kS4MaxSlots;
+  if (slots >= kbps) return kbps < 2 ? 2 : kbps;   // no wrap; the ring doubles as the send buffer of the exchange
+  slots -= slots % ks;
+  return slots < 2 ? 2 : slots;
+}
+
 // K splits (cluster size) and ring depth. One CTA streams kbps groups; the SMs' load is what counts
 // (two CTAs may share an SM when M <= 32), plus a fixed cost per wave and a little per split for the
 // exchange.
 static S4Plan plan_int4_stream(int M, int N, int K, int sms, int force_splits) {
   S4Plan best{0, 0, 0, 0, 0};
   const int mb = M <= 16 ? 1 : (M <= 32 ? 2 : 4);
-  const int ks = 1;
+  const int ks = s4_sets(mb);
   const int n_tiles = N / 128;
   const int KBt = K / 128;
   const int slot = kS4PackedBytes + 2 * 16 * mb * 128;
@@ -383,10 +398,7 @@ static S4Plan plan_int4_stream(int M, int N, int K, int sms, int force_splits) {
     // next launch are resident (and prefetching) while this one computes
     const int cps = mb <= 2 ? 2 : 1;
     const int fixed = (16 * mb + 8) * 512 + kbps * 256 + 2048;
-    int slots = (232448 / cps - 1024 - fixed) / slot;
-    if (slots > kS4MaxSlots) slots = kS4MaxSlots;
-    if (slots > kbps) slots = kbps;
-    if (slots < 2) slots = 2;   // the ring doubles as the send buffer of the exchange
+    const int slots = s4_ring((232448 / cps - 1024 - fixed) / slot, kbps, ks);
     if (slots * slot + fixed > 232448) continue;
     const long waves = (ctas + sms - 1) / sms;
     const double cost = static_cast<double>(per_sm) * kbps + 6.0 * waves + 0.5 * s_eff;
@@ -454,10 +466,20 @@ int launch_int4_stream(void* c, const void* a, const void* wq, const void* scale
     // M=16, N=K=8192: 21.0 -> 19.6 us a call (24.6 -> 22.5 us with cold caches). Sharing the K steps of
     // a group out instead repeats the promotion and was slower than one set (23.5 against 21.5 us), as
     // were four n-blocks per warp (22.8 / 24.5 us). 33 to 64 tokens: accumulators for one set only.
-    case 1: return launch_int4_stream_mb<1, 2, 2>(tmap, p, stream);
-    case 2: return launch_int4_stream_mb<2, 2, 2>(tmap, p, stream);
-    default: return launch_int4_stream_mb<4, 2, 1>(tmap, p, stream);
+    case 1: return launch_int4_stream_mb<1, 2, s4_sets(1)>(tmap, p, stream);
+    case 2: return launch_int4_stream_mb<2, 2, s4_sets(2)>(tmap, p, stream);
+    default: return launch_int4_stream_mb<4, 2, s4_sets(4)>(tmap, p, stream);
   }
 }
 
 }  // namespace flyb200
+
+extern "C" int flyb200_int4_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t sms, int32_t* plan) {
+  using namespace flyb200;
+  if (!plan || M < 1 || M > 64 || N < 128 || N % 128 || K < 128 || K % 128)
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_plan: bad arguments (M=%d N=%d K=%d)", M, N, K);
+  if (sms <= 0 && (sms = sm_count()) <= 0) return FLYB200_ERR_CUDA;
+  const S4Plan p = plan_int4_stream(M, N, K, sms, split_k);
+  plan[0] = p.mb; plan[1] = p.ks; plan[2] = p.splits; plan[3] = p.kbps; plan[4] = p.slots;
+  return FLYB200_OK;
+}

@@ -358,6 +358,12 @@ int flyb200_int4_repack(const int8_t* q, const void* scales, int32_t N, int32_t 
 int flyb200_int4_gemm(void* c, const void* a, const void* wq, const void* scales_t, int32_t M, int32_t N,
                       int32_t K, const flyb200_gemm_cfg* cfg, void* stream);
 
+/* What the mma.sync kernel of flyb200_int4_gemm (path 1) plans for a problem on a GPU of `sms` SMs (0 =
+ * the current device): plan[0] blocks of 16 tokens, [1] sets of consumer warps (set s takes groups s, s +
+ * sets, ... of the CTA's K range), [2] CTAs per cluster (K splits), [3] K groups per CTA, [4] ring slots.
+ * Host only; split_k as in the cfg. */
+int flyb200_int4_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t sms, int32_t* plan);
+
 /* Masked top-k reduce of the local experts' route rows (the arithmetic of flyb200_moe_reduce with a
  * valid_mask) whose result rows go straight into the owners' memory: row i of routes' [W*T, k, H]
  * belongs to source rank i / T, slot i % T and is stored at row rank*T + slot of that rank's back area

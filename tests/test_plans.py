@@ -1,0 +1,33 @@
+"""Launch plans over ranges of sizes. Host code: no GPU is needed."""
+import ctypes
+
+import pytest
+
+SMS = 148
+
+
+def _int4_plan(M, N, K, split_k):
+    from flydsl_b200 import _lib
+
+    plan = (ctypes.c_int32 * 5)()
+    _lib.check(_lib.load().flyb200_int4_plan(M, N, K, split_k, SMS, plan))
+    return tuple(plan)
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("split_k", [0, 1, 3, 8])
+def test_int4_ring_slots_belong_to_one_set(M, split_k):
+    """A consumer warp waits for the fills of the groups that its set takes. Parity waits are sound only
+    if it sees every fill of a slot, so no slot may hold groups of two sets."""
+    wrapped = 0
+    for N in range(128, 16385, 384):
+        for K in range(128, 16385, 128):
+            _, sets, splits, groups, slots = _int4_plan(M, N, K, split_k)
+            if splits == 0:   # no plan: the call is refused
+                continue
+            assert sets == (2 if M <= 32 else 1) and 2 <= slots <= 16
+            owner = {}
+            for g in range(groups):
+                assert owner.setdefault(g % slots, g % sets) == g % sets, (N, K, sets, groups, slots)
+            wrapped += groups > slots
+    assert wrapped > 100
