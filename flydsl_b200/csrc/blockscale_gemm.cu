@@ -1086,7 +1086,7 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         cluster_wait();
         exchanged = true;
         fence_proxy_async_smem();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (!epi_sync()) { alive = false; break; }   // bounded: a warp that gave up never comes here
         constexpr uint32_t kRecvOff = BM * kRowBytes;   // receive area: [sender, own rank left out][row of the slice]
         if (ew < p.splits && ew != split && lane == 0) {   // one copy per owner, each from a warp of its own
           const int lo = ew * rps;

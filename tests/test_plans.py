@@ -31,3 +31,25 @@ def test_int4_ring_slots_belong_to_one_set(M, split_k):
                 assert owner.setdefault(g % slots, g % sets) == g % sets, (N, K, sets, groups, slots)
             wrapped += groups > slots
     assert wrapped > 100
+
+
+def _kernel_source(name):
+    import os
+    import re
+
+    from flydsl_b200 import build
+
+    text = open(os.path.join(build.CSRC, name)).read()
+    return re.sub(r"//[^\n]*", "", text)
+
+
+@pytest.mark.parametrize("name", ["blockscale_gemm.cu", "moe_swap.cu", "pt_pair_gemm.cu"])
+def test_roles_that_may_give_up_meet_at_bounded_barriers_only(name):
+    """In these kernels a warp whose bounded wait runs out leaves its loop at once, so nobody may wait for
+    it at a named hardware barrier, which has no limit (decode_gemm.cu, int4_gemm.cu and int4_stream.cu send
+    the warps that gave up through theirs). __syncthreads is reached by every warp on every path."""
+    import re
+
+    source = _kernel_source(name)
+    assert "mbar_wait" in source
+    assert not re.search(r"\bbar(rier)?\.(cta\.)?sync", source)
