@@ -310,6 +310,11 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   const uint32_t cfree_bar = bar_base + 8u * (kNumBars - 1);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(misc + 1024 + 8 * kNumBars);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 1024 + 8 * kNumBars + 4);
+  // a role gave up: time for the copies that are still in flight to land in shared memory
+  auto drain_if_aborted = [&]() {
+    if (__any_sync(0xffffffffu, *abort_flag != 0))
+      for (int i = 0; i < 200; ++i) __nanosleep(1000);
+  };
   // wait until the stage that iteration `it` is about to overwrite has been consumed
   auto wait_stage_free = [&](uint32_t it, int code) -> bool {
     if (it < static_cast<uint32_t>(kStages)) return true;
@@ -1406,19 +1411,21 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   if constexpr (SPLIT) {
     __syncwarp();
     if (warp < kEpiWarp0) cluster_sync_all();   // (exchange barrier, see the epilogue)
-    // nobody leaves before every copy that reads its shared memory has landed: owners arrive after
-    // their receive barrier
+    // Nobody leaves before every copy that reads its shared memory has landed: owners arrive after
+    // their receive barrier, and an owner that gave up after a pause in which the copies sent to it
+    // land (they are issued right after the exchange barrier, which it has passed).
+    drain_if_aborted();
     cluster_sync_all();
   }
 
   // ---------------- teardown ----------------
   tc_fence_before();
   __syncthreads();
-  if (*abort_flag) {
-    // A role gave up: let copies that are still in flight land before the CTA's shared memory and
-    // TMEM are handed back.
-    for (int i = 0; i < 200; ++i) __nanosleep(1000);
-    __syncthreads();
+  if constexpr (!SPLIT) {   // before the CTA's shared memory and TMEM are handed back
+    if (*abort_flag) {
+      drain_if_aborted();
+      __syncthreads();
+    }
   }
   if (warp == 1) {
     tc_fence_after();

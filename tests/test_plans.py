@@ -53,3 +53,13 @@ def test_roles_that_may_give_up_meet_at_bounded_barriers_only(name):
     source = _kernel_source(name)
     assert "mbar_wait" in source
     assert not re.search(r"\bbar(rier)?\.(cta\.)?sync", source)
+
+
+def test_split_k_cta_that_gave_up_outlives_the_copies_sent_to_it():
+    """A sender leaves once every CTA of its cluster has arrived at the last cluster barrier, and its copies
+    read its shared memory until they land. So an owner that no longer waits for them (it gave up) has to
+    pause before that barrier: behind it the sender may be gone."""
+    source = _kernel_source("blockscale_gemm.cu")
+    end = source[source.index("if (warp < kEpiWarp0) cluster_sync_all();"):]
+    end = end[:end.index("__syncthreads();")]
+    assert end.index("drain_if_aborted();") < end.rindex("cluster_sync_all();")
