@@ -86,6 +86,7 @@ SIGNATURES = {
     "flyb200_ep_reduce_push": (c_int, [c_void_p, c_void_p, c_void_p, c_int64] + [c_int32] * 6 + [c_void_p]),
     "flyb200_int4_repack": (c_int, [c_void_p, c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_void_p]),
     "flyb200_int4_gemm": (c_int, [c_void_p] * 4 + [c_int32] * 3 + [POINTER(GemmCfg), c_void_p]),
+    "flyb200_gemm_plan": (c_int, [c_int32] * 4 + [POINTER(GemmCfg), c_int32, POINTER(c_int32)]),
     "flyb200_int4_plan": (c_int, [c_int32] * 5 + [POINTER(c_int32)]),
     "flyb200_query_device_error": (c_int, [c_void_p, POINTER(c_int32)]),
     "flyb200_last_error_string": (c_char_p, []),

@@ -1641,7 +1641,7 @@ static int max_clusters(int splits) {
 struct SplitPlan {
   int bn, splits, kbps;
 };
-static SplitPlan pick_split(int M, int N, int K, int sms, bool pertoken, int force_bn, int force_splits) {
+static SplitPlan pick_split(int M, int N, int K, int sms, bool live, bool pertoken, int force_bn, int force_splits) {
   const int m_blocks = cdiv(M, BM), kbt = K / BK;
   const int rows = M < BM ? M : BM;
   // per-token scales: no promotion per K block, 256-wide tiles at the tensor core's pace
@@ -1664,7 +1664,7 @@ static SplitPlan pick_split(int M, int N, int K, int sms, bool pertoken, int for
       if (force_splits && sp != force_splits) continue;
       const int kbps = cdiv(kbt, sp);
       if (cdiv(kbt, kbps) != sp) continue;           // some CTA would have no K block
-      if (!force_splits && (tiles * sp > sms || tiles > max_clusters(sp))) continue;
+      if (!force_splits && (tiles * sp > sms || tiles > (live ? max_clusters(sp) : sms / sp))) continue;
       const double exchange = 3000.0 + rows * bn * 4.0 * (sp - 1) / sp / 20.0;
       const double cost = kbps * kb_ns(bn) + exchange;
       if (cost < best_cost - 1e-9) {
@@ -1687,7 +1687,7 @@ static int check_ptr(const void* p, size_t align, const char* name) {
 int launch_decode_gemm(void* c, const void* a, const void* b_repacked, const float* scale_a_t,
                        const float* scale_b, int M, int N, int K, int out_dtype, int force_splits,
                        cudaStream_t stream, bool pertoken);
-bool decode_path_pays_off(int M, int N, int K);
+bool decode_path_pays_off(int M, int N, int K, int sms);
 // moe_swap.cu
 int launch_moe_swap(int stage, bool pertoken, void* out, const void* act, const void* w_repacked,
                     const float* scale_x, const float* scale_w, const int32_t* sorted_ids, const int32_t* expert_ids,
@@ -1725,6 +1725,133 @@ static bool tiled_beats_decode(int M, int N, int K) {
   return n_tiles >= 96 || (M > 16 && M <= 32 && n_tiles >= 56 && K <= 4096);
 }
 
+// What a dense call launches.
+struct DensePlan {
+  int kernel;   // cfg.path of that kernel: 1 tiled, 2 decode, 3 CTA pairs
+  int bn;       // tiled: tile width, CTAs that share a tile's K range, K blocks of each, grid
+  int splits, kbps, grid;
+};
+
+static int check_dense(bool pertoken, int M, int N, int K, const flyb200_gemm_cfg* cfg) {
+  if (M < 1 || N < 16 || K < 128)
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "bad shape M=%d N=%d K=%d", M, N, K);
+  if (N % 16) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "N (%d) must be a multiple of 16", N);
+  if (K % 128) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "K (%d) must be a multiple of 128", K);
+  const int path = cfg ? cfg->path : 0;
+  if (pertoken && cfg && cfg->block_n && cfg->block_n != 256)
+    return set_error(FLYB200_ERR_UNSUPPORTED, "the per-token-scale GEMM is built with 256-wide tiles only");
+  if (path < 0 || path > (pertoken ? 3 : 2))
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, pertoken
+                         ? "cfg.path must be 0 (auto), 1 (tiled), 2 (decode) or 3 (CTA pairs)"
+                         : "cfg.path must be 0 (auto), 1 (tiled) or 2 (decode)");
+  if (path == 2 && M > 64)
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "the decode path takes M <= 64 (got %d)", M);
+  if (path == 3 && (M < 256 || N % 256))
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "the CTA-pair path takes M >= 256 and N %% 256 == 0");
+  return FLYB200_OK;
+}
+
+// The kernel for a call that check_dense has passed. `live`: sms are those of the current device, which is
+// asked how many clusters it holds; otherwise that number is estimated.
+static DensePlan plan_dense(bool pertoken, int M, int N, int K, const flyb200_gemm_cfg* cfg, int sms, bool live) {
+  const int path = cfg ? cfg->path : 0, block_n = cfg ? cfg->block_n : 0;
+  const int max_ctas = cfg ? cfg->max_ctas : 0, split_k = cfg ? cfg->split_k : 0;
+  DensePlan plan{1, 0, 1, K / BK, 0};
+  // Decode-size M: the swap-AB split-K kernel (decode_gemm.cu; per-token: the token's scale on every K
+  // block, the channel's once), unless a tile width or the tiled path was asked for, or the shape is
+  // wide and nothing was asked for that the tiled kernel would not honour.
+  const bool wide = !pertoken && !split_k && !max_ctas && tiled_beats_decode(M, N, K);
+  if (path == 2 || (path == 0 && M <= 64 && !block_n && !wide && decode_path_pays_off(M, N, K, sms))) {
+    plan.kernel = 2;
+    return plan;
+  }
+  // Large per-token problems: the CTA-pair kernel (256 x 256 tiles over two SMs, 32 KB stages), measured
+  // faster than the single-CTA tiles on every benchmarked shape from M = 1024 up (equal at 256-512).
+  if (path == 3 || (pertoken && path == 0 && M >= 1024 && N % 256 == 0 && !block_n)) {
+    plan.kernel = 3;
+    return plan;
+  }
+  const int m_blocks = cdiv(M, BM);
+  SplitPlan split{0, 1, K / BK};
+  if (path == 1 && split_k > 1 && block_n != 32) {
+    split = pick_split(M, N, K, sms, live, pertoken, pertoken ? 256 : block_n, split_k);
+    // a limit on the CTAs comes before the split: its clusters have no persistent loop
+    if (max_ctas > 0 && static_cast<long>(m_blocks) * cdiv(N, split.bn ? split.bn : 256) * split.splits > max_ctas)
+      split = SplitPlan{0, 1, K / BK};
+  } else if (path == 0 && !block_n && !max_ctas && !split_k) {
+    split = pick_split(M, N, K, sms, live, pertoken, pertoken ? 256 : 0, 0);
+  }
+  plan.splits = split.splits;
+  plan.kbps = split.kbps;
+  plan.bn = pertoken ? 256 : block_n ? block_n : split.splits > 1 ? split.bn : pick_block_n(m_blocks, N, sms, false);
+  const long tiles = static_cast<long>(m_blocks) * cdiv(N, plan.bn);
+  plan.grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
+  if (split.splits > 1) plan.grid = static_cast<int>(tiles * split.splits);
+  else if (tiles < plan.grid) plan.grid = static_cast<int>(tiles);
+  return plan;
+}
+
+extern "C" int flyb200_gemm_plan(int32_t pertoken, int32_t M, int32_t N, int32_t K, const flyb200_gemm_cfg* cfg,
+                                 int32_t sms, int32_t* out) {
+  if (!out) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "gemm_plan: NULL buffer");
+  const int rc = check_dense(pertoken != 0, M, N, K, cfg);
+  if (rc) return rc;
+  const bool live = sms <= 0;
+  if (live && (sms = sm_count()) <= 0) return FLYB200_ERR_CUDA;
+  const DensePlan plan = plan_dense(pertoken != 0, M, N, K, cfg, sms, live);
+  out[0] = plan.kernel; out[1] = plan.bn; out[2] = plan.splits; out[3] = plan.kbps; out[4] = plan.grid;
+  return FLYB200_OK;
+}
+
+// The two dense GEMMs. scale_a: [K/128, M], per token [M]; scale_b: [ceil(N/128), K/128], per token [N].
+static int dense_gemm(bool pertoken, void* c, const void* a, const void* b_repacked, const float* scale_a,
+                      const float* scale_b, int M, int N, int K, int out_dtype, const flyb200_gemm_cfg* cfg,
+                      cudaStream_t st) {
+  int rc = check_dense(pertoken, M, N, K, cfg);
+  if (rc) return rc;
+  const int sms = sm_count();
+  if (sms <= 0) return FLYB200_ERR_CUDA;
+  const DensePlan plan = plan_dense(pertoken, M, N, K, cfg, sms, true);
+  if (plan.kernel == 2)
+    return launch_decode_gemm(c, a, b_repacked, scale_a, scale_b, M, N, K, out_dtype, cfg ? cfg->split_k : 0, st,
+                              pertoken);
+  if (plan.kernel == 3)
+    return launch_pertoken_pair_gemm(c, a, b_repacked, scale_a, scale_b, M, N, K, out_dtype,
+                                     cfg ? cfg->max_ctas : 0, dense_group_m(M, K), st);
+  GemmParams p{};
+  p.a = reinterpret_cast<const uint8_t*>(a);
+  p.b = reinterpret_cast<const uint8_t*>(b_repacked);
+  p.scale_a = scale_a;
+  p.scale_b = scale_b;
+  p.out = c;
+  p.err = device_error_word();
+  if (!p.err) return FLYB200_ERR_CUDA;
+  p.M = M; p.N = N; p.K = K;
+  p.group_m = dense_group_m(M, K);
+  // Small M: bring only as many rows as exist (rounded up to the 8-row swizzle atom).
+  p.a_box_rows = M >= BM ? BM : ((M + 7) / 8) * 8;
+  p.splits = plan.splits;
+  p.kbps = plan.kbps;
+
+  CUtensorMap tmap_a, tmap_c;
+  if ((rc = make_tensor_map_2d(&tmap_a, a, M, K, 1, p.a_box_rows))) return rc;
+  if ((rc = make_tensor_map_2d(&tmap_c, c, M, N, 2, p.a_box_rows))) return rc;
+  const bool bf16 = out_dtype == FLYB200_BF16;
+  if (plan.splits > 1) {
+    const int tiles = plan.grid / plan.splits;
+    if (pertoken)
+      return bf16 ? launch_split<256, kDensePT, __nv_bfloat16>(tmap_a, p, tiles, st)
+                  : launch_split<256, kDensePT, __half>(tmap_a, p, tiles, st);
+    return bf16 ? launch_split_bn<kDense, __nv_bfloat16>(plan.bn, tmap_a, p, tiles, st)
+                : launch_split_bn<kDense, __half>(plan.bn, tmap_a, p, tiles, st);
+  }
+  if (pertoken)
+    return bf16 ? launch<256, kDensePT, __nv_bfloat16>(tmap_a, tmap_c, p, plan.grid, st)
+                : launch<256, kDensePT, __half>(tmap_a, tmap_c, p, plan.grid, st);
+  return bf16 ? launch_bn<kDense, __nv_bfloat16>(plan.bn, tmap_a, tmap_c, p, plan.grid, st)
+              : launch_bn<kDense, __half>(plan.bn, tmap_a, tmap_c, p, plan.grid, st);
+}
+
 extern "C" int flyb200_blockscale_gemm(void* c, const void* a, const void* b_repacked,
                                        const float* scale_a_t, const float* scale_b, int32_t M,
                                        int32_t N, int32_t K, int32_t out_dtype,
@@ -1734,66 +1861,10 @@ extern "C" int flyb200_blockscale_gemm(void* c, const void* a, const void* b_rep
       (rc = check_ptr(b_repacked, 16, "b_repacked")) || (rc = check_ptr(scale_a_t, 4, "scale_a_t")) ||
       (rc = check_ptr(scale_b, 4, "scale_b")))
     return rc;
-  if (M < 1 || N < 16 || K < 128)
-    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "bad shape M=%d N=%d K=%d", M, N, K);
-  if (N % 16) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "N (%d) must be a multiple of 16", N);
-  if (K % 128) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "K (%d) must be a multiple of 128", K);
   if (out_dtype != FLYB200_BF16 && out_dtype != FLYB200_F16)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "out_dtype must be BF16 or F16");
-
-  // Decode-size M: the swap-AB split-K kernel (decode_gemm.cu), unless a tile width or the tiled
-  // path was asked for explicitly.
-  const int path = cfg ? cfg->path : 0;
-  if (path < 0 || path > 2)
-    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "cfg.path must be 0 (auto), 1 (tiled) or 2 (decode)");
-  if (path == 2 && M > 64)
-    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "the decode path takes M <= 64 (got %d)", M);
-  if (path == 2 || (path == 0 && M <= 64 && !(cfg && cfg->block_n) && !tiled_beats_decode(M, N, K) &&
-                    decode_path_pays_off(M, N, K)))
-    return launch_decode_gemm(c, a, b_repacked, scale_a_t, scale_b, M, N, K, out_dtype,
-                              cfg ? cfg->split_k : 0, reinterpret_cast<cudaStream_t>(stream), false);
-
-  const int sms = sm_count();
-  if (sms <= 0) return FLYB200_ERR_CUDA;
-  const int m_blocks = cdiv(M, BM);
-  SplitPlan plan{0, 1, K / BK};
-  if (path == 1 && cfg->split_k > 1 && cfg->block_n != 32)   // asked for: split if the plan exists
-    plan = pick_split(M, N, K, sms, false, cfg->block_n, cfg->split_k);
-  else if (path == 0 && !(cfg && (cfg->block_n || cfg->max_ctas || cfg->split_k)))
-    plan = pick_split(M, N, K, sms, false, 0, 0);
-  int bn = (cfg && cfg->block_n) ? cfg->block_n : plan.splits > 1 ? plan.bn : pick_block_n(m_blocks, N, sms, false);
-  int grid = sms;
-  if (cfg && cfg->max_ctas > 0 && cfg->max_ctas < grid) grid = cfg->max_ctas;
-  const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
-  if (tiles < grid) grid = static_cast<int>(tiles);
-
-  GemmParams p{};
-  p.a = reinterpret_cast<const uint8_t*>(a);
-  p.b = reinterpret_cast<const uint8_t*>(b_repacked);
-  p.scale_a = scale_a_t;
-  p.scale_b = scale_b;
-  p.out = c;
-  p.err = device_error_word();
-  if (!p.err) return FLYB200_ERR_CUDA;
-  p.M = M; p.N = N; p.K = K;
-  p.group_m = dense_group_m(M, K);
-  // Small M: bring only as many rows as exist (rounded up to the 8-row swizzle atom).
-  p.a_box_rows = M >= BM ? BM : ((M + 7) / 8) * 8;
-
-  CUtensorMap tmap_a, tmap_c;
-  if ((rc = make_tensor_map_2d(&tmap_a, a, M, K, 1, p.a_box_rows))) return rc;
-  if ((rc = make_tensor_map_2d(&tmap_c, c, M, N, 2, p.a_box_rows))) return rc;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  p.splits = plan.splits;
-  p.kbps = plan.kbps;
-  if (plan.splits > 1) {
-    if (out_dtype == FLYB200_BF16)
-      return launch_split_bn<kDense, __nv_bfloat16>(bn, tmap_a, p, static_cast<int>(tiles), st);
-    return launch_split_bn<kDense, __half>(bn, tmap_a, p, static_cast<int>(tiles), st);
-  }
-  if (out_dtype == FLYB200_BF16)
-    return launch_bn<kDense, __nv_bfloat16>(bn, tmap_a, tmap_c, p, grid, st);
-  return launch_bn<kDense, __half>(bn, tmap_a, tmap_c, p, grid, st);
+  return dense_gemm(false, c, a, b_repacked, scale_a_t, scale_b, M, N, K, out_dtype, cfg,
+                    reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int flyb200_pertoken_gemm(void* c, const void* a, const void* b_repacked, const float* scale_a,
@@ -1804,71 +1875,10 @@ extern "C" int flyb200_pertoken_gemm(void* c, const void* a, const void* b_repac
       (rc = check_ptr(b_repacked, 16, "b_repacked")) || (rc = check_ptr(scale_a, 4, "scale_a")) ||
       (rc = check_ptr(scale_b, 4, "scale_b")))
     return rc;
-  if (M < 1 || N < 16 || K < 128)
-    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "bad shape M=%d N=%d K=%d", M, N, K);
-  if (N % 16) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "N (%d) must be a multiple of 16", N);
-  if (K % 128) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "K (%d) must be a multiple of 128", K);
   if (out_dtype != FLYB200_BF16 && out_dtype != FLYB200_F16)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "out_dtype must be BF16 or F16");
-  if (cfg && cfg->block_n && cfg->block_n != 256)
-    return set_error(FLYB200_ERR_UNSUPPORTED, "the per-token-scale GEMM is built with 256-wide tiles only");
-  // Decode-size M: the swap-AB split-K kernel with the token's scale on every K block and the
-  // channel's scale applied once (cfg.path as for flyb200_blockscale_gemm).
-  const int path = cfg ? cfg->path : 0;
-  if (path < 0 || path > 3)
-    return set_error(FLYB200_ERR_INVALID_ARGUMENT,
-                     "cfg.path must be 0 (auto), 1 (tiled), 2 (decode) or 3 (CTA pairs)");
-  if (path == 2 && M > 64)
-    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "the decode path takes M <= 64 (got %d)", M);
-  if (path == 2 || (path == 0 && M <= 64 && !(cfg && cfg->block_n) && decode_path_pays_off(M, N, K)))
-    return launch_decode_gemm(c, a, b_repacked, scale_a, scale_b, M, N, K, out_dtype,
-                              cfg ? cfg->split_k : 0, reinterpret_cast<cudaStream_t>(stream), true);
-  // Large problems: the CTA-pair kernel (256 x 256 tiles over two SMs, 32 KB stages), measured faster
-  // than the single-CTA tiles on every benchmarked shape from M = 1024 up (equal at 256-512).
-  if (path == 3 && (M < 256 || N % 256))
-    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "the CTA-pair path takes M >= 256 and N %% 256 == 0");
-  if (path == 3 || (path == 0 && M >= 1024 && N % 256 == 0 && !(cfg && cfg->block_n))) {
-    return launch_pertoken_pair_gemm(c, a, b_repacked, scale_a, scale_b, M, N, K, out_dtype,
-                                     cfg ? cfg->max_ctas : 0, dense_group_m(M, K),
-                                     reinterpret_cast<cudaStream_t>(stream));
-  }
-  const int sms = sm_count();
-  if (sms <= 0) return FLYB200_ERR_CUDA;
-  const int m_blocks = cdiv(M, BM);
-  SplitPlan plan{256, 1, K / BK};
-  if (path == 1 && cfg->split_k > 1)
-    plan = pick_split(M, N, K, sms, true, 256, cfg->split_k);
-  else if (path == 0 && !(cfg && (cfg->block_n || cfg->max_ctas || cfg->split_k)))
-    plan = pick_split(M, N, K, sms, true, 256, 0);
-  int grid = sms;
-  if (cfg && cfg->max_ctas > 0 && cfg->max_ctas < grid) grid = cfg->max_ctas;
-  const long tiles = static_cast<long>(m_blocks) * cdiv(N, 256);
-  if (tiles < grid) grid = static_cast<int>(tiles);
-
-  GemmParams p{};
-  p.a = reinterpret_cast<const uint8_t*>(a);
-  p.b = reinterpret_cast<const uint8_t*>(b_repacked);
-  p.scale_a = scale_a;   // [M]
-  p.scale_b = scale_b;   // [N]
-  p.out = c;
-  p.err = device_error_word();
-  if (!p.err) return FLYB200_ERR_CUDA;
-  p.M = M; p.N = N; p.K = K;
-  p.group_m = dense_group_m(M, K);
-  p.a_box_rows = M >= BM ? BM : ((M + 7) / 8) * 8;
-  CUtensorMap tmap_a, tmap_c;
-  if ((rc = make_tensor_map_2d(&tmap_a, a, M, K, 1, p.a_box_rows))) return rc;
-  if ((rc = make_tensor_map_2d(&tmap_c, c, M, N, 2, p.a_box_rows))) return rc;
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  p.splits = plan.splits;
-  p.kbps = plan.kbps;
-  if (plan.splits > 1) {
-    if (out_dtype == FLYB200_BF16)
-      return launch_split<256, kDensePT, __nv_bfloat16>(tmap_a, p, static_cast<int>(tiles), st);
-    return launch_split<256, kDensePT, __half>(tmap_a, p, static_cast<int>(tiles), st);
-  }
-  if (out_dtype == FLYB200_BF16) return launch<256, kDensePT, __nv_bfloat16>(tmap_a, tmap_c, p, grid, st);
-  return launch<256, kDensePT, __half>(tmap_a, tmap_c, p, grid, st);
+  return dense_gemm(true, c, a, b_repacked, scale_a, scale_b, M, N, K, out_dtype, cfg,
+                    reinterpret_cast<cudaStream_t>(stream));
 }
 
 static int moe_common_checks(const void* out, const void* x, const void* w, const float* scale_x,

@@ -434,9 +434,8 @@ static int launch_decode(const CUtensorMap& tmap, const DecodeParams& p, int n_t
 // of its CTAs are resident at once (one wave) -- with more than 32 tokens only if K is deep enough
 // (>= 32 blocks) for split-K to matter; wide-N shapes that need several waves run faster on the
 // persistent tiled kernel.
-bool decode_path_pays_off(int M, int N, int K) {
-  const int sms = sm_count();
-  if (sms <= 0 || M > 64) return false;
+bool decode_path_pays_off(int M, int N, int K, int sms) {
+  if (M > 64) return false;
   const DecodePlan plan = plan_decode(M, N, K, sms, 0);
   if (plan.splits < 1 || plan.rounds != 1) return false;
   if (M > 32 && K / 128 < 32) return false;

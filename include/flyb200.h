@@ -57,7 +57,10 @@ typedef struct flyb200_gemm_cfg {
                      *             bit 1 = stage-1 output in routing order                   */
   int32_t split_k;  /* decode kernel: K splits per weight tile (cluster size, 1..8); 0 = auto.
                      * Dense GEMM with path 1: CTAs that share a tile's K range (0, 1 = none; up to 4
-                     * with 256-wide, 8 with narrower tiles; not with 32); path 0 chooses by size  */
+                     * with 256-wide, 8 with narrower tiles; not with 32). Not split where a CTA
+                     * would be left without K, or where max_ctas is set and smaller than the CTAs
+                     * that the split takes. Path 0 splits by size if no other field is set, and with
+                     * split_k set stays on the decode kernel where that is its choice          */
 } flyb200_gemm_cfg;
 
 /* Weight repack [batch, N, K] (row-major fp8 bytes) -> per batch [K/128][N/8][8 rows][128 B], the
@@ -89,6 +92,13 @@ int flyb200_blockscale_gemm(void* c, const void* a, const void* b_repacked, cons
 int flyb200_pertoken_gemm(void* c, const void* a, const void* b_repacked, const float* scale_a,
                           const float* scale_b, int32_t M, int32_t N, int32_t K, int32_t out_dtype,
                           const flyb200_gemm_cfg* cfg, void* stream);
+
+/* What the dense GEMMs (pertoken 0: flyb200_blockscale_gemm, else flyb200_pertoken_gemm) launch for a
+ * problem on a GPU of `sms` SMs (0 = the current device): plan[0] the kernel as in cfg.path (1 tiled, 2
+ * decode, 3 CTA pairs), and for the tiled kernel [1] tile width, [2] CTAs that share a tile's K range,
+ * [3] K blocks of 128 of each, [4] CTAs. Host only; the same checks as the call. */
+int flyb200_gemm_plan(int32_t pertoken, int32_t M, int32_t N, int32_t K, const flyb200_gemm_cfg* cfg, int32_t sms,
+                      int32_t* plan);
 
 /* MoE routing sort. Bit-exact stand-in for moe_sorting_torch_native
  * (tests/kernels/test_moe_gemm.py:97-161) and the sorter half of build_routing_buffers (:223-295).

@@ -63,3 +63,44 @@ def test_split_k_cta_that_gave_up_outlives_the_copies_sent_to_it():
     end = source[source.index("if (warp < kEpiWarp0) cluster_sync_all();"):]
     end = end[:end.index("__syncthreads();")]
     assert end.index("drain_if_aborted();") < end.rindex("cluster_sync_all();")
+
+
+def _gemm_plan(M, N, K, pertoken=False, sms=SMS, **cfg):
+    from flydsl_b200 import _lib
+
+    cfg = _lib.GemmCfg(*[cfg.get(name, 0) for name in ("block_n", "max_ctas", "path", "split_k")])
+    plan = (ctypes.c_int32 * 5)()
+    _lib.check(_lib.load().flyb200_gemm_plan(int(pertoken), M, N, K, ctypes.byref(cfg), sms, plan))
+    return dict(zip(("kernel", "block_n", "splits", "kbps", "ctas"), plan))
+
+
+TILED, DECODE, PAIR = 1, 2, 3
+
+
+def test_requests_of_the_caller_are_honoured():
+    wide = dict(M=16, N=16384, K=2048)
+    assert _gemm_plan(**wide)["kernel"] == TILED
+    # a cluster size or a limit on the CTAs was asked for: the route of these calls is the decode kernel
+    assert _gemm_plan(**wide, split_k=1)["kernel"] == DECODE
+    assert _gemm_plan(**wide, max_ctas=64)["kernel"] == DECODE
+    # the limit on the CTAs holds with a split as well
+    for pertoken in (False, True):
+        deep = dict(M=256, N=1024, K=8192, pertoken=pertoken, path=TILED, split_k=4)
+        free = _gemm_plan(**deep)
+        assert free["splits"] == 4 and free["ctas"] > 8
+        for limit in (1, 5, 8, free["ctas"] - 1, free["ctas"], 148, 1000):
+            plan = _gemm_plan(**deep, max_ctas=limit)
+            assert plan["ctas"] <= limit and (plan["splits"] == 4) == (limit >= free["ctas"])
+        assert _gemm_plan(256, 1024, 8192, pertoken, max_ctas=8)["ctas"] <= 8
+        # path 0 with some request made stays unsplit, as the tiled kernel always was then
+        assert _gemm_plan(256, 1024, 8192, pertoken)["splits"] > 1
+        assert _gemm_plan(256, 1024, 8192, pertoken, split_k=4)["splits"] == 1
+
+
+def test_plan_refuses_what_the_call_refuses():
+    bad = [dict(M=0, N=128, K=128), dict(M=1, N=8, K=128), dict(M=1, N=24, K=128), dict(M=1, N=128, K=192),
+           dict(M=65, N=128, K=128, path=DECODE), dict(M=1, N=128, K=128, path=4),
+           dict(M=1, N=128, K=128, path=PAIR), dict(M=255, N=256, K=128, path=PAIR, pertoken=True)]
+    for case in bad:
+        with pytest.raises(ValueError):
+            _gemm_plan(**case)
