@@ -118,8 +118,13 @@ struct Cfg {
   // and behind it one slice of rows from every other CTA of the cluster; kSplitMax CTAs fit.
   static constexpr int kSplitMax = BN == 256 ? 4 : 8;
   __host__ __device__ static constexpr int split_rows(int rows, int splits) { return (rows + splits - 1) / splits; }
-  static_assert(!SPLIT || BM * BN * 4 + (kSplitMax - 1) * split_rows(BM, kSplitMax) * BN * 4 <= kAvail,
-                "split-K exchange does not fit");
+  static constexpr int most_received() {   // rows, over all cluster sizes (seven slices of 19 are more than eight of 16)
+    int most = 0;
+    for (int s = 2; s <= kSplitMax; ++s)
+      if ((s - 1) * split_rows(BM, s) > most) most = (s - 1) * split_rows(BM, s);
+    return most;
+  }
+  static_assert(!SPLIT || (BM + most_received()) * BN * 4 <= kAvail, "split-K exchange does not fit");
   static constexpr int kRingBytes = SPLIT ? kAvail : kStages * kStageBytes;
   static constexpr int kSmemBytes = kRingBytes + kCBytes + kMiscBytes + 1024;
   static_assert(kStages >= 3, "pipeline too shallow");

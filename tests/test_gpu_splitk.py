@@ -4,6 +4,7 @@ import pytest
 import torch
 
 from oracle import blockscale_ref as O
+from tests.test_plans import DECODE, TILED, _gemm_plan
 
 pytestmark = pytest.mark.gpu
 
@@ -15,15 +16,25 @@ def _bound(ref, a, b, extra):
 
 
 # M: fewer rows than CTAs, one row in the last row block, slices of unequal length; N: a multiple of 16
-# only, fewer columns than a tile; K: one K block per CTA, a shorter last range
-@pytest.mark.parametrize("M,N,K", [(1, 512, 512), (7, 528, 1152), (129, 528, 2048), (300, 1040, 1152), (255, 256, 8320)])
-@pytest.mark.parametrize("block_n", [64, 128, 256])
-@pytest.mark.parametrize("split_k", [2, 3, 4, 8])
+# only, fewer columns than a tile; K: one K block per CTA, a shorter last range. Every cluster size the
+# automatic plan may choose, where each of its CTAs has K blocks.
+SHAPES = [(1, 512, 512), (7, 528, 1152), (129, 528, 896), (129, 528, 2048), (300, 1040, 1152), (255, 256, 8320)]
+
+
+def _splits(K, most):
+    blocks = K // 128
+    each = {s: -(-blocks // s) for s in range(2, most + 1)}
+    return [s for s in each if -(-blocks // each[s]) == s]
+
+
+@pytest.mark.parametrize("M,N,K,block_n,split_k", [(M, N, K, bn, s) for M, N, K in SHAPES for bn in (64, 128, 256)
+                                                   for s in _splits(K, 4 if bn == 256 else 8)])
 def test_split_k_matches_unsplit(M, N, K, block_n, split_k):
     from flydsl_b200 import _lib
     from flydsl_b200.kernels import compile_blockscale_preshuffle_gemm
     from flydsl_b200.utils import shuffle_weight
 
+    assert _gemm_plan(M, N, K, sms=0, block_n=block_n, path=TILED, split_k=split_k)["splits"] == split_k
     case = O.make_dense_case(M, N, K, seed=M + N + K)
     b = shuffle_weight(case["b_q"].cuda())
     sa, sb = case["a_scale"].cuda().t().contiguous(), case["b_scale"].cuda().contiguous()
@@ -48,6 +59,8 @@ def test_split_k_pertoken(M, N, K):
     from flydsl_b200.kernels import compile_preshuffle_gemm_a8
     from flydsl_b200.utils import quant_pertoken, shuffle_weight
 
+    assert _gemm_plan(M, N, K, pertoken=True, sms=0)["splits"] > 1
+    assert _gemm_plan(M, N, K, pertoken=True, sms=0, path=TILED)["splits"] == 1
     g = torch.Generator("cuda").manual_seed(M + N)
     a_q, sa = quant_pertoken(torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16))
     w = torch.randn(N, K, generator=g, device="cuda").to(torch.float8_e4m3fn)
