@@ -3,7 +3,8 @@
 The reference ships the two stage kernels and leaves the chaining to its test
 (tests/kernels/test_moe_blockscale.py:293-380): routing sort -> stage 1 -> 1x128 re-quantisation ->
 stage 2 (-> top-k reduce). ``BlockscaleMoE`` is that chain with persistent buffers, so a step
-launches kernels only (sort, gemm1, quant, gemm2[, reduce]) and allocates nothing after warm-up.
+launches kernels only (sort, gemm1, quant, gemm2[, reduce]) and allocates only the routing arrays after
+warm-up, and the result unless ``out`` is given (small blocks: see ``BlockscaleMoE._buffers``).
 """
 from __future__ import annotations
 
@@ -18,6 +19,9 @@ from .kernels.moe_blockscale_2stage import (
     compile_moe_reduction,
 )
 from .utils import moe_gather_rows, moe_sorting, quant_1x128, shuffle_weight
+
+# Scratch that one layer keeps for blocks of at most 32 rows, over all token counts (see _buffers).
+_KEPT_SMALL_BYTES = 256 << 20
 
 _DT_NAME = {torch.float16: "f16", torch.bfloat16: "bf16", torch.float32: "f32"}
 
@@ -87,6 +91,7 @@ class BlockscaleMoE:
         self.reduce = compile_moe_reduction(topk=self.topk, model_dim=self.H,
                                             dtype_str=_DT_NAME[out_dtype]) if mode == "reduce" else None
         self._buf = {}
+        self._kept_small = 0
 
     @classmethod
     def from_unpacked(cls, w1_q, w1_scale, w2_q, w2_scale, **kw):
@@ -94,13 +99,20 @@ class BlockscaleMoE:
         return cls(shuffle_weight(w1_q), w1_scale, shuffle_weight(w2_q), w2_scale, **kw)
 
     def _buffers(self, T: int, dev, in_order: Optional[bool] = None):
+        """Scratch for T tokens, kept by token count. The routing-order buffers of small blocks are mostly
+        padding (256 experts of 7168 x 2048: 63 MB for 32 tokens in blocks of 16, 170 MB for 256 in blocks of
+        32), and a server meets every batch size: they are kept up to _KEPT_SMALL_BYTES per layer, and beyond
+        that a call takes its own from torch's allocator (about 10 us on the host) and gives them back. Nothing
+        kept is ever freed or shared between token counts, so captured graphs and calls on other streams
+        find it as they left it."""
         in_order = self.sorted_layout if in_order is None else in_order
         key = (T, dev, in_order)
         b = self._buf.get(key)
         if b is None:
             # rows of padding positions are never written and never looked at, whatever they hold; the
             # layouts that a caller's routing can meet start out as zeros all the same
-            new = torch.empty if in_order and not self.sorted_layout else torch.zeros
+            small = in_order and not self.sorted_layout
+            new = torch.empty if small else torch.zeros
             # rows of the stage-1 output / stage-2 input: routes, or sorted positions incl. padding
             L = (T * self.topk + self.E * self.tile_m - self.topk) if in_order else T * self.topk
             b = {
@@ -115,6 +127,11 @@ class BlockscaleMoE:
                 "routes": torch.empty((T * self.topk, self.H), dtype=self.out_dtype, device=dev)
                 if self.mode == "reduce" else None,
             }
+            if small:
+                nbytes = sum(t.numel() * t.element_size() for t in b.values() if torch.is_tensor(t))
+                if self._kept_small + nbytes > _KEPT_SMALL_BYTES:
+                    return b
+                self._kept_small += nbytes
             self._buf[key] = b
         return b
 

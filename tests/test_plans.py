@@ -104,3 +104,28 @@ def test_plan_refuses_what_the_call_refuses():
     for case in bad:
         with pytest.raises(ValueError):
             _gemm_plan(**case)
+
+
+@pytest.mark.parametrize("mode", ["reduce", "atomic"])
+@pytest.mark.parametrize("tile_m", [8, 16, 32])
+def test_moe_layer_scratch_is_bounded_over_token_counts(tile_m, mode):
+    """A server's decode batches, every size from 1 to 512, on a layer of the benchmark's size."""
+    import torch
+
+    from flydsl_b200 import moe
+
+    def meta(*shape, dtype=torch.float8_e4m3fn):
+        return torch.empty(shape, dtype=dtype, device="meta")
+
+    E, H, I, topk, dev = 256, 7168, 2048, 8, torch.device("meta")
+    layer = moe.BlockscaleMoE(meta(E, 2 * I, H), meta(E, 2 * I // 128 * (H // 128), dtype=torch.float32),
+                              meta(E, H, I), meta(E, H // 128 * (I // 128), dtype=torch.float32), topk=topk,
+                              tile_m=tile_m, mode=mode)
+    for T in range(1, 513):
+        b = layer._buffers(T, dev, True)
+        rows = T * topk + E * tile_m - topk
+        assert b["rows"] == rows and b["x_sorted"].shape == (rows, H) and b["out1"].shape == (rows, I)
+    kept = sum(t.numel() * t.element_size() for b in layer._buf.values() for t in b.values() if torch.is_tensor(t))
+    assert 0 < kept <= moe._KEPT_SMALL_BYTES
+    first = layer._buffers(1, dev, True)
+    assert layer._buffers(1, dev, True) is first   # the sizes met first keep theirs
