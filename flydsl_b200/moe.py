@@ -148,7 +148,8 @@ class BlockscaleMoE:
         T = x_q.shape[0]
         dev = x_q.device
         dense_in = x_q.is_contiguous() and x_scale_t.is_contiguous()
-        small = self._small_stages is not None and routing is None and dense_in
+        small = (self._small_stages is not None and routing is None and dense_in
+                 and tuple(topk_ids.shape) == (T, self.topk))   # the fused permute takes no other routing
         gemm1, gemm2 = self._small_stages if small else (self.gemm1, self.gemm2)
         in_order = self.sorted_layout or small
         b = self._buffers(T, dev, in_order)

@@ -95,3 +95,29 @@ def test_more_blocks_than_the_list_and_blocks_without_expert():
             out.append(o)
         assert torch.equal(*out)
         assert out[0].abs().sum() > 0
+
+
+@pytest.mark.parametrize("tokens,rows", [(40, 33), (33, 40)])
+def test_routing_of_another_number_of_tokens(tokens, rows):
+    """Fewer routed tokens than activation rows (the others get nothing), or more (dropped): layers with
+    small blocks take these as the layers with gathered activations do."""
+    from flydsl_b200 import _lib
+    from flydsl_b200.moe import BlockscaleMoE
+
+    H, I, E, k = 512, 256, 8, 2
+    m = _case(40, H, I, E, k)
+    args = (m["x_q"][:tokens], m["x_scale"][:tokens].t().contiguous(), m["topk_ids"][:rows], m["topk_weights"][:rows])
+    both = min(tokens, rows)
+    for mode in ("reduce", "atomic"):
+        out = []
+        for layout in (None, False):
+            layer = BlockscaleMoE.from_unpacked(m["w1_q"], m["w1_scale"], m["w2_q"], m["w2_scale"], topk=k, tile_m=16,
+                                                mode=mode, sorted_layout=layout)
+            out.append(layer.forward(*args))
+            assert _lib.query_device_error() == 0 and out[-1].shape == (tokens, H)
+        if mode == "reduce":   # rows without routes are unspecified there
+            assert torch.equal(out[0][:both], out[1][:both])
+        else:
+            assert not out[0][both:].any() and not out[1][both:].any()
+            scale = out[1].float().abs().max()
+            assert (out[0].float() - out[1].float()).abs().max() <= (k + 1) * 2.0 ** -8 * 4 * scale
