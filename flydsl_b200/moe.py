@@ -140,6 +140,8 @@ class BlockscaleMoE:
         """x_q fp8 ``[T, H]``; x_scale_t f32 ``[H/128, T]``; topk_ids i32 ``[T, k]``; topk_weights f32.
         Returns ``out [T, H]``. ``routing`` may carry precomputed sort buffers
         ``(sorted_ids, sorted_weights, sorted_expert_ids, num_valid_ids)``."""
+        if stream is None:   # the current stream: every launch below takes it by itself
+            return self._forward(x_q, x_scale_t, topk_ids, topk_weights, out, routing)
         with torch.cuda.stream(_as_torch_stream(stream)):
             return self._forward(x_q, x_scale_t, topk_ids, topk_weights, out, routing)
 
@@ -149,7 +151,7 @@ class BlockscaleMoE:
         dev = x_q.device
         dense_in = x_q.is_contiguous() and x_scale_t.is_contiguous()
         small = (self._small_stages is not None and routing is None and dense_in
-                 and tuple(topk_ids.shape) == (T, self.topk))   # the fused permute takes no other routing
+                 and topk_ids.shape == (T, self.topk))   # the fused permute takes no other routing
         gemm1, gemm2 = self._small_stages if small else (self.gemm1, self.gemm2)
         in_order = self.sorted_layout or small
         b = self._buffers(T, dev, in_order)

@@ -172,14 +172,14 @@ def moe_sorting(topk_ids: torch.Tensor, topk_weights: torch.Tensor, *, num_exper
                 sorted_expert_ids.data_ptr(), num_post_pad.data_ptr(), _lib.stream_handle(stream)))
         else:
             x, xs_t, x_sorted, xs_sorted = permute
-            if x.shape[0] != tokens or tuple(x_sorted.shape) != (max_len, x.shape[1]) or \
-                    tuple(xs_sorted.shape) != (x.shape[1] // 128, max_len):
+            rows, K = x.shape
+            if rows != tokens or x_sorted.shape != (max_len, K) or xs_sorted.shape != (K // 128, max_len):
                 raise ValueError("permute buffers do not match [T, K] -> [T*k + E*block - k, K]")
             _lib.check(_lib.load().flyb200_moe_sort_permute(
                 topk_ids.data_ptr(), topk_weights.data_ptr(), tokens, topk, int(num_experts),
                 int(block_size), mask_ptr, nlt, sorted_ids.data_ptr(), sorted_weights.data_ptr(),
                 sorted_expert_ids.data_ptr(), num_post_pad.data_ptr(), x.data_ptr(), xs_t.data_ptr(),
-                x_sorted.data_ptr(), xs_sorted.data_ptr(), int(x.shape[1]), _lib.stream_handle(stream)))
+                x_sorted.data_ptr(), xs_sorted.data_ptr(), K, _lib.stream_handle(stream)))
     return sorted_ids, sorted_weights, sorted_expert_ids, num_post_pad
 
 
