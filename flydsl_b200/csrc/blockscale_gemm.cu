@@ -1719,15 +1719,29 @@ static int dense_group_m(int M, int K) {
   return cdiv(M, BM) >= 2 * gm ? gm : 0;
 }
 
-// Wide decode shapes on the tiled kernel: with this many weight tiles it fills the GPU without split-K,
-// and a narrow tile's K block takes 0.25 us. Measured, decode against tiled kernel (us, graph replay, cold
-// weights): M = 16, N = 10240 (80 tiles of 128) K = 2048 9.1 / 9.4, K = 4096 13.7 / 14.3; N = 12288 (96)
-// 9.9 / 9.5, 15.0 / 14.3; N = 16384 11.0 / 10.1, 19.9 / 15.1. M = 32, N = 7168 (56) K = 1024 6.4 / 5.3, K =
-// 2048 8.7 / 7.7, K = 4096 11.9 / 11.6, K = 7168 16.9 / 17.2; N = 16384, K = 2048 12.5 / 10.3. (Block scales
-// only: the per-token tiles are 256 wide and lose to the decode kernel on such shapes.)
-static bool tiled_beats_decode(int M, int N, int K) {
+// Wide decode shapes on the tiled kernel (block scales only: the per-token tiles are 256 wide and lose to the
+// decode kernel on such shapes). With enough weight tiles of 128 the tiled kernel fills the GPU in one pass
+// and a narrow tile's K block takes 0.25 us. The decode kernel's plan runs up to two CTAs per SM: three
+// per weight tile as long as 3 n_tiles <= 2 sms, fewer beyond, which costs it a quarter of its speed.
+// Measured, decode / tiled kernel (us, graph replay, cold weights; M = 1 and 16):
+//   96 tiles  K = 1536 7.3 / 7.7 and 7.8 / 7.8, K = 3072 10.2 / 11.2 and 10.7 / 11.3, K = 4096 13.0 / 13.5 and 13.5 /
+//             13.7, K = 5120 16.1 / 15.0 and 17.1 / 16.1
+//   100 tiles K = 1536 7.4 / 7.7 and 8.0 / 7.8, K = 2048 9.0 / 8.8 and 9.6 / 8.9, K = 3072 13.1 / 11.2 and 13.5 / 11.4
+//   128 tiles K = 1024 6.4 / 6.7 and 6.9 / 6.7, K = 2048 9.2 / 9.2 and 9.6 / 9.3, K = 4096 17.8 / 13.8 and 19.2 / 14.1
+//   192 tiles K = 1024 9.1 / 8.6 and 9.6 / 8.6, K = 2048 16.4 / 12.9 and 17.3 / 13.1
+// M = 17 and 32:
+//   56 tiles  K = 1024 5.5 / 5.1 and 5.9 / 5.2, K = 2048 7.2 / 7.0 and 7.8 / 7.1, K = 4096 10.3 / 10.1 and 10.5 / 10.8
+//   64 tiles  K = 4096 10.6 / 10.9 and 11.1 / 10.8; 72 tiles K = 3072 9.5 / 8.9 and 9.9 / 9.0, K = 4096 11.3 / 10.8 and
+//             11.6 / 11.0; 80 tiles K = 3072 10.2 / 10.5 and 11.3 / 11.3, K = 4096 12.6 / 12.1 and 13.7 / 12.7
+//   96 tiles  K = 3072 11.3 / 11.2 and 11.9 / 11.3, K = 4096 14.0 / 13.6 and 14.6 / 13.9
+// M = 33 to 64, 96 tiles: 13.4 / 6.5 (K = 1024) to 41.5 / 20.8 (K = 7168).
+static bool tiled_beats_decode(int M, int N, int K, int sms) {
   const int n_tiles = cdiv(N, 128);
-  return n_tiles >= 96 || (M > 16 && M <= 32 && n_tiles >= 56 && K <= 4096);
+  if (M > 32) return n_tiles >= 96;
+  if (M > 16)
+    return n_tiles >= 96 || (n_tiles >= 56 && K <= 2048) ||
+           (n_tiles >= 66 && K <= 4096 && (2 * n_tiles <= sms || K > 3584));
+  return n_tiles > sms || (3 * n_tiles > 2 * sms && K >= 2048) || (n_tiles >= 96 && K >= 5120);
 }
 
 // What a dense call launches.
@@ -1765,7 +1779,7 @@ static DensePlan plan_dense(bool pertoken, int M, int N, int K, const flyb200_ge
   // Decode-size M: the swap-AB split-K kernel (decode_gemm.cu; per-token: the token's scale on every K
   // block, the channel's once), unless a tile width or the tiled path was asked for, or the shape is
   // wide and nothing was asked for that the tiled kernel would not honour.
-  const bool wide = !pertoken && !split_k && !max_ctas && tiled_beats_decode(M, N, K);
+  const bool wide = !pertoken && !split_k && !max_ctas && tiled_beats_decode(M, N, K, sms);
   if (path == 2 || (path == 0 && M <= 64 && !block_n && !wide && decode_path_pays_off(M, N, K, sms))) {
     plan.kernel = 2;
     return plan;

@@ -77,14 +77,18 @@ def test_split_k_pertoken(M, N, K):
     assert torch.equal(out[1], out[2])
 
 
-# Decode-size M on both sides of the line between the decode and the tiled kernel
-@pytest.mark.parametrize("M,N,K", [(1, 12288, 256), (16, 12272, 256), (16, 12160, 256), (17, 7168, 512), (32, 7056, 512),
-                                   (17, 7040, 512), (32, 7168, 4224)])
-def test_decode_or_tiled(M, N, K):
+# Decode-size M on both sides of the lines between the decode and the tiled kernel
+@pytest.mark.parametrize("M,N,K,kernel", [(1, 12288, 256, DECODE), (16, 12688, 2048, TILED), (16, 12544, 2048, DECODE),
+                                          (16, 12688, 1920, DECODE), (8, 12288, 5120, TILED), (1, 19072, 256, TILED),
+                                          (17, 7168, 512, TILED), (32, 7056, 512, TILED), (17, 7040, 512, DECODE),
+                                          (32, 7168, 4224, DECODE), (32, 8448, 2304, TILED), (20, 8320, 2304, DECODE),
+                                          (24, 9600, 2304, DECODE), (33, 12288, 4096, TILED), (33, 12160, 4096, DECODE)])
+def test_decode_or_tiled(M, N, K, kernel):
     from flydsl_b200 import _lib
     from flydsl_b200.kernels import compile_blockscale_preshuffle_gemm
     from flydsl_b200.utils import shuffle_weight
 
+    assert _gemm_plan(M, N, K, sms=0)["kernel"] == kernel
     case = O.make_dense_case(M, N, K, seed=M + N)
     b = shuffle_weight(case["b_q"].cuda())
     sa, sb = case["a_scale"].cuda().t().contiguous(), case["b_scale"].cuda().contiguous()

@@ -129,3 +129,19 @@ def test_moe_layer_scratch_is_bounded_over_token_counts(tile_m, mode):
     assert 0 < kept <= moe._KEPT_SMALL_BYTES
     first = layer._buffers(1, dev, True)
     assert layer._buffers(1, dev, True) is first   # the sizes met first keep theirs
+
+
+def test_wide_decode_shapes_take_the_tiled_kernel_only_where_it_measured_faster():
+    def kernels(N, Ks, *Ms):
+        return {_gemm_plan(M, N, K)["kernel"] for K in Ks for M in Ms}
+
+    shallow, deep = range(1024, 2048, 128), range(2048, 8321, 128)
+    few, some, many = (1, 4, 8, 12, 16), (17, 20, 24, 28, 32), (33, 48, 64)
+    assert kernels(12288, range(1024, 5120, 128), *few) == {DECODE}
+    assert kernels(12800, shallow, *few) == kernels(18944, shallow, *few) == {DECODE}
+    assert kernels(12800, deep, *few) == kernels(18944, deep, *few) == {TILED}
+    assert kernels(12288, range(5120, 8321, 128), *few) == kernels(19072, shallow, *few) == {TILED}
+    assert kernels(7040, range(1024, 4097, 128), *some) == kernels(9600, range(2176, 3585, 128), *some) == {DECODE}
+    assert kernels(7168, range(1024, 2049, 128), *some) == kernels(8448, range(1024, 4097, 128), *some) == {TILED}
+    assert kernels(12288, range(1024, 8321, 128), *some, *many) == {TILED}
+    assert kernels(8192, range(4096, 8321, 128), *many) == {DECODE}
