@@ -1623,8 +1623,9 @@ static int query_clusters(int splits) {
   }
   return n;
 }
-// Every width's kernel takes a whole SM, so one width answers for all. Asked once per device and thread.
-static int max_clusters(int splits) {
+// Every width's kernel takes a whole SM, so one width answers for all (and for the int4 kernel where it
+// does). Asked once per device and thread.
+int max_clusters(int splits) {
   static thread_local int dev_of = -1;
   static thread_local int known[9];
   int dev = 0;

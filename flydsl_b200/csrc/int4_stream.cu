@@ -14,19 +14,19 @@
 //
 //   * CTA = one 128-row weight tile x one K range (split-K over a thread-block cluster, partial sums
 //     exchanged through distributed shared memory and added in rank order, as in decode_gemm.cu).
-//   * warp 8 (one thread): ring of slots, each = one packed 128 x 128 group (8 KB, one bulk copy)
+//   * last warp (one thread): ring of slots, each = one packed 128 x 128 group (8 KB, one bulk copy)
 //     + the tokens' 128 K columns (two TMA tiles of 64 K, 128-byte swizzle); group scales of the whole
 //     K range in one go.
-//   * warps 0-15 (0-7 beyond 32 tokens): warp w owns weight rows [16 (w % 8), +16) = two n-blocks of mma.m16n8k16 (tokens are
-//     the M=16 side). Per group: 8 x 16-byte loads of its rows' packed words (the four threads of a
-//     quad read the same row: a broadcast), per K step one ldmatrix.x4 of the token fragment and two
-//     MMAs into a per-group accumulator, then acc += group_sum * scale[n][group] in fp32 -- the same
+//   * consumer warps, one or two sets of eight (s4_two_sets): warp w owns weight rows [16 (w % 8), +16) = two
+//     n-blocks of mma.m16n8k16 (tokens are the M=16 side). Per group: 8 x 16-byte loads of its rows'
+//     packed words (the four threads of a quad read the same row: a broadcast), per K step one
+//     ldmatrix.x4 of the token fragment and two MMAs into a per-group accumulator, then acc += group_sum * scale[n][group] in fp32 -- the same
 //     promotion structure as the block-scale kernels: equals dequantise-then-matmul with the products
-//     q*a summed in fp32 before scaling. Warps 8-15 take every other group; their sums are added
-//     once, before the exchange.
+//     q*a summed in fp32 before scaling. With two sets each takes every other group; their sums are
+//     added once, before the exchange.
 //
-// Where the time goes with eight warps (ncu, M=16, N=K=8192): the schedulers issue on 43 % of the cycles, the integer
-// ALU pipe is the busiest at 41 %, the legacy tensor pipe 22 %, DRAM 17 %: the unpack instructions
+// Where the time goes with one set (ncu, M=16, N=K=8192): the schedulers issue on 43 % of the cycles, the
+// integer ALU pipe is the busiest at 41 %, the legacy tensor pipe 22 %, DRAM 17 %: the unpack instructions
 // (three per two weights) bound the kernel at ~960 cycles per 8 KB group against ~330 for the SM's
 // share of HBM bandwidth.
 //
@@ -361,9 +361,7 @@ struct S4Plan {
   int mb, ks, splits, kbps, slots;
 };
 
-// Sets of consumer warps (KS of the kernel) with `mb` blocks of 16 tokens: accumulators of 33 to 64 tokens
-// leave registers for one set only.
-static constexpr int s4_sets(int mb) { return mb <= 2 ? 2 : 1; }
+int max_clusters(int splits);   // blockscale_gemm.cu
 
 // Groups a ring may hold. A ring that wraps is a multiple of the sets deep, so that a slot's groups all
 // belong to one set: a warp then waits for every fill of the slots that it reads. With an odd ring and
@@ -376,17 +374,39 @@ static int s4_ring(int slots, int kbps, int ks) {
   return slots < 2 ? 2 : slots;
 }
 
-// K splits (cluster size) and ring depth. One CTA streams kbps groups; the SMs' load is what counts
-// (two CTAs may share an SM when M <= 32), plus a fixed cost per wave and a little per split for the
-// exchange.
-static S4Plan plan_int4_stream(int M, int N, int K, int sms, int force_splits) {
+// Two sets of consumer warps, each taking every other group? One set leaves a scheduler idle more than half
+// of the time (a group is a chain of shared loads, unpacking and MMAs), but two CTAs of one set share an
+// SM (288 threads, at most 88 registers) and one of two sets fills it (544 threads): nothing of the next
+// launch is then resident, and CTAs beyond one per SM wait for a second wave. So two sets, and the
+// whole SM's shared memory for their ring, where every cluster is resident at one CTA per SM and a CTA
+// has enough groups to make up for the later start. Measured, one / two sets (us a call, cold weights):
+//   M = 16  N = K = 8192 (128 CTAs, 32 groups) 20.5 / 19.0, 9216 x 4096 (144 CTAs, 16 groups, clusters of 2) 11.4 / 11.7,
+//           16384 x 2048 (128 CTAs, 16 groups, no clusters) 11.6 / 11.5, 4096 x 6144 (128 CTAs, 12 groups, clusters of 4)
+//           10.9 / 9.6, 4096 x 2048 (4 groups) 5.1 / 5.4; not all resident: 3072 x 8192 (24 clusters of 6) 12.5 / 16.1,
+//           10240 x 4096 (240 CTAs) 13.6 / 17.8
+//   M = 32  N = K = 8192 24.9 / 23.3, 9216 x 4096 14.0 / 14.3, 9216 x 2048 (8 groups) 8.8 / 9.5, 4096 x 6144 13.7 / 11.9,
+//           3072 x 8192 16.0 / 20.1, 10240 x 4096 16.7 / 22.5
+// 33 to 64 tokens: accumulators for one set only.
+static bool s4_two_sets(int mb, int splits, int kbps, int n_tiles, int sms, bool live) {
+  if (mb > 2 || n_tiles * splits > sms) return false;
+  const int least = splits == 4 ? 6 : mb == 2 ? 16 : splits == 1 ? 12 : splits == 2 ? 24 : 16;
+  return kbps >= least && (splits == 1 || n_tiles <= (live ? max_clusters(splits) : sms / splits));
+}
+
+// K splits (cluster size) and ring depth. One CTA streams kbps groups; the SMs' load is what counts, plus
+// a fixed cost per wave and a little per split for the exchange. `live`: sms are those of the current
+// device, which is asked how many clusters it holds; otherwise that number is estimated.
+static S4Plan plan_int4_stream(int M, int N, int K, int sms, int force_splits, bool live) {
   S4Plan best{0, 0, 0, 0, 0};
   const int mb = M <= 16 ? 1 : (M <= 32 ? 2 : 4);
-  const int ks = s4_sets(mb);
   const int n_tiles = N / 128;
   const int KBt = K / 128;
   const int slot = kS4PackedBytes + 2 * 16 * mb * 128;
   double best_cost = 1e30;
+  auto fixed_bytes = [&](int kbps) { return (16 * mb + 8) * 512 + kbps * 256 + 2048; };
+  auto ring = [&](int kbps, int ks, int cps) {
+    return s4_ring((232448 / cps - 1024 - fixed_bytes(kbps)) / slot, kbps, ks);
+  };
   for (int s = 1; s <= 8; ++s) {
     if (force_splits > 0 && s != force_splits) continue;
     const int kbps = (KBt + s - 1) / s;
@@ -394,18 +414,20 @@ static S4Plan plan_int4_stream(int M, int N, int K, int sms, int force_splits) {
     if (s_eff != s && force_splits <= 0) continue;
     const long ctas = static_cast<long>(n_tiles) * s_eff;
     const long per_sm = (ctas + sms - 1) / sms;
-    // up to 32 tokens a CTA takes at most half of an SM's shared memory, so that the CTAs of the
-    // next launch are resident (and prefetching) while this one computes
-    const int cps = mb <= 2 ? 2 : 1;
-    const int fixed = (16 * mb + 8) * 512 + kbps * 256 + 2048;
-    const int slots = s4_ring((232448 / cps - 1024 - fixed) / slot, kbps, ks);
-    if (slots * slot + fixed > 232448) continue;
+    // up to 32 tokens a CTA of one set takes at most half of an SM's shared memory, so that the CTAs of
+    // the next launch are resident (and prefetching) while this one computes
+    const int slots = ring(kbps, 1, mb <= 2 ? 2 : 1);
+    if (slots * slot + fixed_bytes(kbps) > 232448) continue;
     const long waves = (ctas + sms - 1) / sms;
     const double cost = static_cast<double>(per_sm) * kbps + 6.0 * waves + 0.5 * s_eff;
     if (cost < best_cost - 1e-9) {
       best_cost = cost;
-      best = S4Plan{mb, ks, s_eff, kbps, slots};
+      best = S4Plan{mb, 1, s_eff, kbps, slots};
     }
+  }
+  if (best.splits && s4_two_sets(mb, best.splits, best.kbps, n_tiles, sms, live)) {
+    best.ks = 2;
+    best.slots = ring(best.kbps, 2, 1);
   }
   return best;
 }
@@ -446,7 +468,7 @@ int launch_int4_stream(void* c, const void* a, const void* wq, const void* scale
                        int force_splits, cudaStream_t stream) {
   const int sms = sm_count();
   if (sms <= 0) return FLYB200_ERR_CUDA;
-  const S4Plan plan = plan_int4_stream(M, N, K, sms, force_splits);
+  const S4Plan plan = plan_int4_stream(M, N, K, sms, force_splits, true);
   if (plan.splits < 1)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_gemm: no plan for M=%d N=%d K=%d", M, N, K);
   Int4StreamParams p{};
@@ -461,14 +483,13 @@ int launch_int4_stream(void* c, const void* a, const void* wq, const void* scale
   const int rc = make_tensor_map_2d(&tmap, a, M, K, 2, 16 * plan.mb);
   if (rc) return rc;
   switch (plan.mb) {
-    // Two sets of eight consumer warps, each taking every other group: a group is a chain of shared
-    // loads, unpacking and MMAs that leaves a scheduler with two warps idle more than half of the time.
-    // M=16, N=K=8192: 21.0 -> 19.6 us a call (24.6 -> 22.5 us with cold caches). Sharing the K steps of
-    // a group out instead repeats the promotion and was slower than one set (23.5 against 21.5 us), as
-    // were four n-blocks per warp (22.8 / 24.5 us). 33 to 64 tokens: accumulators for one set only.
-    case 1: return launch_int4_stream_mb<1, 2, s4_sets(1)>(tmap, p, stream);
-    case 2: return launch_int4_stream_mb<2, 2, s4_sets(2)>(tmap, p, stream);
-    default: return launch_int4_stream_mb<4, 2, s4_sets(4)>(tmap, p, stream);
+    // Sharing the K steps of a group out over 16 warps instead repeats the promotion and was slower than
+    // one set (M=16, N=K=8192: 23.5 against 21.5 us), as were four n-blocks per warp (22.8 / 24.5 us).
+    case 1: return plan.ks == 2 ? launch_int4_stream_mb<1, 2, 2>(tmap, p, stream)
+                                : launch_int4_stream_mb<1, 2, 1>(tmap, p, stream);
+    case 2: return plan.ks == 2 ? launch_int4_stream_mb<2, 2, 2>(tmap, p, stream)
+                                : launch_int4_stream_mb<2, 2, 1>(tmap, p, stream);
+    default: return launch_int4_stream_mb<4, 2, 1>(tmap, p, stream);
   }
 }
 
@@ -478,8 +499,9 @@ extern "C" int flyb200_int4_plan(int32_t M, int32_t N, int32_t K, int32_t split_
   using namespace flyb200;
   if (!plan || M < 1 || M > 64 || N < 128 || N % 128 || K < 128 || K % 128)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_plan: bad arguments (M=%d N=%d K=%d)", M, N, K);
-  if (sms <= 0 && (sms = sm_count()) <= 0) return FLYB200_ERR_CUDA;
-  const S4Plan p = plan_int4_stream(M, N, K, sms, split_k);
+  const bool live = sms <= 0;
+  if (live && (sms = sm_count()) <= 0) return FLYB200_ERR_CUDA;
+  const S4Plan p = plan_int4_stream(M, N, K, sms, split_k, live);
   plan[0] = p.mb; plan[1] = p.ks; plan[2] = p.splits; plan[3] = p.kbps; plan[4] = p.slots;
   return FLYB200_OK;
 }

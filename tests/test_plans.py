@@ -6,11 +6,11 @@ import pytest
 SMS = 148
 
 
-def _int4_plan(M, N, K, split_k):
+def _int4_plan(M, N, K, split_k, sms=SMS):
     from flydsl_b200 import _lib
 
     plan = (ctypes.c_int32 * 5)()
-    _lib.check(_lib.load().flyb200_int4_plan(M, N, K, split_k, SMS, plan))
+    _lib.check(_lib.load().flyb200_int4_plan(M, N, K, split_k, sms, plan))
     return tuple(plan)
 
 
@@ -25,12 +25,29 @@ def test_int4_ring_slots_belong_to_one_set(M, split_k):
             _, sets, splits, groups, slots = _int4_plan(M, N, K, split_k)
             if splits == 0:   # no plan: the call is refused
                 continue
-            assert sets == (2 if M <= 32 else 1) and 2 <= slots <= 16
+            assert sets in ((1, 2) if M <= 32 else (1,)) and 2 <= slots <= 16
             owner = {}
             for g in range(groups):
                 assert owner.setdefault(g % slots, g % sets) == g % sets, (N, K, sets, groups, slots)
             wrapped += groups > slots
     assert wrapped > 100
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64])
+def test_int4_two_sets_only_where_every_cta_has_an_sm(M):
+    """A CTA with two sets of warps fills an SM: no second wave, and enough groups for both sets."""
+    seen = set()
+    for N in range(128, 24577, 128):
+        for K in range(128, 16385, 256):
+            mb, sets, splits, groups, slots = _int4_plan(M, N, K, 0)
+            ctas = N // 128 * splits
+            seen.add(sets)
+            if sets == 2:
+                assert ctas <= SMS and groups >= 6
+            else:   # two CTAs of up to 32 tokens share an SM's shared memory
+                slot, rest = 8192 + mb * 4096, (16 * mb + 8) * 512 + groups * 256 + 2048
+                assert slots * slot + rest + 1024 <= 233472 // (2 if M <= 32 else 1)
+    assert seen == ({1, 2} if M <= 32 else {1})
 
 
 def _kernel_source(name):
