@@ -1949,8 +1949,12 @@ static int moe_sorted_layout(const flyb200_gemm_cfg* cfg, int T, int E, int k, i
 
 // Small routing blocks take the kernel with the weights on the MMA's M side (moe_swap.cu), unless a tile
 // width was asked for: up to 32 tokens per block, where the tiled kernel's 128 rows are mostly padding.
+// With more blocks than that kernel lists (it does not merge neighbours then) only up to 16: 128 experts of
+// 1024 x 256, 16384 tokens in blocks of 32 (up to 4224 blocks), tiled / weights on the M side: stage 1 431 /
+// 378 us, stage 2 450 / 535, with atomic adds 404 / 772; in blocks of 16 (8320 blocks) 760 / 512, 748 / 664,
+// 679 / 894.
 static bool moe_swap_pays_off(const flyb200_gemm_cfg* cfg, const GemmParams& p) {
-  return p.a_sorted && p.tile_m <= 32 && !cfg->block_n;
+  return p.a_sorted && p.tile_m <= 32 && !cfg->block_n && (p.tile_m <= 16 || p.num_blocks <= kMoeSwapListed);
 }
 
 static int moe_gemm1_impl(void* out, void* out_q, float* out_scale_t, const void* x, const void* w_repacked,

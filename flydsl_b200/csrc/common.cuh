@@ -17,6 +17,9 @@ int set_error(int status, const char* fmt, ...);
 int* device_error_word();  // address of the current device's error word (cached per device)
 int sm_count();            // SM count of the current device (cached per device)
 
+// Routing blocks up to which the MoE kernel for small blocks (moe_swap.cu) lists and merges neighbours.
+constexpr int kMoeSwapListed = 4096;
+
 #define FLYB200_CUDA_CHECK(expr)                                                               \
   do {                                                                                         \
     cudaError_t _e = (expr);                                                                   \

@@ -37,7 +37,6 @@ namespace {
 constexpr int kSwThreads = 320;
 constexpr int kSwEpiWarp0 = 2;
 constexpr int kSwEpiWarps = 8;
-constexpr int kSwMaxBlocks = 4096;   // routing blocks up to which neighbours are merged
 constexpr int kSwW = 128 * 128;   // bytes of a weight tile's K block
 
 struct SwapParams {
@@ -63,7 +62,7 @@ struct SwapCfg {
   static constexpr int kAccBufs = 512 / (2 * NT) > 8 ? 8 : 512 / (2 * NT);
   static constexpr int kTmemCols = 2 * NT * kAccBufs;
   static constexpr int kDone = kStages + kAccBufs;
-  static constexpr int kListBytes = kSwMaxBlocks * 2;
+  static constexpr int kListBytes = kMoeSwapListed * 2;
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + kListBytes + 1024;
   static_assert(kSmemBytes <= 232448, "shared memory");
 };
@@ -143,7 +142,7 @@ moe_swap_kernel(const __grid_constant__ CUtensorMap tmap_x, const SwapParams p) 
   constexpr int kCols = STAGE == 1 ? 128 : 256;   // output channels per tile
   const int num_n = (p.N + kCols - 1) / kCols;
   const int num_m = max(0, min(p.num_blocks, (p.num_valid[0] + p.tile_m - 1) / p.tile_m));
-  const bool listed = num_m <= kSwMaxBlocks;
+  const bool listed = num_m <= kMoeSwapListed;
   uint16_t* const list = reinterpret_cast<uint16_t*>(misc + 1024);
   volatile int* const list_len = reinterpret_cast<volatile int*>(misc + 8 * kNumBars + 8);
   if (warp == 0 && listed) {
