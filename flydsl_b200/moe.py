@@ -64,7 +64,8 @@ class BlockscaleMoE:
         # Measured on the 256-expert layer: 4.31 -> 3.76 ms at 128-token blocks, but slightly slower
         # for decode-size batches (one more launch, nothing to hide), hence the default by block size.
         # Blocks of at most 32 rows take these layouts all the same where forward() does the routing
-        # itself: the stages are then the kernel with the weights on the MMA's M side.
+        # itself and it pays off (_small_pays_off): the stages are then the kernel with the weights on the
+        # MMA's M side.
         self.sorted_layout = (self.tile_m >= 64 and self.tile_m % 8 == 0) if sorted_layout is None \
             else bool(sorted_layout)
         # Optional: re-quantisation between the stages fused into the stage-1 epilogue (routing-order
@@ -135,6 +136,29 @@ class BlockscaleMoE:
             self._buf[key] = b
         return b
 
+    def _small_pays_off(self, T: int) -> bool:
+        """Whether T tokens in blocks of at most 32 rows take routing-order layouts. The stages gain from
+        blocks that follow one another in the same expert (one pass over its weights for two) and, in a
+        steady stream of calls, from the tensor work that is not done for padding; the permute and the
+        re-quantiser of padded rows cost 10 to 30 us. Measured in steady streams, routing order / gathered
+        (us a layer; uniform routing, and with every 16th expert hot):
+          blocks of 16  256 experts of 7168 x 2048, top 8, 32 tokens 1089 / 1105 and 536 / 548, 128 x 4096 x 1536, 64
+                        tokens 394 / 411 and 336 / 363, 8 tokens 182 / 183 and 137 / 124, 256 x 3072 x 1024, top 4, 128
+                        tokens 356 / 350 and 157 / 174, 32 tokens 180 / 174 and 90 / 81, 64 x 2048 x 1024, top 6, 200
+                        tokens 117 / 135 and 125 / 136, 64 tokens 105 / 96 and 102 / 95
+          blocks of 32  256 x 7168 x 2048, 256 tokens 1769 / 1861 and 1658 / 1846, 128 x 4096 x 1536, 256 tokens 443 /
+                        426 and 459 / 507, 512 tokens 463 / 602 and 538 / 611, 256 x 3072 x 1024, 384 tokens 485 /
+                        419 and 357 / 354, 64 x 2048 x 1024, 384 tokens 129 / 144 and 136 / 142
+        and with more blocks than the kernel lists: see moe_swap_pays_off in blockscale_gemm.cu."""
+        routes, rows = T * self.topk, self.E * self.tile_m
+        if self.tile_m > 16 and routes + rows - self.topk > 4096 * self.tile_m:
+            return False
+        nbytes = min(self.E, routes) * 3 * self.H * self.I   # weights of the experts that may be hit
+        if nbytes >= 4e9:
+            return True
+        least = 0.75 if nbytes < 1e9 else 0.1 if self.tile_m <= 16 else 0.5
+        return routes >= least * rows
+
     def forward(self, x_q, x_scale_t, topk_ids, topk_weights, out=None, stream=None,
                 routing=None):
         """x_q fp8 ``[T, H]``; x_scale_t f32 ``[H/128, T]``; topk_ids i32 ``[T, k]``; topk_weights f32.
@@ -151,7 +175,8 @@ class BlockscaleMoE:
         dev = x_q.device
         dense_in = x_q.is_contiguous() and x_scale_t.is_contiguous()
         small = (self._small_stages is not None and routing is None and dense_in
-                 and topk_ids.shape == (T, self.topk))   # the fused permute takes no other routing
+                 and topk_ids.shape == (T, self.topk)   # the fused permute takes no other routing
+                 and self._small_pays_off(T))
         gemm1, gemm2 = self._small_stages if small else (self.gemm1, self.gemm2)
         in_order = self.sorted_layout or small
         b = self._buffers(T, dev, in_order)

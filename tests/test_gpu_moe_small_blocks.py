@@ -30,17 +30,19 @@ def test_block_scale_layer(T, H, I, E, k, tile_m, out_dtype):
     args = (m["x_q"], m["x_scale"].t().contiguous(), m["topk_ids"], m["topk_weights"])
     out = {}
     for mode in ("reduce", "atomic"):
-        for layout in (False, None):
+        for layout in (False, True, None):   # gathered, routing order, the layer's choice
             layer = BlockscaleMoE.from_unpacked(m["w1_q"], m["w1_scale"], m["w2_q"], m["w2_scale"], topk=k, tile_m=tile_m,
                                                 mode=mode, sorted_layout=layout, out_dtype=out_dtype)
             out[mode, layout] = layer.forward(*args).float()
             assert _lib.query_device_error() == 0
+    assert torch.equal(out["reduce", True], out["reduce", False])
     assert torch.equal(out["reduce", None], out["reduce", False])
     # 16-bit atomics round the running sum at each of the k additions, in any order: k half ulps of the
     # largest partial sum, which 4 times the largest result covers for these weights (softmax, sum 1)
     ulp = 2.0 ** -8 if out_dtype == torch.bfloat16 else 2.0 ** -11
-    scale = out["reduce", None].abs().max()
-    assert (out["atomic", None] - out["reduce", None]).abs().max() <= (k + 1) * ulp * 4 * scale
+    scale = out["reduce", True].abs().max()
+    for layout in (True, None):
+        assert (out["atomic", layout] - out["reduce", True]).abs().max() <= (k + 1) * ulp * 4 * scale
 
 
 @pytest.mark.parametrize("T,H,I,E,k,tile_m", SHAPES)
@@ -97,7 +99,7 @@ def test_more_blocks_than_the_list_and_blocks_without_expert():
         assert out[0].abs().sum() > 0
 
 
-@pytest.mark.parametrize("tokens,rows", [(40, 33), (33, 40)])
+@pytest.mark.parametrize("tokens,rows", [(80, 66), (66, 80)])
 def test_routing_of_another_number_of_tokens(tokens, rows):
     """Fewer routed tokens than activation rows (the others get nothing), or more (dropped): layers with
     small blocks take these as the layers with gathered activations do."""
@@ -105,7 +107,7 @@ def test_routing_of_another_number_of_tokens(tokens, rows):
     from flydsl_b200.moe import BlockscaleMoE
 
     H, I, E, k = 512, 256, 8, 2
-    m = _case(40, H, I, E, k)
+    m = _case(80, H, I, E, k)
     args = (m["x_q"][:tokens], m["x_scale"][:tokens].t().contiguous(), m["topk_ids"][:rows], m["topk_weights"][:rows])
     both = min(tokens, rows)
     for mode in ("reduce", "atomic"):
@@ -113,6 +115,7 @@ def test_routing_of_another_number_of_tokens(tokens, rows):
         for layout in (None, False):
             layer = BlockscaleMoE.from_unpacked(m["w1_q"], m["w1_scale"], m["w2_q"], m["w2_scale"], topk=k, tile_m=16,
                                                 mode=mode, sorted_layout=layout)
+            assert layer._small_pays_off(tokens)
             out.append(layer.forward(*args))
             assert _lib.query_device_error() == 0 and out[-1].shape == (tokens, H)
         if mode == "reduce":   # rows without routes are unspecified there

@@ -123,6 +123,34 @@ def test_plan_refuses_what_the_call_refuses():
             _gemm_plan(**case)
 
 
+def _moe_layer(E, H, I, topk, tile_m, mode="reduce"):
+    import torch
+
+    from flydsl_b200.moe import BlockscaleMoE
+
+    def meta(*shape, dtype=torch.float8_e4m3fn):
+        return torch.empty(shape, dtype=dtype, device="meta")
+
+    return BlockscaleMoE(meta(E, 2 * I, H), meta(E, 2 * I // 128 * (H // 128), dtype=torch.float32), meta(E, H, I),
+                         meta(E, H // 128 * (I // 128), dtype=torch.float32), topk=topk, tile_m=tile_m, mode=mode)
+
+
+@pytest.mark.parametrize("E,H,I,topk,tile_m,least", [
+    (256, 7168, 2048, 8, 16, 12), (256, 7168, 2048, 8, 32, 12),           # from 4 GB of weights in use on
+    (128, 4096, 1536, 8, 16, 26), (128, 4096, 1536, 8, 32, 256),          # routes for 0.1 / 0.5 of all blocks
+    (64, 2048, 1024, 6, 16, 128), (64, 2048, 1024, 6, 32, 256), (128, 2048, 512, 2, 8, 384)])   # small layers: 0.75
+def test_moe_small_blocks_take_routing_order_where_it_pays_off(E, H, I, topk, tile_m, least):
+    layer = _moe_layer(E, H, I, topk, tile_m)
+    for T in range(1, 1025):
+        assert layer._small_pays_off(T) == (T >= least), T
+
+
+def test_moe_more_blocks_than_the_kernel_lists():
+    wide, narrow = _moe_layer(128, 1024, 256, 8, 32), _moe_layer(128, 1024, 256, 8, 16)
+    assert wide._small_pays_off(15873) and not wide._small_pays_off(15874)   # 4096 blocks, one more
+    assert narrow._small_pays_off(100000)
+
+
 @pytest.mark.parametrize("mode", ["reduce", "atomic"])
 @pytest.mark.parametrize("tile_m", [8, 16, 32])
 def test_moe_layer_scratch_is_bounded_over_token_counts(tile_m, mode):
@@ -131,13 +159,8 @@ def test_moe_layer_scratch_is_bounded_over_token_counts(tile_m, mode):
 
     from flydsl_b200 import moe
 
-    def meta(*shape, dtype=torch.float8_e4m3fn):
-        return torch.empty(shape, dtype=dtype, device="meta")
-
     E, H, I, topk, dev = 256, 7168, 2048, 8, torch.device("meta")
-    layer = moe.BlockscaleMoE(meta(E, 2 * I, H), meta(E, 2 * I // 128 * (H // 128), dtype=torch.float32),
-                              meta(E, H, I), meta(E, H // 128 * (I // 128), dtype=torch.float32), topk=topk,
-                              tile_m=tile_m, mode=mode)
+    layer = _moe_layer(E, H, I, topk, tile_m, mode)
     for T in range(1, 513):
         b = layer._buffers(T, dev, True)
         rows = T * topk + E * tile_m - topk
