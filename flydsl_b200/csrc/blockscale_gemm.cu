@@ -918,10 +918,9 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             const int buf = it % kAccBufs;
             const float s0 = ring_a[j] * ring_b0[j];
             const float s1 = ring_a[j] * ring_b1[j];
-            // Both products exist before the ring slots are loaded again. Left to itself the compiler
-            // forms them where they are used, loads into other registers and moves the values over at
-            // the end of the trip, which waits there for loads issued in this very trip: a memory
-            // latency in every K block (M = 256, N = 4096, K = 7168, 64-wide tiles: 28.6 -> 21 us).
+            // Both products are formed before the ring slots are loaded again (the empty asm takes them).
+            // Without it a clock trace showed 400-550 cycles per K block outside the drain, about a memory
+            // latency, and M = 256, N = 4096, K = 7168 in 64-wide tiles took 28.6 us instead of 21.
             asm volatile("" ::"f"(s0), "f"(s1));
             if (kb + kRing < KB) {
               ring_a[j] = __ldg(pf_a);
@@ -1564,6 +1563,10 @@ static inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 // Time of one K block of a tile (ns), measured on B200: the slope over K of graph replays with cold
 // operands (M = 256, N = 4096: 32 columns 0.25, 64 0.21-0.25, 128 0.27, 256 0.46 us) and of full waves
 // (M = N = 4096, K = 7168: 128 columns 0.36, 256 0.50 us).
+// The MoE stages use the same figures. Against 360 + 0.9 bn, which stood here before, stage 1's width is
+// the same for all sizes, stage 2's and the dense one's goes from 256 to 128 columns where four rounds
+// take the place of three: 9 row blocks, N = 8320, K = 2048 stage 2 40.2 -> 34.1 us (gathered rows 69.0 ->
+// 57.5), dense 26.6 -> 26.2; K = 512 23.1 -> 19.1 (24.8 -> 25.4), 11.2 -> 11.6.
 static double tile_kb_ns(int bn) { return bn == 256 ? 490.0 : bn == 128 ? 330.0 : bn == 64 ? 250.0 : 245.0; }
 
 // Tile-width heuristic (role of select_tile_config in the reference's test). Cost model per K block

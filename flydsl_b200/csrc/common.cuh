@@ -93,8 +93,8 @@ __device__ __forceinline__ bool mbar_test_both(uint32_t bar0, uint32_t parity0, 
   return ok != 0;
 }
 // One lane of a converged warp. A loop that the whole warp runs, with only the tcgen05 instructions under
-// the elected lane, issues them faster than the same loop under `lane == 0`, whose operands the compiler
-// cannot take as warp-uniform (4096 x 4096 x 7168 in 32-wide tiles, bound by issue: 546 -> 404 us).
+// the elected lane, issues them faster than the same loop under `lane == 0` (4096 x 4096 x 7168 in 32-wide
+// tiles, bound by issue: 546 -> 404 us).
 __device__ __forceinline__ bool elect_one() {
   uint32_t ok;
   asm volatile(
