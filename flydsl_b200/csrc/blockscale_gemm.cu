@@ -1626,19 +1626,19 @@ static int query_clusters(int splits) {
   }
   return n;
 }
-// Every width's kernel takes a whole SM, so one width answers for all (and for the int4 kernel where it
-// does). Asked once per device and thread.
-int max_clusters(int splits) {
+// By cluster size, 2 to 8. Every width's kernel takes a whole SM, so one width answers for all (and for the
+// int4 kernel where it does). Asked once per device and thread; a plan takes the table once, not an entry
+// per candidate (a dozen cudaGetDevice calls were 0.5 to 1 us of a call).
+const int* max_clusters() {
   static thread_local int dev_of = -1;
   static thread_local int known[9];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  if (dev != dev_of) {
-    for (int i = 0; i < 9; ++i) known[i] = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+  if (dev != dev_of || dev < 0) {
+    for (int i = 0; i < 9; ++i) known[i] = dev >= 0 && i >= 2 ? query_clusters<128>(i) : 0;
     dev_of = dev;
   }
-  if (known[splits] < 0) known[splits] = query_clusters<128>(splits);
-  return known[splits];
+  return known;
 }
 
 // Split-K plan of a dense problem: the tile width and cluster size with the smallest estimated time, or
@@ -1657,12 +1657,15 @@ static SplitPlan pick_split(int M, int N, int K, int sms, bool live, bool pertok
   auto kb_ns = [&](int bn) { return pertoken ? 330.0 : tile_kb_ns(bn); };
   SplitPlan best{force_bn, 1, kbt};
   double best_cost = 1e30;
+  const int* clusters = nullptr;
   if (!force_splits) {
     const int bn = pertoken ? 256 : pick_block_n(m_blocks, N, sms, false);
     const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
     best = SplitPlan{bn, 1, kbt};
     if (static_cast<long>(m_blocks) * cdiv(N, 256) * 2 > sms) return best;   // no room even for the widest tiles
     best_cost = ((tiles + sms - 1) / sms) * kbt * kb_ns(bn);
+    if (best_cost <= 3000.0) return best;   // the exchange alone takes as long
+    if (live) clusters = max_clusters();
   }
   const int widths[3] = {256, 128, 64};
   for (int w = 0; w < 3; ++w) {
@@ -1673,7 +1676,7 @@ static SplitPlan pick_split(int M, int N, int K, int sms, bool live, bool pertok
       if (force_splits && sp != force_splits) continue;
       const int kbps = cdiv(kbt, sp);
       if (cdiv(kbt, kbps) != sp) continue;           // some CTA would have no K block
-      if (!force_splits && (tiles * sp > sms || tiles > (live ? max_clusters(sp) : sms / sp))) continue;
+      if (!force_splits && (tiles * sp > sms || tiles > (clusters ? clusters[sp] : sms / sp))) continue;
       const double exchange = 3000.0 + rows * bn * 4.0 * (sp - 1) / sp / 20.0;
       const double cost = kbps * kb_ns(bn) + exchange;
       if (cost < best_cost - 1e-9) {

@@ -361,7 +361,7 @@ struct S4Plan {
   int mb, ks, splits, kbps, slots;
 };
 
-int max_clusters(int splits);   // blockscale_gemm.cu
+const int* max_clusters();   // blockscale_gemm.cu
 
 // Groups a ring may hold. A ring that wraps is a multiple of the sets deep, so that a slot's groups all
 // belong to one set: a warp then waits for every fill of the slots that it reads. With an odd ring and
@@ -390,7 +390,7 @@ static int s4_ring(int slots, int kbps, int ks) {
 static bool s4_two_sets(int mb, int splits, int kbps, int n_tiles, int sms, bool live) {
   if (mb > 2 || n_tiles * splits > sms) return false;
   const int least = splits == 4 ? 6 : mb == 2 ? 16 : splits == 1 ? 12 : splits == 2 ? 24 : 16;
-  return kbps >= least && (splits == 1 || n_tiles <= (live ? max_clusters(splits) : sms / splits));
+  return kbps >= least && (splits == 1 || n_tiles <= (live ? max_clusters()[splits] : sms / splits));
 }
 
 // K splits (cluster size) and ring depth. One CTA streams kbps groups; the SMs' load is what counts, plus
