@@ -505,7 +505,7 @@ extern "C" int flyb200_int4_gemm(void* c, const void* a, const void* wq, const v
   if (N < 128 || N % 128 || K < 128 || K % 128)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_gemm: N and K must be multiples of 128 (N=%d K=%d)", N, K);
   // cfg.path: 1 = the register-dequantising mma.sync kernel (int4_stream.cu), 2 = the tcgen05 kernel
-  // of this file, 0 = whichever was measured faster: up to 32 tokens the former (21.5 / 26.9 us
+  // of this file, 0 = whichever was measured faster: up to 32 tokens the former (19.0 / 23.3 us
   // against 32.3 / 33.5 us at N = K = 8192), above that the latter (35.6 against 38.4 us at 64)
   const int path = (cfg && cfg->path) ? cfg->path : (M <= 32 ? 1 : 2);
   if (path != 2)
