@@ -1664,7 +1664,8 @@ static SplitPlan pick_split(int M, int N, int K, int sms, bool live, bool pertok
     best = SplitPlan{bn, 1, kbt};
     if (static_cast<long>(m_blocks) * cdiv(N, 256) * 2 > sms) return best;   // no room even for the widest tiles
     best_cost = ((tiles + sms - 1) / sms) * kbt * kb_ns(bn);
-    if (best_cost <= 3000.0) return best;   // the exchange alone takes as long
+    // the least that any plan takes: one K block and half of a 64-wide tile exchanged
+    if (best_cost <= 3245.0 + 6.4 * rows) return best;
     if (live) clusters = max_clusters();
   }
   const int widths[3] = {256, 128, 64};
