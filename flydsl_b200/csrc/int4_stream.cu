@@ -378,18 +378,22 @@ static int s4_ring(int slots, int kbps, int ks) {
 // of the time (a group is a chain of shared loads, unpacking and MMAs), but two CTAs of one set share an
 // SM (288 threads, at most 88 registers) and one of two sets fills it (544 threads): nothing of the next
 // launch is then resident, and CTAs beyond one per SM wait for a second wave. So two sets, and the
-// whole SM's shared memory for their ring, where every cluster is resident at one CTA per SM and a CTA
-// has enough groups to make up for the later start. Measured, one / two sets (us a call, cold weights):
+// whole SM's shared memory for their ring, only where every cluster is resident at one CTA per SM.
+// Measured, one / two sets (us a call, cold weights, graph replay):
 //   M = 16  N = K = 8192 (128 CTAs, 32 groups) 20.5 / 19.0, 9216 x 4096 (144 CTAs, 16 groups, clusters of 2) 11.4 / 11.7,
 //           16384 x 2048 (128 CTAs, 16 groups, no clusters) 11.6 / 11.5, 4096 x 6144 (128 CTAs, 12 groups, clusters of 4)
-//           10.9 / 9.6, 4096 x 2048 (4 groups) 5.1 / 5.4; not all resident: 3072 x 8192 (24 clusters of 6) 12.5 / 16.1,
+//           10.9 / 9.6, 8192 x 2048 (8 groups) 6.8 / 7.4; not all resident: 3072 x 8192 (24 clusters of 6) 12.5 / 16.1,
 //           10240 x 4096 (240 CTAs) 13.6 / 17.8
-//   M = 32  N = K = 8192 24.9 / 23.3, 9216 x 4096 14.0 / 14.3, 9216 x 2048 (8 groups) 8.8 / 9.5, 4096 x 6144 13.7 / 11.9,
+//   M = 32  N = K = 8192 24.9 / 23.3, 9216 x 4096 14.0 / 14.3, 8192 x 2048 (8 groups) 8.7 / 9.3, 4096 x 6144 13.7 / 11.9,
 //           3072 x 8192 16.0 / 20.1, 10240 x 4096 16.7 / 22.5
-// 33 to 64 tokens: accumulators for one set only.
+// The least number of groups: launched one by one, a call of one set that takes about as long as its launch
+// from the host (9 us) falls into a slow rhythm, in which the next launch's CTAs pile up on some SMs:
+// M = 16, 8192 x 2944 (12 groups) 13.5 / 9.8, 5120 x 4096 (11 groups) 12.6 / 9.9; M = 32, 8192 x 2048 12.7 / 9.7, 5120 x
+// 2944 (8 groups) 12.6 / 9.9. Calls with fewer groups are over before the next launch and gain from one set
+// in a graph; longer ones queue up. 33 to 64 tokens: accumulators for one set only.
 static bool s4_two_sets(int mb, int splits, int kbps, int n_tiles, int sms, bool live) {
   if (mb > 2 || n_tiles * splits > sms) return false;
-  const int least = splits == 4 ? 6 : mb == 2 ? 16 : splits == 1 ? 12 : splits == 2 ? 24 : 16;
+  const int least = splits == 4 ? 6 : mb == 2 ? 8 : 10;
   return kbps >= least && (splits == 1 || n_tiles <= (live ? max_clusters()[splits] : sms / splits));
 }
 

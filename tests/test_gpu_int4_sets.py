@@ -10,9 +10,9 @@ from tests.test_plans import _int4_plan
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M,N,K,split_k,sets", [(1, 128, 1408, 1, 1), (5, 128, 2176, 1, 2), (16, 256, 4352, 1, 2),
-                                                (16, 384, 5888, 2, 1), (9, 256, 6272, 2, 2), (16, 128, 2816, 4, 2),
-                                                (17, 128, 1920, 1, 1), (20, 256, 2176, 1, 2), (32, 128, 5888, 2, 2),
+@pytest.mark.parametrize("M,N,K,split_k,sets", [(1, 128, 1152, 1, 1), (5, 128, 2176, 1, 2), (16, 256, 4352, 1, 2),
+                                                (16, 384, 2176, 2, 1), (9, 256, 6272, 2, 2), (16, 128, 2816, 4, 2),
+                                                (17, 128, 896, 1, 1), (20, 256, 2176, 1, 2), (32, 128, 5888, 2, 2),
                                                 (32, 384, 2816, 4, 2), (31, 128, 2944, 8, 1), (33, 128, 2176, 1, 1)])
 def test_int4_sets_of_warps(M, N, K, split_k, sets):
     from flydsl_b200 import _lib
