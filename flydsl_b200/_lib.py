@@ -5,9 +5,12 @@ object has not been built, loading raises with the build command.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from ctypes import c_char_p, c_int, c_int32, c_int64, c_size_t, c_uint32, c_void_p, POINTER
+
+import torch
 
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("FLYB200_LIB_PATH") or os.path.join(_PKG_DIR, "lib", "libflyb200.so")
@@ -131,8 +134,10 @@ def stream_handle(stream) -> int:
     (python/flydsl/expr/typing.py:312-332).
     """
     if stream is None:
-        import torch
-
+        # The handle itself: building a torch.cuda.Stream to read it from took 3.2 us of a decode call's 8.8
+        # on the host (0.3 us now). A process that cannot use CUDA gets torch's own error.
+        if torch.cuda.is_initialized():
+            return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
         return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
@@ -140,6 +145,18 @@ def stream_handle(stream) -> int:
     if handle is None:
         raise TypeError(f"stream must be a torch.cuda.Stream, an int handle or None, got {type(stream)!r}")
     return int(handle)
+
+
+_NO_GUARD = contextlib.nullcontext()
+
+
+def device_guard(t):
+    """``with`` block in which the device of CUDA tensor ``t`` is current. Where it is already (every call of
+    a process that uses one GPU) there is nothing to switch: 0.4 us instead of the 1.5 of torch.cuda.device."""
+    index = t.get_device()
+    if index == torch._C._cuda_getDevice():
+        return _NO_GUARD
+    return torch.cuda.device(index)
 
 
 def query_device_error(stream=None) -> int:

@@ -45,7 +45,7 @@ def pack_int4_weight(q: torch.Tensor, scales: torch.Tensor) -> Tuple[torch.Tenso
     scales = scales.to(torch.bfloat16).contiguous()
     wq = torch.empty((K // GROUP, N // 8, 4, 8, 16), dtype=torch.uint8, device=q.device)
     st = torch.empty((K // GROUP, N), dtype=torch.bfloat16, device=q.device)
-    with torch.cuda.device(q.device):
+    with _lib.device_guard(q):
         _lib.check(_lib.load().flyb200_int4_repack(q.data_ptr(), scales.data_ptr(), N, K, wq.data_ptr(),
                                                    st.data_ptr(), _lib.stream_handle(None)))
     return wq, st

@@ -18,7 +18,7 @@ from .kernels.moe_blockscale_2stage import (
     compile_moe_blockscale_gemm2,
     compile_moe_reduction,
 )
-from .utils import moe_gather_rows, moe_sorting, quant_1x128, shuffle_weight
+from .utils import moe_gather_rows, moe_sorting, quant_1x128, quant_pertoken, shuffle_weight
 
 # Scratch that one layer keeps for blocks of at most 32 rows, over all token counts (see _buffers).
 _KEPT_SMALL_BYTES = 256 << 20
@@ -299,33 +299,36 @@ class PertokenMoE:
         """x_q fp8 ``[T, H]``; x_scale f32 ``[T]`` (or ``[T, 1]``); topk_ids i32 ``[T, k]``; topk_weights
         f32. Returns ``out [T, H]``. ``routing`` may carry precomputed sort buffers
         ``(sorted_ids, sorted_weights, sorted_expert_ids, num_valid_ids)``."""
-        from .utils import quant_pertoken
-
+        if stream is None:   # the current stream: every launch below takes it by itself
+            return self._forward(x_q, x_scale, topk_ids, topk_weights, out, routing)
         with torch.cuda.stream(_as_torch_stream(stream)):
-            T = x_q.shape[0]
-            dev = x_q.device
-            b = self._buffers(T, dev)
-            if routing is None:
-                sid, sw, seid, npp = moe_sorting(topk_ids, topk_weights, num_experts=self.E,
-                                                 block_size=self.tile_m)
-            else:
-                sid, sw, seid, npp = routing
-            if sid.numel() != b["rows"]:
-                raise ValueError("routing buffers do not match this layer's experts/tile_m/topk")
-            nblk = seid.numel()
-            moe_gather_rows(x_q, x_scale.reshape(-1), sid, npp, topk=self.topk, out=b["x_sorted"],
-                            scale_out=b["xs_sorted"], per_token=True)
-            self.gemm1(b["out1"], b["x_sorted"], self.w1, b["xs_sorted"], self.w1_scale, sid, seid, sw, npp,
-                       T, self.I, self.H, nblk, None)
-            quant_pertoken(b["out1"], npp, out=b["a2_q"], scale_out=b["a2_s"])
-            if out is None:
-                out = torch.empty((T, self.H), dtype=self.out_dtype, device=dev)
-            if routing is not None:
-                b["routes"].zero_()   # a caller's routing may drop routes: their rows must sum as zero
-            self.gemm2(b["routes"], b["a2_q"], self.w2, b["a2_s"], self.w2_scale, sid, seid, sw, npp, T,
-                       self.H, self.I, nblk, None)
-            self.reduce(b["routes"], out, None, T, None)
-            return out
+            return self._forward(x_q, x_scale, topk_ids, topk_weights, out, routing)
+
+    def _forward(self, x_q, x_scale, topk_ids, topk_weights, out, routing):
+        T = x_q.shape[0]
+        dev = x_q.device
+        b = self._buffers(T, dev)
+        if routing is None:
+            sid, sw, seid, npp = moe_sorting(topk_ids, topk_weights, num_experts=self.E,
+                                             block_size=self.tile_m)
+        else:
+            sid, sw, seid, npp = routing
+        if sid.numel() != b["rows"]:
+            raise ValueError("routing buffers do not match this layer's experts/tile_m/topk")
+        nblk = seid.numel()
+        moe_gather_rows(x_q, x_scale.reshape(-1), sid, npp, topk=self.topk, out=b["x_sorted"],
+                        scale_out=b["xs_sorted"], per_token=True)
+        self.gemm1(b["out1"], b["x_sorted"], self.w1, b["xs_sorted"], self.w1_scale, sid, seid, sw, npp,
+                   T, self.I, self.H, nblk, None)
+        quant_pertoken(b["out1"], npp, out=b["a2_q"], scale_out=b["a2_s"])
+        if out is None:
+            out = torch.empty((T, self.H), dtype=self.out_dtype, device=dev)
+        if routing is not None:
+            b["routes"].zero_()   # a caller's routing may drop routes: their rows must sum as zero
+        self.gemm2(b["routes"], b["a2_q"], self.w2, b["a2_s"], self.w2_scale, sid, seid, sw, npp, T,
+                   self.H, self.I, nblk, None)
+        self.reduce(b["routes"], out, None, T, None)
+        return out
 
     #: kernels one forward() launches: sort, permute, gemm1, quant, gemm2, reduce
     launches_per_step = 6

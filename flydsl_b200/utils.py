@@ -50,7 +50,7 @@ def shuffle_weight(x: torch.Tensor, layout=(16, 16), use_int4: bool = False) -> 
     batch = x.numel() // (n * k) if x.numel() else 0
     out = torch.empty_like(x)
     if batch:
-        with torch.cuda.device(x.device):
+        with _lib.device_guard(x):
             _lib.check(_lib.load().flyb200_repack_weight_fp8(
                 out.data_ptr(), x.data_ptr(), batch, n, k, _lib.stream_handle(None)))
     out.is_shuffled = True
@@ -99,9 +99,9 @@ def quant_1x128(x: torch.Tensor, stream=None) -> Tuple[torch.Tensor, torch.Tenso
     if x.dim() != 2:
         raise ValueError("quant_1x128 expects [rows, cols]")
     rows, cols = x.shape
-    q = torch.empty((rows, cols), dtype=FP8_DTYPE, device=x.device)
-    st = torch.empty((cols // 128, rows), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    q = x.new_empty(rows, cols, dtype=FP8_DTYPE)
+    st = x.new_empty(cols // 128, rows, dtype=torch.float32)
+    with _lib.device_guard(x):
         _lib.check(_lib.load().flyb200_quant_1x128(
             x.data_ptr(), q.data_ptr(), st.data_ptr(), rows, cols, _dtype_code(x.dtype),
             _lib.stream_handle(stream)))
@@ -118,10 +118,10 @@ def quant_pertoken(x: torch.Tensor, num_rows_dev: Optional[torch.Tensor] = None,
         raise ValueError("quant_pertoken expects f16/bf16 [rows, cols]")
     rows, cols = x.shape
     if out is None:
-        out = torch.empty((rows, cols), dtype=FP8_DTYPE, device=x.device)
+        out = x.new_empty(rows, cols, dtype=FP8_DTYPE)
     if scale_out is None:
-        scale_out = torch.empty((rows,), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+        scale_out = x.new_empty(rows, dtype=torch.float32)
+    with _lib.device_guard(x):
         _lib.check(_lib.load().flyb200_quant_pertoken(
             x.data_ptr(), out.data_ptr(), scale_out.data_ptr(),
             None if num_rows_dev is None else num_rows_dev.data_ptr(), rows, cols, _dtype_code(x.dtype),
@@ -150,10 +150,10 @@ def moe_sorting(topk_ids: torch.Tensor, topk_weights: torch.Tensor, *, num_exper
     dev = topk_ids.device
     max_len = int(topk_ids.numel() + int(num_experts) * int(block_size) - int(topk))
     max_blocks = (max_len + int(block_size) - 1) // int(block_size)
-    sorted_ids = torch.empty((max_len,), dtype=torch.int32, device=dev)
-    sorted_weights = torch.empty((max_len,), dtype=torch.float32, device=dev)
-    sorted_expert_ids = torch.empty((max_blocks,), dtype=torch.int32, device=dev)
-    num_post_pad = torch.empty((2,), dtype=torch.int32, device=dev)
+    sorted_ids = topk_ids.new_empty(max_len)
+    sorted_weights = topk_ids.new_empty(max_len, dtype=torch.float32)
+    sorted_expert_ids = topk_ids.new_empty(max_blocks)
+    num_post_pad = topk_ids.new_empty(2)
     mask_ptr = None
     if expert_mask is not None:
         expert_mask = expert_mask.to(device=dev, dtype=torch.int32).contiguous()
@@ -164,7 +164,7 @@ def moe_sorting(topk_ids: torch.Tensor, topk_weights: torch.Tensor, *, num_exper
         nlt = int(num_local_tokens.item())
     else:
         nlt = int(num_local_tokens)
-    with torch.cuda.device(dev):
+    with _lib.device_guard(topk_ids):
         if permute is None:
             _lib.check(_lib.load().flyb200_moe_sort(
                 topk_ids.data_ptr(), topk_weights.data_ptr(), tokens, topk, int(num_experts),
@@ -193,10 +193,10 @@ def route_topk(logits: torch.Tensor, topk: int, stream=None) -> Tuple[torch.Tens
     if logits.dtype != torch.float32:
         logits = logits.float()
     T, E = logits.shape
-    ids = torch.empty((T, int(topk)), dtype=torch.int32, device=logits.device)
-    w = torch.empty((T, int(topk)), dtype=torch.float32, device=logits.device)
+    ids = logits.new_empty(T, int(topk), dtype=torch.int32)
+    w = logits.new_empty(T, int(topk))
     if T:
-        with torch.cuda.device(logits.device):
+        with _lib.device_guard(logits):
             _lib.check(_lib.load().flyb200_moe_route_topk(logits.data_ptr(), T, E, int(topk), ids.data_ptr(),
                                                           w.data_ptr(), _lib.stream_handle(stream)))
     return ids, w
@@ -244,7 +244,7 @@ def moe_gather_rows(x, scale_t, sorted_ids, num_valid_ids, *, topk: int, by_slot
             raise ValueError(f"per_token gather needs one scale per row ({rows_in}), got {scale_t.numel()}")
         if scale_out is None:
             scale_out = torch.empty((rows_out,), dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
+        with _lib.device_guard(x):
             _lib.check(_lib.load().flyb200_moe_gather_rows_pertoken(
                 x.data_ptr(), scale_t.data_ptr(), sorted_ids.data_ptr(), num_valid_ids.data_ptr(),
                 out.data_ptr(), scale_out.data_ptr(), rows_in, K, int(topk), rows_out, int(bool(by_slot)),
@@ -252,7 +252,7 @@ def moe_gather_rows(x, scale_t, sorted_ids, num_valid_ids, *, topk: int, by_slot
         return out, scale_out
     if scale_out is None:
         scale_out = torch.empty((K // 128, rows_out), dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.device_guard(x):
         _lib.check(_lib.load().flyb200_moe_gather_rows(
             x.data_ptr(), scale_t.data_ptr(), sorted_ids.data_ptr(), num_valid_ids.data_ptr(),
             out.data_ptr(), scale_out.data_ptr(), rows_in, K, int(topk), rows_out, int(bool(by_slot)),
