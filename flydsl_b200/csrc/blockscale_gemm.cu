@@ -1707,6 +1707,10 @@ int launch_moe_swap(int stage, bool pertoken, void* out, const void* act, const 
                     const float* sorted_weights, const int32_t* num_valid_ids, int T, int n, int kdim, int num_blocks,
                     int E, int k, int tile_m, int doweight, int accumulate, int out_sorted, int a_rows, int out_dtype,
                     int max_ctas, cudaStream_t stream);
+// bs_pair_gemm.cu
+int launch_blockscale_pair_gemm(void* c, const void* a, const void* b_repacked, const float* scale_a_t,
+                                const float* scale_b, int M, int N, int K, int out_dtype, int ctas, int group_m,
+                                cudaStream_t stream);
 // pt_pair_gemm.cu
 int launch_pertoken_pair_gemm(void* c, const void* a, const void* b_repacked, const float* scale_a,
                               const float* scale_b, int M, int N, int K, int out_dtype, int max_ctas, int group_m,
@@ -1750,6 +1754,22 @@ static bool tiled_beats_decode(int M, int N, int K, int sms) {
     return n_tiles >= 96 || (n_tiles >= 56 && K <= 2048) ||
            (n_tiles >= 66 && K <= 4096 && (2 * n_tiles <= sms || K > 3584));
   return n_tiles > sms || (3 * n_tiles > 2 * sms && K >= 2048) || (n_tiles >= 96 && K >= 5120);
+}
+
+// Block scales: 256 x 256 tiles on CTA pairs (bs_pair_gemm.cu) instead of the tiled kernel, which takes
+// tiled_ns per K block. A pair's K block takes about 460 ns; measured in steady streams of calls, tiled / pairs (us):
+//   as many rounds of 256-wide tiles either way: 147 x 21312 x 1536 18.1 / 16.6, 245 x 20608 x 3968 38.7 / 34.4,
+//     1485 x 9984 x 4608 84.3 / 79.6, 4096 x 7168 x 2048 72.1 / 69.0, 16384 x 4096 x 7168 487 / 462
+//   a round more: 1126 x 12416 x 1280 25.6 / 28.9, 1093 x 12000 x 3840 61.1 / 68.1, 302 x 19200 x 3200 33.6 / 40.2
+//   few K blocks in all (the pair's set-up takes ~0.5 us more): 1914 x 1536 x 1536 10.2 / 10.6
+//   narrower tiles in one round: 533 x 3328 x 3584 13.0 / 16.9, 231 x 4736 x 5120 13.9 / 21.0
+// With an odd number of 128-row blocks half of a pair's last row block is padding: 313 x 7920 x 4736 24.0 / 24.5,
+// 316 x 14848 x 6272 55.8 / 56.2, but 591 x 10368 x 2688 27.4 / 27.3, 1089 x 10816 x 5376 77.2 / 74.4.
+static bool pair_beats_tiled(int M, int N, int kblocks, int ctas, double tiled_ns) {
+  if (M < 512 && cdiv(M, BM) % 2) return false;
+  const long tiles = static_cast<long>(cdiv(M, 256)) * cdiv(N, 256);
+  const long pairs = ctas / 2;
+  return kblocks * ((tiles + pairs - 1) / pairs) * 460.0 + 500.0 < kblocks * tiled_ns;
 }
 
 // What a dense call launches.
@@ -1813,6 +1833,14 @@ static DensePlan plan_dense(bool pertoken, int M, int N, int K, const flyb200_ge
   plan.bn = pertoken ? 256 : block_n ? block_n : split.splits > 1 ? split.bn : pick_block_n(m_blocks, N, sms, false);
   const long tiles = static_cast<long>(m_blocks) * cdiv(N, plan.bn);
   plan.grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
+  if (!pertoken && path == 0 && !block_n && !split_k && split.splits == 1 && plan.grid >= 2 &&
+      pair_beats_tiled(M, N, K / BK, plan.grid, ((tiles + plan.grid - 1) / plan.grid) * tile_kb_ns(plan.bn))) {
+    const long pairs = static_cast<long>(cdiv(M, 256)) * cdiv(N, 256);
+    plan.kernel = 3;
+    plan.bn = 256;
+    plan.grid = 2 * static_cast<int>(pairs < plan.grid / 2 ? pairs : plan.grid / 2);
+    return plan;
+  }
   if (split.splits > 1) plan.grid = static_cast<int>(tiles * split.splits);
   else if (tiles < plan.grid) plan.grid = static_cast<int>(tiles);
   return plan;
@@ -1842,6 +1870,9 @@ static int dense_gemm(bool pertoken, void* c, const void* a, const void* b_repac
   if (plan.kernel == 2)
     return launch_decode_gemm(c, a, b_repacked, scale_a, scale_b, M, N, K, out_dtype, cfg ? cfg->split_k : 0, st,
                               pertoken);
+  if (plan.kernel == 3 && !pertoken)
+    return launch_blockscale_pair_gemm(c, a, b_repacked, scale_a, scale_b, M, N, K, out_dtype, plan.grid,
+                                       dense_group_m(M, K), st);
   if (plan.kernel == 3)
     return launch_pertoken_pair_gemm(c, a, b_repacked, scale_a, scale_b, M, N, K, out_dtype,
                                      cfg ? cfg->max_ctas : 0, dense_group_m(M, K), st);

@@ -11,6 +11,13 @@
 // the chain MMAs -> completion seen -> drained -> buffer handed back, which has to fit into two K blocks: with
 // one 256-wide group the MMAs take one of the two, with halves half of one.
 //
+// Measured, steady streams of calls, single-CTA tiles / pairs: 4096 x 7168 x 2048 72.1 / 69.0 us, 4096 x 4096 x
+// 7168 131 / 125, 16384 x 4096 x 7168 487 / 462, 256 x 24576 x 1536 19.6 / 17.6 (rested: 60.7 / 57.9, 113 / 108, 419 /
+// 396, 19.8 / 18.1). What bounds it now is the promotion and the power cap together: with the drain left out
+// (a probe) 4096 x 4096 x 7168 takes 103 us, with the TMEM loads but no FMAs 113. Not kept: the next K block's first
+// load requested ahead of its turn (a conditional tcgen05.ld; 6 % slower), 8- and 32-column loads (3 and 2 %
+// slower), unpacked FMAs (6 %); without asking for the next completion ahead of time it is 6 % slower.
+//
 // Roles per CTA (384 threads): warp 0 producer, warp 1 MMA issuer (leader CTA) and TMEM allocation, warp 2 store
 // thread, warp 3 relay (peer: tells the leader that a stage has landed), warps 4-11 epilogue. A completed group
 // is announced to both CTAs by one multicast commit. Every wait is bounded; on expiry the role records a code in
@@ -292,8 +299,7 @@ bs_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     uint32_t tiles = 0;
     int buf = 0;
     uint32_t dn_i = 0, dn_ph = 0;   // iteration % kDone and (iteration / kDone) & 1
-    bool loading = false;           // the next K block's first quarter is being loaded (warp-uniform)
-    uint32_t va[32], vb[32];
+    bool ready = false;             // the next K block's group is known to have completed (warp-uniform)
     // where this half's buffers are handed back: barriers of the leader CTA
     const uint32_t tempty0 = leader ? tempty_bar(half, 0) : map_to_cta(tempty_bar(half, 0), 0);
     const uint32_t tempty1 = leader ? tempty_bar(half, 1) : map_to_cta(tempty_bar(half, 1), 0);
@@ -320,16 +326,18 @@ bs_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         for (int j = 0; j < kRing; ++j) {
           const int kb = kb0 + j;
           if (kb < KB && alive) {
-            if (!loading) {   // the first quarter has not been asked for ahead of time
+            if (!ready) {
               const bool got = mbar_wait(done_bar(half, dn_i), dn_ph, abort_flag, p.err, kErrWaitTmemFull);
               if (!__all_sync(0xffffffffu, got)) {
                 alive = false;
                 break;
               }
-              tc_fence_after();
-              tmem_ld<32>(tmem_h + buf * 128, va);
             }
-            // in the shadow of that load: the scale, the loads of later scales, the counters
+            tc_fence_after();
+            const uint32_t src = tmem_h + buf * 128;
+            uint32_t va[16], vb[16];
+            tmem_ld<16>(src, va);
+            // in the shadow of the first load: the scale, the loads of later scales, the counters
             const float s = ring_a[j] * ring_b[j];
             asm volatile("" ::"f"(s));   // formed before the slot is loaded again (see blockscale_gemm.cu)
             if (kb + kRing < KB) {
@@ -338,42 +346,35 @@ bs_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             }
             pf_a += p.M;
             ++pf_b;
-            const uint32_t src = tmem_h + buf * 128;
             const uint32_t rel = buf ? tempty1 : tempty0;
             if (++dn_i == kDone) {
               dn_i = 0;
               dn_ph ^= 1;
             }
-            buf ^= 1;
             const float2 s2 = make_float2(s, s);
-            auto promote = [&](const uint32_t* v, int q) {
+            tmem_wait_dep<16>(va);
 #pragma unroll
-              for (int c = 0; c < 16; ++c) {
-                float2& d = acc[q * 16 + c];
-                d = __ffma2_rn(make_float2(__uint_as_float(v[2 * c]), __uint_as_float(v[2 * c + 1])), s2, d);
+            for (int q = 0; q < 8; ++q) {
+              uint32_t* cv = (q & 1) ? vb : va;
+              uint32_t* nv = (q & 1) ? va : vb;
+              if (q < 7) tmem_ld<16>(src + (q + 1) * 16, nv);   // in flight during the FMAs
+              if (q == 6) ready = mbar_test(done_bar(half, dn_i), dn_ph);   // the next K block's
+              float2* a = acc + q * 8;
+#pragma unroll
+              for (int c = 0; c < 8; ++c)
+                a[c] = __ffma2_rn(make_float2(__uint_as_float(cv[2 * c]), __uint_as_float(cv[2 * c + 1])), s2, a[c]);
+              if (q < 7) tmem_wait_dep<16>(nv);
+              // Everything has been read: the buffer goes back to the issuer. The wait above is one instruction
+              // of the whole warp (.sync.aligned), for the loads of all its lanes, so lane 0 may speak for them
+              // without a __syncwarp (which costs 1.5 %).
+              if (q == 6) {
+                tc_fence_before();
+                mbar_arrive_if(rel, lane == 0 && leader);
+                mbar_arrive_cluster_if(rel, lane == 0 && !leader);
               }
-            };
-            tmem_wait_dep<32>(va);
-            tmem_ld<32>(src + 32, vb);   // in flight during the FMAs of the quarter before
-            promote(va, 0);
-            tmem_wait_dep<32>(vb);
-            tmem_ld<32>(src + 64, va);
-            promote(vb, 1);
-            tmem_wait_dep<32>(va);
-            tmem_ld<32>(src + 96, vb);
-            loading = mbar_test(done_bar(half, dn_i), dn_ph);   // the next K block's group has completed?
-            promote(va, 2);
-            loading = __all_sync(0xffffffffu, loading);
-            tmem_wait_dep<32>(vb);
-            // everything has been read: the buffer goes back to the issuer
-            tc_fence_before();
-            mbar_arrive_if(rel, lane == 0 && leader);
-            mbar_arrive_cluster_if(rel, lane == 0 && !leader);
-            if (loading) {
-              tc_fence_after();
-              tmem_ld<32>(tmem_h + buf * 128, va);
             }
-            promote(vb, 3);
+            ready = __all_sync(0xffffffffu, ready);
+            buf ^= 1;
           }
         }
       }

@@ -38,17 +38,7 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t local_bar, uint32_t 
   const uint32_t remote = map_to_cta(local_bar, rank);
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
 }
-// Predicated forms (no branch): a local arrival; a relaxed one on a barrier given by its cluster address.
-__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool pred) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %1, 0;\n\t"
-      "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t"
-      "}" ::"r"(bar),
-      "r"(static_cast<uint32_t>(pred))
-      : "memory");
-}
+// Predicated, relaxed, on a barrier given by its cluster address.
 __device__ __forceinline__ void mbar_arrive_cluster_if(uint32_t bar, bool pred) {
   asm volatile(
       "{\n\t"
@@ -58,19 +48,6 @@ __device__ __forceinline__ void mbar_arrive_cluster_if(uint32_t bar, bool pred) 
       "}" ::"r"(bar),
       "r"(static_cast<uint32_t>(pred))
       : "memory");
-}
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {   // never suspends
-  uint32_t ok;
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
 }
 // Three queries in flight together; the first two are answered as one, the third through `third`.
 __device__ __forceinline__ bool mbar_test_2_1(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1,

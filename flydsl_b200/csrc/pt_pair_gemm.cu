@@ -20,6 +20,7 @@
 #include "cluster.cuh"
 #include "common.cuh"
 #include "flyb200.h"
+#include "pair.cuh"
 
 namespace flyb200 {
 
@@ -46,40 +47,6 @@ struct PairParams {
   int M, N, K;
   int group_m;   // pair-row blocks per group of the tile order (0 = one group)
 };
-
-__device__ __forceinline__ void tmem_alloc2(uint32_t dst_smem, uint32_t cols) {
-  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish2() {
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t cols) {
-  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-// completion of all MMAs issued so far -> one arrival on a barrier of the issuing (leader) CTA; the
-// leader's relay thread passes it on to the peer
-__device__ __forceinline__ void tc_commit2(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tc_mma_f8_2(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                            uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// One arrival on an mbarrier of another CTA of the cluster. Relaxed: the arriving threads publish no
-// data of their own (they pass on a completion they have observed on a local barrier); with release
-// semantics at cluster scope each such arrival took ~700-900 cycles and was the bottleneck of the loop.
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t local_bar, uint32_t rank) {
-  const uint32_t remote = map_to_cta(local_bar, rank);
-  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(remote) : "memory");
-}
 
 struct PairTile {
   int pm, n;   // pair-row block (256 rows), column tile (256 columns)
