@@ -1477,6 +1477,23 @@ int make_tensor_map_2d(CUtensorMap* map, const void* base, int rows, int cols, i
   return FLYB200_OK;
 }
 
+// Row-major [rows, cols] of 16-bit elements seen as [cols / 64][rows][64]: box = box_slabs slabs of 128 bytes x box_rows
+// rows, one 128-byte-swizzled tile after the other; out-of-range rows read as 0.
+int make_tensor_map_slabs16(CUtensorMap* map, const void* base, int rows, int cols, int box_rows, int box_slabs) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return set_error(FLYB200_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
+  cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / 64)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(cols) * 2, 128};
+  cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_slabs)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return set_error(FLYB200_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", static_cast<int>(r));
+  return FLYB200_OK;
+}
+
 template <int BN, int MODE, typename OutT>
 static int launch(const CUtensorMap& tmap_a, const CUtensorMap& tmap_c, const GemmParams& p,
                   int grid, cudaStream_t stream) {

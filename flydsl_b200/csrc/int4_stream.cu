@@ -1,16 +1,12 @@
-// Weight-only int4 x bf16 GEMM for decode-size M (<= 64), register-dequantising kernel: the default
-// path of flyb200_int4_gemm (int4_gemm.cu keeps the tcgen05 variant and the packed layout's
-// description; both read the same packed weights and give the same arithmetic contract).
+// Weight-only int4 x bf16 GEMM for decode-size M (<= 64), register-dequantising kernel for problems with little
+// to stream (int4_gemm.cu has the tcgen05 kernel for the others and the packed layout's description; both
+// read the same packed weights and give the same arithmetic contract).
 //
-// Why not tcgen05 here: with 16-64 tokens the tensor work is negligible and the kernel lives or dies
-// by how cheaply 4-bit weights become MMA operands at HBM speed. tcgen05.mma reads its operands
-// from shared memory, so every weight takes a round trip nibble -> bf16 -> shared memory (4x the
-// packed bytes, written and read again: ~660 cycles of shared-memory bandwidth per 8 KB group), and
-// one thread issues eight K=16 instructions per group at ~60 cycles each plus the commit (~690
-// cycles per group, measured) where the SM's share of HBM bandwidth allows ~330. mma.sync takes the
-// weight operand from REGISTERS: a thread unpacks exactly the nibbles of its own B fragment (shift,
-// and/or, subtract: three instructions per two weights), every warp issues its own MMAs, and shared
-// memory only carries the packed bytes once.
+// mma.sync takes the weight operand from REGISTERS: a thread unpacks exactly the nibbles of its own B fragment
+// (shift, and/or, subtract: three instructions per two weights), every warp issues its own MMAs, and shared
+// memory only carries the packed bytes once. There is less to set up than for tcgen05 (no tensor memory, no
+// hand-over between dequantisers, issuer and epilogue), which is faster where little is streamed
+// (stream_beats_tensor in int4_gemm.cu); elsewhere the unpacking bounds it.
 //
 //   * CTA = one 128-row weight tile x one K range (split-K over a thread-block cluster, partial sums
 //     exchanged through distributed shared memory and added in rank order, as in decode_gemm.cu).

@@ -81,7 +81,7 @@ def compile_int4_weight_only_gemm(*, N: int, K: int, group_size: int = GROUP, sp
                                   path: str = "auto"):
     """Launcher for ``C[m, N] = A[m, K] @ dequant(W)^T``, ``m <= 64`` chosen per call. ``path`` picks
     the kernel: ``"stream"`` (csrc/int4_stream.cu), ``"tensor"`` (csrc/int4_gemm.cu) or ``"auto"``
-    (the default: the former up to 32 tokens, the latter above)."""
+    (the default: the former where there is little to stream, else the latter)."""
     if group_size != GROUP:
         raise ValueError(f"group_size must be {GROUP}")
     if N % 128 or K % 128:

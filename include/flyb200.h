@@ -363,8 +363,8 @@ int flyb200_int4_repack(const int8_t* q, const void* scales, int32_t N, int32_t 
 /* c bf16 [M, N] = a bf16 [M, K] * dequant(W)^T, W as produced by flyb200_int4_repack; fp32
  * accumulation, the group scale applied per 128-K group in fp32. 1 <= M <= 64; N, K % 128 == 0.
  * cfg (optional): split_k forces the split-K factor (cluster size, 1..8); path picks the kernel:
- * 1 = weights unpacked in registers and fed to mma.sync (faster up to 32 tokens), 2 = weights
- * unpacked through shared memory for tcgen05.mma, 0 = by token count. Same arithmetic either way. */
+ * 1 = weights unpacked in registers and fed to mma.sync (faster where there is little to stream), 2 =
+ * weights unpacked into tensor memory for tcgen05.mma, 0 = by size. Same arithmetic either way. */
 int flyb200_int4_gemm(void* c, const void* a, const void* wq, const void* scales_t, int32_t M, int32_t N,
                       int32_t K, const flyb200_gemm_cfg* cfg, void* stream);
 
