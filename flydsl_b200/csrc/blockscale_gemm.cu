@@ -376,9 +376,13 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   // that pool: 40 x 128 + 232 x 256 = 64512 <= 64512.
   if (warp < kEpiWarp0) {
     reg_dealloc<40>();
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
       // ---------------- producer: weights (and dense A) via TMA ----------------
-      uint32_t it = 0;
+      // The whole warp runs the loop and one elected lane issues; slots, phases and addresses are counters. As a
+      // chain of scalar instructions with divisions in one thread a K block took this role about 450 cycles, more
+      // than the MMAs of all but the widest tiles.
+      const bool copier = elect_one();
+      uint32_t st = 0, filled = 0, dn = 0, dph = 0;   // stage; stages filled so far (at most kStages); completion barrier
       bool alive = true;
       const uint64_t pol_evict_first = l2_policy_evict_first();
       auto load_w = [&](uint32_t dst, const uint8_t* src, uint32_t bytes, uint32_t bar, bool last_use) {
@@ -415,30 +419,43 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             row_stride_kb = static_cast<size_t>(p.N) * BK;
           }
         }
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          const int s = it % kStages;
-          if (!wait_stage_free(it, kErrWaitSmemEmpty)) {
-            alive = false;
-            break;
-          }
-          const uint32_t sa = smem_base + s * C::kStageBytes;
-          const uint32_t sb = sa + kATileBytes;
-          const uint8_t* src = wbase + (kb_first + kb) * row_stride_kb + static_cast<size_t>(n0) * BK;
-          if constexpr (is_dense(MODE)) {
-            mbar_arrive_expect_tx(full_bar(s), p.a_box_rows * BK + rows_b * BK);
-            tma_load_2d(sa, &tmap_a, (kb_first + kb) * BK, m_blk * BM, full_bar(s));
-            bulk_load(sb, src, rows_b * BK, full_bar(s));
-          } else if constexpr (is_moe1(MODE)) {
-            mbar_arrive_expect_tx(full_bar(s), 2 * rows_b * BK + (p.a_sorted ? p.a_box_rows * BK : 0));
-            if (p.a_sorted) tma_load_2d(sa, &tmap_a, kb * BK, m_blk * p.tile_m, full_bar(s));
-            load_w(sb, src, rows_b * BK, full_bar(s), w_last_use);
-            load_w(sb + (BN / 2) * BK, src + static_cast<size_t>(p.N) * BK, rows_b * BK, full_bar(s),
-                   w_last_use);
+        const uint32_t w_bytes = static_cast<uint32_t>(rows_b) * BK;
+        const uint32_t stage_bytes = (is_moe1(MODE) ? 2 : 1) * w_bytes +
+                                     (is_dense(MODE) || p.a_sorted ? static_cast<uint32_t>(p.a_box_rows) * BK : 0u);
+        const uint8_t* src = wbase + kb_first * row_stride_kb + static_cast<size_t>(n0) * BK;
+        const size_t up = static_cast<size_t>(p.N) * BK;   // stage 1: from the gate rows to the up rows
+        int ax = kb_first * BK;
+        const int ay = m_blk * (is_dense(MODE) ? BM : p.tile_m);
+        for (int kb = 0; kb < KB; ++kb) {
+          if (filled == kStages) {   // the MMAs that read this stage last
+            const bool ok = mbar_wait(done_bar(dn), dph, abort_flag, p.err, kErrWaitSmemEmpty);
+            if (!__all_sync(0xffffffffu, ok)) {
+              alive = false;
+              break;
+            }
+            if (++dn == kDone) {
+              dn = 0;
+              dph ^= 1;
+            }
           } else {
-            mbar_arrive_expect_tx(full_bar(s), rows_b * BK + (p.a_sorted ? p.a_box_rows * BK : 0));
-            if (p.a_sorted) tma_load_2d(sa, &tmap_a, kb * BK, m_blk * p.tile_m, full_bar(s));
-            load_w(sb, src, rows_b * BK, full_bar(s), w_last_use);
+            ++filled;
           }
+          if (copier) {
+            const uint32_t sa = smem_base + st * C::kStageBytes;
+            const uint32_t sb = sa + kATileBytes, bar = full_bar(st);
+            mbar_arrive_expect_tx(bar, stage_bytes);
+            if (is_dense(MODE) || p.a_sorted) tma_load_2d(sa, &tmap_a, ax, ay, bar);
+            if constexpr (is_dense(MODE)) {
+              bulk_load(sb, src, w_bytes, bar);
+            } else {
+              load_w(sb, src, w_bytes, bar, w_last_use);
+              if constexpr (is_moe1(MODE)) load_w(sb + (BN / 2) * BK, src + up, w_bytes, bar, w_last_use);
+            }
+          }
+          __syncwarp();
+          src += row_stride_kb;
+          ax += BK;
+          if (++st == kStages) st = 0;
         }
       }
     } else if (warp == 1) {
@@ -456,8 +473,12 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         return __all_sync(0xffffffffu, ok);
       };
       constexpr uint32_t idesc = umma_idesc_e4m3_f32(BM, BN);
-      uint32_t it = 0;
+      uint32_t it = 0;             // kDensePT
       uint32_t tiles_issued = 0;   // kDensePT
+      // stage, accumulator buffer and completion barrier of the next K block, their phases, and whether its
+      // operands and its buffer are known to be there
+      uint32_t st = 0, ph = 0, buf = 0, tph = 0, dn = 0;
+      bool ready = false;
       bool alive = true;
       for (TilePos pos = walk.start(); walk.valid(pos) && alive; walk.advance(pos)) {
         if constexpr (!is_dense(MODE)) {
@@ -467,7 +488,7 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         if constexpr (is_pt(MODE)) {
           // one accumulator buffer per TILE: wait for it once, accumulate every K block into it,
           // then tell the epilogue; the per-K-block commits only hand the stages back
-          const int buf = static_cast<int>(tiles_issued % kAccBufs);
+          buf = tiles_issued % kAccBufs;
           const bool free_ok = mbar_wait(tempty_bar(buf), ((tiles_issued / kAccBufs) & 1) ^ 1, abort_flag, p.err,
                                          kErrWaitTmemEmpty);
           if (!__all_sync(0xffffffffu, free_ok)) {
@@ -500,30 +521,40 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
           ++tiles_issued;
           continue;
         }
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          const int s = it % kStages;
-          const uint32_t ph = (it / kStages) & 1;
-          const int buf = it % kAccBufs;
-          const uint32_t tph = (it / kAccBufs) & 1;
-          const uint32_t sa = smem_base + s * C::kStageBytes;
-          const uint64_t adesc = umma_desc_sw128(sa);
-          const uint64_t bdesc = umma_desc_sw128(sa + kATileBytes);
-          const uint32_t d = tmem_u + buf * BN;
+        for (int kb = 0; kb < KB; ++kb) {
           // The operands normally landed long ago; the accumulator buffer is what the issuer really
           // waits for, so that wait comes last and nothing but the fence separates it from the MMAs.
-          if (!wait_both(full_bar(s), ph, tempty_bar(buf), tph ^ 1)) {
+          if (!ready && !wait_both(full_bar(st), ph, tempty_bar(buf), tph ^ 1)) {
             alive = false;
             break;
           }
           tc_fence_after();
-          if (leader) {
-#pragma unroll
-            for (int k = 0; k < BK / 32; ++k)
-              tc_mma_f8(d, adesc + 2 * k, bdesc + 2 * k, idesc, k > 0 ? 1u : 0u);
-            // the MMAs of the K block are done: partial sums in TMEM, operands consumed
-            tc_commit(done_bar(it % kDone));
+          const uint64_t adesc = umma_desc_sw128(smem_base + st * C::kStageBytes);
+          const uint64_t bdesc = adesc + (kATileBytes >> 4);
+          const uint32_t d = tmem_u + buf * BN;
+          const uint32_t done = done_bar(dn);
+          if (++st == kStages) {
+            st = 0;
+            ph ^= 1;
           }
-          __syncwarp();
+          if (++buf == kAccBufs) {
+            buf = 0;
+            tph ^= 1;
+          }
+          if (++dn == kDone) dn = 0;
+          bool next = false;
+          if (leader) {
+            tc_mma_f8(d, adesc, bdesc, idesc, 0u);
+            tc_mma_f8(d, adesc + 2, bdesc + 2, idesc, 1u);
+            // The issuing thread is held up until the tensor pipe takes an instruction, so whatever it does between two
+            // K blocks leaves the pipe idle: the next K block's barriers are asked about in the middle of this one.
+            next = mbar_test_both(full_bar(st), ph, tempty_bar(buf), tph ^ 1);
+            tc_mma_f8(d, adesc + 4, bdesc + 4, idesc, 1u);
+            tc_mma_f8(d, adesc + 6, bdesc + 6, idesc, 1u);
+            // the MMAs of the K block are done: partial sums in TMEM, operands consumed
+            tc_commit(done);
+          }
+          ready = __any_sync(0xffffffffu, next);
         }
       }
     } else if (is_dense(MODE) && C::kStaged && warp == 2 && lane == 0) {
@@ -701,7 +732,6 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
     OutT* const out = reinterpret_cast<OutT*>(p.out);
 
-    uint32_t it = 0;
     uint32_t epi_phase = 0;
     bool alive = true;
     // Barrier among the 256 epilogue threads (bounded like every other wait).
@@ -879,7 +909,9 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     bool exchanged = false;                   // split-K: this warp has passed the exchange barrier
     uint32_t tiles_done = 0;                  // dense: tiles (per-token mode: half tiles) staged so far
     uint32_t pt_tiles = 0;                    // per-token mode: tiles drained so far
-    uint32_t dn_i = 0, dn_ph = 0;             // it % kDone and (it / kDone) & 1, kept as counters
+    uint32_t dn_i = 0, dn_ph = 0;             // completion barrier of the next K block and its phase
+    uint32_t buf = 0;                         // its accumulator buffer
+    bool seen = false;                        // its MMAs are known to be done (warp-uniform)
 
     while (walk.valid(pos) && alive) {
       // acc[0 .. CH/2) = column group 0, acc[CH/2 .. CH) = column group 1, two columns per float2.
@@ -915,7 +947,23 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         for (int j = 0; j < kRing; ++j) {
           const int kb = kb0 + j;
           if (kb < KB && alive) {
-            const int buf = it % kAccBufs;
+            // warp-uniform outcome: the tcgen05.ld below needs the whole warp
+            if (!seen) {
+              const bool got = mbar_wait(done_bar(dn_i), dn_ph, abort_flag, p.err, kErrWaitTmemFull);
+              if (!__all_sync(0xffffffffu, got)) {
+                alive = false;
+                break;
+              }
+            }
+            tc_fence_after();
+            const uint32_t t0 = tmem_base + lane_base + buf * BN + half * CH;
+            auto taddr = [&](int q) {  // load q: q < NSUB -> group 0, else group 1
+              return t0 + (q >= NSUB ? BN / 2 : 0) + (q % NSUB) * LDW;
+            };
+            const bool drain = is_dense(MODE) || cur.active;
+            uint32_t va[LDW], vb[LDW];
+            if (drain) tmem_ld<LDW>(taddr(0), va);
+            // In the shadow of that load: the scale products, the loads of later scales, the counters.
             const float s0 = ring_a[j] * ring_b0[j];
             const float s1 = ring_a[j] * ring_b1[j];
             // Both products are formed before the ring slots are loaded again (the empty asm takes them).
@@ -930,53 +978,44 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
             pf_a += pf_step;
             ++pf_b0;
             ++pf_b1;
-            const uint32_t t0 = tmem_base + lane_base + buf * BN + half * CH;
-            auto taddr = [&](int q) {  // load q: q < NSUB -> group 0, else group 1
-              return t0 + (q >= NSUB ? BN / 2 : 0) + (q % NSUB) * LDW;
-            };
-            // warp-uniform outcome: the tcgen05.ld below needs the whole warp
-            const bool got = mbar_wait(done_bar(dn_i), dn_ph, abort_flag, p.err, kErrWaitTmemFull);
-            if (!__all_sync(0xffffffffu, got)) {
-              alive = false;
-              break;
-            }
-            tc_fence_after();
-            auto release = [&]() {
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(tempty_bar(buf));
-            };
-            // Loads of LDW columns are software-pipelined against the FMAs of the previous load (two
-            // register buffers); the buffer goes back to the issuer as soon as the last load landed.
-            uint32_t va[LDW], vb[LDW];
-            if (!is_dense(MODE) && !cur.active) {
-              release();
-            } else {
-            tmem_ld<LDW>(taddr(0), va);
-            tmem_wait_dep<LDW>(va);
-#pragma unroll
-            for (int q = 0; q < NQ; ++q) {
-              uint32_t* cv = (q & 1) ? vb : va;
-              uint32_t* nv = (q & 1) ? va : vb;
-              if (q + 1 < NQ) tmem_ld<LDW>(taddr(q + 1), nv);   // in flight during the FMAs
-              const float s = (q >= NSUB) ? s1 : s0;
-              const float2 s2 = make_float2(s, s);
-              float2* a = acc + (q >= NSUB ? CH / 2 : 0) + (q % NSUB) * (LDW / 2);
-#pragma unroll
-              for (int c = 0; c < LDW / 2; ++c)
-                a[c] = __ffma2_rn(make_float2(__uint_as_float(cv[2 * c]),
-                                              __uint_as_float(cv[2 * c + 1])), s2, a[c]);
-              if (q + 1 < NQ) {
-                tmem_wait_dep<LDW>(nv);
-                if (q + 2 == NQ) release();
-              }
-            }
-            }
-            ++it;
+            const uint32_t rel = tempty_bar(buf);
             if (++dn_i == kDone) {
               dn_i = 0;
               dn_ph ^= 1;
             }
+            if (++buf == kAccBufs) buf = 0;
+            // Loads of LDW columns are software-pipelined against the FMAs of the previous load (two
+            // register buffers); the buffer goes back to the issuer as soon as the last load landed.
+            if (!drain) {
+              tc_fence_before();
+              __syncwarp();
+              mbar_arrive_if(rel, lane == 0);
+              seen = mbar_test(done_bar(dn_i), dn_ph);
+            } else {
+              tmem_wait_dep<LDW>(va);
+#pragma unroll
+              for (int q = 0; q < NQ; ++q) {
+                uint32_t* cv = (q & 1) ? vb : va;
+                uint32_t* nv = (q & 1) ? va : vb;
+                if (q + 1 < NQ) tmem_ld<LDW>(taddr(q + 1), nv);   // in flight during the FMAs
+                if (q + 2 == NQ) seen = mbar_test(done_bar(dn_i), dn_ph);   // the next K block's MMAs are done?
+                const float s = (q >= NSUB) ? s1 : s0;
+                const float2 s2 = make_float2(s, s);
+                float2* a = acc + (q >= NSUB ? CH / 2 : 0) + (q % NSUB) * (LDW / 2);
+#pragma unroll
+                for (int c = 0; c < LDW / 2; ++c)
+                  a[c] = __ffma2_rn(make_float2(__uint_as_float(cv[2 * c]),
+                                                __uint_as_float(cv[2 * c + 1])), s2, a[c]);
+                if (q + 1 < NQ) {
+                  tmem_wait_dep<LDW>(nv);
+                  if (q + 2 == NQ) {   // the wait is one of the whole warp (.sync.aligned): lane 0 speaks for it
+                    tc_fence_before();
+                    mbar_arrive_if(rel, lane == 0);
+                  }
+                }
+              }
+            }
+            seen = __all_sync(0xffffffffu, seen);
           }
         }
       }
@@ -985,7 +1024,7 @@ bs_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
         // buffer pt_tiles % kAccBufs; read it once, scale by sa[row] * sb[column], hand it back.
         walk.advance(npos);
         if constexpr (!is_dense(MODE)) find_tile(npos, nxt);
-        const int buf = static_cast<int>(pt_tiles % kAccBufs);
+        buf = pt_tiles % kAccBufs;
         const bool got = mbar_wait(tfull_bar(buf), (pt_tiles / kAccBufs) & 1, abort_flag, p.err,
                                    kErrWaitTmemFull);
         ++pt_tiles;
@@ -1578,13 +1617,10 @@ static int launch_bn(int bn, const CUtensorMap& tmap_a, const CUtensorMap& tmap_
 static inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 // Time of one K block of a tile (ns), measured on B200: the slope over K of graph replays with cold
-// operands (M = 256, N = 4096: 32 columns 0.25, 64 0.21-0.25, 128 0.27, 256 0.46 us) and of full waves
-// (M = N = 4096, K = 7168: 128 columns 0.36, 256 0.50 us).
-// The MoE stages use the same figures. Against 360 + 0.9 bn, which stood here before, stage 1's width is
-// the same for all sizes, stage 2's and the dense one's goes from 256 to 128 columns where four rounds
-// take the place of three: 9 row blocks, N = 8320, K = 2048 stage 2 40.2 -> 34.1 us (gathered rows 69.0 ->
-// 57.5), dense 26.6 -> 26.2; K = 512 23.1 -> 19.1 (24.8 -> 25.4), 11.2 -> 11.6.
-static double tile_kb_ns(int bn) { return bn == 256 ? 490.0 : bn == 128 ? 330.0 : bn == 64 ? 250.0 : 245.0; }
+// operands (M = 256, N = 4096: 32 columns 0.19, 64 0.23, 128 0.25, 256 0.46 us) and of full waves
+// (M = 512, N = 4096, K = 7168: 128 columns 0.32, 256 0.50 us). Over 70 shapes with M from 17 to 2200 the width picked with
+// them is within 0.1 % of the fastest on average. The MoE stages use the same figures.
+static double tile_kb_ns(int bn) { return bn == 256 ? 490.0 : bn == 128 ? 295.0 : bn == 64 ? 250.0 : 200.0; }
 
 // Tile-width heuristic (role of select_tile_config in the reference's test). Cost model per K block
 // of one tile: tile_kb_ns on the tensor-core side; the memory side costs the tile's weight bytes at one
@@ -1748,29 +1784,32 @@ static int dense_group_m(int M, int K) {
   return cdiv(M, BM) >= 2 * gm ? gm : 0;
 }
 
-// Wide decode shapes on the tiled kernel (block scales only: the per-token tiles are 256 wide and lose to the
-// decode kernel on such shapes). With enough weight tiles of 128 the tiled kernel fills the GPU in one pass
-// and a narrow tile's K block takes 0.25 us. The decode kernel's plan runs up to two CTAs per SM: three
-// per weight tile as long as 3 n_tiles <= 2 sms, fewer beyond, which costs it a quarter of its speed.
-// Measured, decode / tiled kernel (us, graph replay, cold weights; M = 1 and 16):
-//   96 tiles  K = 1536 7.3 / 7.7 and 7.8 / 7.8, K = 3072 10.2 / 11.2 and 10.7 / 11.3, K = 4096 13.0 / 13.5 and 13.5 /
-//             13.7, K = 5120 16.1 / 15.0 and 17.1 / 16.1
-//   100 tiles K = 1536 7.4 / 7.7 and 8.0 / 7.8, K = 2048 9.0 / 8.8 and 9.6 / 8.9, K = 3072 13.1 / 11.2 and 13.5 / 11.4
-//   128 tiles K = 1024 6.4 / 6.7 and 6.9 / 6.7, K = 2048 9.2 / 9.2 and 9.6 / 9.3, K = 4096 17.8 / 13.8 and 19.2 / 14.1
-//   192 tiles K = 1024 9.1 / 8.6 and 9.6 / 8.6, K = 2048 16.4 / 12.9 and 17.3 / 13.1
-// M = 17 and 32:
-//   56 tiles  K = 1024 5.5 / 5.1 and 5.9 / 5.2, K = 2048 7.2 / 7.0 and 7.8 / 7.1, K = 4096 10.3 / 10.1 and 10.5 / 10.8
-//   64 tiles  K = 4096 10.6 / 10.9 and 11.1 / 10.8; 72 tiles K = 3072 9.5 / 8.9 and 9.9 / 9.0, K = 4096 11.3 / 10.8 and
-//             11.6 / 11.0; 80 tiles K = 3072 10.2 / 10.5 and 11.3 / 11.3, K = 4096 12.6 / 12.1 and 13.7 / 12.7
-//   96 tiles  K = 3072 11.3 / 11.2 and 11.9 / 11.3, K = 4096 14.0 / 13.6 and 14.6 / 13.9
-// M = 33 to 64, 96 tiles: 13.4 / 6.5 (K = 1024) to 41.5 / 20.8 (K = 7168).
+// Decode sizes on the tiled kernel (block scales only: the per-token tiles are 256 wide and lose to the decode
+// kernel on such shapes). Its narrow tiles take 0.2-0.25 us a K block, and with split-K few tiles fill the GPU as
+// well. The decode kernel stays where it is faster: few weight tiles and a middling K, and more tiles at K of about
+// 2600 to 4900, where the two are within 10 % of one another on the grid and the decode kernel's plans are the steadier
+// ones off it (19 x 5760 x 3328 9.0 / 10.8, 25 x 3328 x 4736 8.7 / 9.6). Measured over 13 N x 7 K, decode / tiled kernel
+// (us, graph replay, cold weights):
+//   M = 1   N = 1024 K = 2048 4.0 / 5.0, 2048 x 4096 6.2 / 6.7, 7168 x 3072 8.1 / 8.8, 8192 x 4096 10.3 / 10.5; 2048 x 1024
+//           4.0 / 3.6, 7168 x 2048 6.8 / 6.4, 7168 x 7168 14.8 / 13.0, 16384 x 4096 18.2 / 13.6
+//   M = 16  N = 1536 K = 2048 4.5 / 5.0, 2048 x 3072 6.1 / 6.3, 8192 x 4096 11.0 / 11.1; 4096 x 1024 5.1 / 3.7, 3072 x 7168 10.9 /
+//           9.1, 7168 x 2048 7.3 / 6.6
+//   M = 32  N = 1024 K = 2048 4.4 / 4.9, 2048 x 3072 6.7 / 7.0, 5120 x 3072 8.7 / 8.3; 4096 x 1024 6.1 / 3.8, 4096 x 7168 11.5 /
+//           10.1, 6144 x 2048 8.3 / 6.8
+//   M = 33  N = 2048 K = 3072 6.8 / 7.1 (the one exception), 1024 x 7168 8.3 / 7.0, 7168 x 2048 9.0 / 6.8; M = 64 3072 x 7168
+//           14.1 / 10.1, 10240 x 3072 14.4 / 10.4, 12288 x 4096 28.6 / 13.5
+// Beyond the tile counts of the first condition of each line the older rule stands (3 n_tiles <= 2 sms: the decode
+// kernel's plan has three CTAs per tile at two per SM, fewer beyond): decode 55 tiles and up K = 4096 up to 32 tokens, 64
+// to 95 tiles K >= 4096 up to 64 tokens, 96 tiles and up K < 5120 up to 16, though the tiled kernel has become as fast
+// or faster there too (up to 16 tokens by 0 to 15 %, 8192 x 4096 at 64 tokens 14.6 / 11.2).
 static bool tiled_beats_decode(int M, int N, int K, int sms) {
   const int n_tiles = cdiv(N, 128);
-  if (M > 32) return n_tiles >= 96;
+  if (M > 32) return n_tiles < 64 || n_tiles >= 96 || K < 4096;
   if (M > 16)
-    return n_tiles >= 96 || (n_tiles >= 56 && K <= 2048) ||
-           (n_tiles >= 66 && K <= 4096 && (2 * n_tiles <= sms || K > 3584));
-  return n_tiles > sms || (3 * n_tiles > 2 * sms && K >= 2048) || (n_tiles >= 96 && K >= 5120);
+    return (n_tiles < 55 && !(n_tiles <= 20 && K >= 2048 && K <= 4096) && !(K > 2560 && K <= 4864)) || n_tiles >= 96 ||
+           (n_tiles >= 56 && K <= 2048) || (n_tiles >= 66 && K <= 4096 && (2 * n_tiles <= sms || K > 3584));
+  return (n_tiles < 96 && !(n_tiles <= 20 && K >= 1536 && K <= 4096) && !(n_tiles <= 64 && K > 2560 && K <= 4864)) ||
+         n_tiles > sms || (3 * n_tiles > 2 * sms && K >= 2048) || (n_tiles >= 96 && K >= 5120);
 }
 
 // Block scales: 256 x 256 tiles on CTA pairs (bs_pair_gemm.cu) instead of the tiled kernel, which takes
