@@ -163,7 +163,9 @@ __device__ __forceinline__ void quant_group16(const uint4& raw, uint8_t* __restr
 template <typename T>
 __device__ __forceinline__ void quant_rows16(const T* __restrict__ x, uint8_t* __restrict__ q,
                                              float* __restrict__ scale_t, int64_t rows,
-                                             int64_t scale_stride, int cols, int parts) {
+                                             int64_t scale_stride, int cols, int parts,
+                                             const int* __restrict__ sorted_ids = nullptr, int tokens = 0,
+                                             int topk = 0) {
   constexpr int kInFlight = 4;
   const int groups = cols / 128;
   const int per_part = ((groups + parts - 1) / parts + 7) / 8 * 8;
@@ -174,6 +176,12 @@ __device__ __forceinline__ void quant_rows16(const T* __restrict__ x, uint8_t* _
   const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   for (int64_t item = warp0; item < rows * parts; item += nwarps) {
     const int64_t row = parts == 1 ? item : item / parts;
+    // Rows in routing order: those without a route are left alone (256 experts of 7168 x 2048, 256 tokens in blocks
+    // of 32: three quarters of the rows, 1777 -> 1755 us the layer; 32 tokens in blocks of 16: 583 -> 575).
+    if (sorted_ids) {
+      const int id = __ldg(sorted_ids + row);
+      if ((id & 0xFFFFFF) >= tokens || static_cast<int>(static_cast<unsigned>(id) >> 24) >= topk) continue;
+    }
     const int g_first = static_cast<int>(item - row * parts) * per_part;
     const int g_last = min(groups, g_first + per_part);
     const T* xrow = x + row * cols + sub * 8;
@@ -644,15 +652,16 @@ namespace flyb200 {
 template <typename T>
 __global__ void __launch_bounds__(256)
 quant_1x128_devrows_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale_t,
-                           const int* __restrict__ num_rows_dev, int64_t rows_alloc, int cols, int parts) {
+                           const int* __restrict__ num_rows_dev, int64_t rows_alloc, int cols, int parts,
+                           const int* __restrict__ sorted_ids, int tokens, int topk) {
   const int64_t rows = min(static_cast<int64_t>(num_rows_dev[0]), rows_alloc);
-  quant_rows16<T>(x, q, scale_t, rows, rows_alloc, cols, parts);
+  quant_rows16<T>(x, q, scale_t, rows, rows_alloc, cols, parts, sorted_ids, tokens, topk);
 }
 }  // namespace flyb200
 
-extern "C" int flyb200_quant_1x128_devrows(const void* x, void* q, float* scale_t,
-                                           const int32_t* num_rows_dev, int64_t rows_alloc,
-                                           int32_t cols, int32_t in_dtype, void* stream) {
+static int quant_devrows(const void* x, void* q, float* scale_t, const int32_t* num_rows_dev,
+                         const int32_t* sorted_ids, int tokens, int topk, int64_t rows_alloc, int32_t cols,
+                         int32_t in_dtype, void* stream) {
   if (!x || !q || !scale_t || !num_rows_dev)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "quant_devrows: NULL buffer");
   if ((reinterpret_cast<uintptr_t>(x) % 16) || (reinterpret_cast<uintptr_t>(q) % 8))
@@ -668,10 +677,25 @@ extern "C" int flyb200_quant_1x128_devrows(const void* x, void* q, float* scale_
   const int parts = quant_parts(rows_alloc, cols, sms);
   if (in_dtype == FLYB200_BF16)
     quant_1x128_devrows_kernel<__nv_bfloat16><<<sms * 16, 256, 0, st>>>(
-        static_cast<const __nv_bfloat16*>(x), qo, scale_t, num_rows_dev, rows_alloc, cols, parts);
+        static_cast<const __nv_bfloat16*>(x), qo, scale_t, num_rows_dev, rows_alloc, cols, parts, sorted_ids, tokens,
+        topk);
   else
     quant_1x128_devrows_kernel<__half><<<sms * 16, 256, 0, st>>>(
-        static_cast<const __half*>(x), qo, scale_t, num_rows_dev, rows_alloc, cols, parts);
+        static_cast<const __half*>(x), qo, scale_t, num_rows_dev, rows_alloc, cols, parts, sorted_ids, tokens, topk);
   FLYB200_CUDA_CHECK(cudaGetLastError());
   return FLYB200_OK;
+}
+
+extern "C" int flyb200_quant_1x128_devrows(const void* x, void* q, float* scale_t,
+                                           const int32_t* num_rows_dev, int64_t rows_alloc,
+                                           int32_t cols, int32_t in_dtype, void* stream) {
+  return quant_devrows(x, q, scale_t, num_rows_dev, nullptr, 0, 0, rows_alloc, cols, in_dtype, stream);
+}
+
+extern "C" int flyb200_quant_1x128_routes(const void* x, void* q, float* scale_t, const int32_t* num_rows_dev,
+                                          const int32_t* sorted_ids, int32_t T, int32_t k, int64_t rows_alloc,
+                                          int32_t cols, int32_t in_dtype, void* stream) {
+  if (!sorted_ids || T < 1 || T >= (1 << 24) || k < 1 || k > 255)
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "quant_routes: sorted_ids, T or k");
+  return quant_devrows(x, q, scale_t, num_rows_dev, sorted_ids, T, k, rows_alloc, cols, in_dtype, stream);
 }

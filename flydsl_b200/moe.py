@@ -204,9 +204,9 @@ class BlockscaleMoE:
             else:
                 gemm1(b["out1"], b["x_sorted"], self.w1, b["xs_sorted"], self.w1_scale, sid, seid, sw,
                       npp, T, self.I, self.H, nblk, None)
-                _lib.check(_lib.load().flyb200_quant_1x128_devrows(
+                _lib.check(_lib.load().flyb200_quant_1x128_routes(
                     b["out1"].data_ptr(), b["a2_q"].data_ptr(), b["a2_s"].data_ptr(), npp.data_ptr(),
-                    b["rows"], self.I, mid_code, _lib.stream_handle(None)))
+                    sid.data_ptr(), T, self.topk, b["rows"], self.I, mid_code, _lib.stream_handle(None)))
         else:
             gemm1(b["out1"], x_q, self.w1, x_scale_t, self.w1_scale, sid, seid, sw, npp, T, self.I,
                   self.H, nblk, None)

@@ -286,6 +286,13 @@ int flyb200_quant_pertoken(const void* x, void* q, float* scale, const int32_t* 
 int flyb200_quant_1x128_devrows(const void* x, void* q, float* scale_t, const int32_t* num_rows_dev,
                                 int64_t rows_alloc, int32_t cols, int32_t in_dtype, void* stream);
 
+/* The same for rows in routing order (sorted_ids [rows_alloc] of flyb200_moe_sort for T tokens, top k): rows
+ * without a route are left as they are, and so are their scales. Up to three quarters of a decode batch's rows are
+ * such padding. */
+int flyb200_quant_1x128_routes(const void* x, void* q, float* scale_t, const int32_t* num_rows_dev,
+                               const int32_t* sorted_ids, int32_t T, int32_t k, int64_t rows_alloc,
+                               int32_t cols, int32_t in_dtype, void* stream);
+
 /* Expert-parallel dispatch preparation (new multi-GPU layer, no reference counterpart). For local
  * tokens x [T,H] fp8 with token-major scales x_scale [T,H/128], topk_ids i32 [T,k], topk_weights f32
  * [T,k] and W ranks owning experts_per_rank consecutive experts each: need_out u8 [T,W] (token t
