@@ -589,8 +589,9 @@ extern "C" int flyb200_int4_repack(const int8_t* q, const void* scales, int32_t 
 extern "C" int flyb200_int4_gemm(void* c, const void* a, const void* wq, const void* scales_t, int32_t M,
                                  int32_t N, int32_t K, const flyb200_gemm_cfg* cfg, void* stream) {
   if (!c || !a || !wq || !scales_t) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_gemm: NULL buffer");
-  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(wq)) % 16)
-    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_gemm: a and wq must be 16-byte aligned");
+  // tokens by TMA, packed weights and group scales by bulk copies
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(wq) | reinterpret_cast<uintptr_t>(scales_t)) % 16)
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_gemm: a, wq and scales_t must be 16-byte aligned");
   if (M < 1 || M > 64) return set_error(FLYB200_ERR_UNSUPPORTED, "int4_gemm: 1 <= M <= 64 (got %d)", M);
   if (N < 128 || N % 128 || K < 128 || K % 128)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_gemm: N and K must be multiples of 128 (N=%d K=%d)", N, K);
