@@ -1694,15 +1694,15 @@ const int* max_clusters() {
   return known;
 }
 
-// Split-K plan of a dense problem: the tile width and cluster size with the smallest estimated time, or
-// splits = 1 where the plain tiled kernel is estimated to be as fast. All clusters have to be resident
-// at once (a second wave doubles the time: M = 256, N = 1024, K = 8192 with 16 clusters of eight 18.2
-// us, with 32 of four 10.7). The exchange costs ~3 us and ~50 ns per KB that leaves a CTA. Measured, 56 K
-// blocks, 1 / 2 / 4 CTAs per tile: 12 tiles of 128 columns 20.2 / 15.6 / 11.5 us, 6 tiles of 256 28.0 /
-// 21.2 / 16.1 us, 64 tiles of 128 (two per tile) 16.8 against 17.7 us for 128 unsplit tiles of 64.
 struct SplitPlan {
   int bn, splits, kbps;
 };
+
+// Split-K plan with per-token scales, or of the cluster size that the caller asked for: the tile width and
+// cluster size with the smallest estimated time, or splits = 1 where the plain tiled kernel is estimated to be
+// as fast. All clusters have to be resident at once (a second wave doubles the time: M = 256, N = 1024, K = 8192
+// with 16 clusters of eight 18.2 us, with 32 of four 10.7). The exchange costs ~3 us and ~50 ns per KB that
+// leaves a CTA.
 static SplitPlan pick_split(int M, int N, int K, int sms, bool live, bool pertoken, int force_bn, int force_splits) {
   const int m_blocks = cdiv(M, BM), kbt = K / BK;
   const int rows = M < BM ? M : BM;
@@ -1712,11 +1712,10 @@ static SplitPlan pick_split(int M, int N, int K, int sms, bool live, bool pertok
   double best_cost = 1e30;
   const int* clusters = nullptr;
   if (!force_splits) {
-    const int bn = pertoken ? 256 : pick_block_n(m_blocks, N, sms, false);
-    const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
-    best = SplitPlan{bn, 1, kbt};
-    if (static_cast<long>(m_blocks) * cdiv(N, 256) * 2 > sms) return best;   // no room even for the widest tiles
-    best_cost = ((tiles + sms - 1) / sms) * kbt * kb_ns(bn);
+    const long tiles = static_cast<long>(m_blocks) * cdiv(N, 256);
+    best = SplitPlan{256, 1, kbt};
+    if (tiles * 2 > sms) return best;   // no room
+    best_cost = ((tiles + sms - 1) / sms) * kbt * kb_ns(256);
     // the least that any plan takes: one K block and half of a 64-wide tile exchanged
     if (best_cost <= 3245.0 + 6.4 * rows) return best;
     if (live) clusters = max_clusters();
@@ -1742,6 +1741,90 @@ static SplitPlan pick_split(int M, int N, int K, int sms, bool live, bool pertok
   return best;
 }
 
+// Estimated times (us) of a block-scale call on the tiled kernel. Fitted to 7300 shapes (M 1 to 2200, N 128 to
+// 24576, K 256 to 16384; graph replays with cold weights), each in every width and cluster size and on the decode
+// kernel (decode_us): within 3-4 % of the measured times. Which kernel, width and cluster size a call takes is
+// decided by them alone: what they pick is 0.4 % slower than the fastest on average, in 95 % of the shapes less
+// than 3 %, at most 20 %. (By limits on N and K, with the K blocks' times only: 1.9 %, 8 % and 118 %.)
+struct TileTimes {
+  double fixed, block;   // a call; a K block
+  double rows;           // a full row block instead of one row
+  double bytes;          // the weights, as a multiple of their time at 6.5 TB/s
+  double round, busy;    // each further round of tiles; a K block with every SM at work
+};
+static double unsplit_us(int M, int N, int K, int bn, int sms) {
+  const TileTimes t = bn == 256 ? TileTimes{3.50, 0.407, 1.12, 0.30, 0.96, 0.060}
+                      : bn == 128 ? TileTimes{3.56, 0.197, 0.54, 0.225, 0.97, 0.059}
+                      : bn == 64 ? TileTimes{2.78, 0.166, 0.32, 0.185, 0.55, 0.040}
+                                 : TileTimes{2.16, 0.163, 0.35, 0.216, 0.37, 0.032};
+  const long tiles = static_cast<long>(cdiv(M, BM)) * cdiv(N, bn);
+  const long rounds = (tiles + sms - 1) / sms;
+  const double fill = tiles < sms ? static_cast<double>(tiles) / sms : 1.0;
+  return t.fixed + (t.block * rounds + t.busy * fill) * (K / BK) + t.rows * (M < BM ? M : BM) / BM +
+         t.bytes * (static_cast<double>(N) * K / 6.5e6) + t.round * (rounds - 1);
+}
+struct SplitTimes {
+  double fixed, block;   // a call with its exchange; a K block
+  double kb;             // 1000 bytes that leave a CTA
+  double bytes, fill;    // the weights, as above; all SMs taken
+};
+static double split_us(int M, int N, int K, int bn, int splits, int sms) {
+  const SplitTimes t = bn == 256 ? SplitTimes{3.34, 0.382, 0.0561, 0.244, 3.31}
+                       : bn == 128 ? SplitTimes{3.59, 0.2255, 0.0497, 0.245, 2.06}
+                                   : SplitTimes{3.17, 0.2045, 0.0496, 0.102, 1.675};
+  const long ctas = static_cast<long>(cdiv(M, BM)) * cdiv(N, bn) * splits;
+  const double sent = (M < BM ? M : BM) * bn * 4.0 * (splits - 1) / splits / 1000.0;
+  return t.fixed + t.block * cdiv(K / BK, splits) + t.kb * sent + t.bytes * (static_cast<double>(N) * K / 6.5e6) +
+         t.fill * ctas / sms;
+}
+
+static double pair_us(int M, int N, int K, int ctas) {   // CTA pairs (bs_pair_gemm.cu)
+  const long tiles = static_cast<long>(cdiv(M, 256)) * cdiv(N, 256), pairs = ctas / 2;
+  const long rounds = (tiles + pairs - 1) / pairs;
+  return 5.0 + 0.46 * rounds * (K / BK) + (rounds - 1);
+}
+// Room for two CTAs per tile, at least of the widest. Larger problems run at the pace of their rounds (and of
+// the power cap), which pick_block_n and pair_beats_tiled count.
+static bool in_fitted_range(int M, int N, int sms) {
+  return static_cast<long>(cdiv(M, BM)) * cdiv(N, 256) * 2 <= sms;
+}
+
+// The tiles of a block-scale call that asked for nothing, and their estimated time. Clusters have to be resident
+// all at once.
+static SplitPlan fastest_tiles(int M, int N, int K, int sms, bool live, double& us) {
+  const int m_blocks = cdiv(M, BM), kbt = K / BK;
+  if (!in_fitted_range(M, N, sms)) {
+    const int bn = pick_block_n(m_blocks, N, sms, false);
+    us = unsplit_us(M, N, K, bn, sms);
+    return SplitPlan{bn, 1, kbt};
+  }
+  SplitPlan best{0, 1, kbt};
+  us = 1e30;
+  for (int bn = 32; bn <= 256; bn *= 2) {
+    const double t = unsplit_us(M, N, K, bn, sms);
+    if (t < us) {
+      us = t;
+      best.bn = bn;
+    }
+  }
+  if (us <= 3.4) return best;   // no split is estimated below that
+  const int* clusters = live ? max_clusters() : nullptr;
+  for (int bn = 64; bn <= 256; bn *= 2) {
+    const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
+    for (int sp = 2; sp <= (bn == 256 ? 4 : 8) && tiles * sp <= sms; ++sp) {
+      const int kbps = cdiv(kbt, sp);
+      if (cdiv(kbt, kbps) != sp) continue;   // some CTA would have no K block
+      if (tiles > (clusters ? clusters[sp] : sms / sp)) continue;
+      const double t = 1.01 * split_us(M, N, K, bn, sp, sms);   // as good: no exchange
+      if (t < us) {
+        us = t;
+        best = SplitPlan{bn, sp, kbps};
+      }
+    }
+  }
+  return best;
+}
+
 static int check_ptr(const void* p, size_t align, const char* name) {
   if (!p) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "%s is NULL", name);
   if (reinterpret_cast<uintptr_t>(p) % align)
@@ -1754,6 +1837,7 @@ int launch_decode_gemm(void* c, const void* a, const void* b_repacked, const flo
                        const float* scale_b, int M, int N, int K, int out_dtype, int force_splits,
                        cudaStream_t stream, bool pertoken);
 bool decode_path_pays_off(int M, int N, int K, int sms);
+double decode_us(int M, int N, int K, int sms);
 // moe_swap.cu
 int launch_moe_swap(int stage, bool pertoken, void* out, const void* act, const void* w_repacked,
                     const float* scale_x, const float* scale_w, const int32_t* sorted_ids, const int32_t* expert_ids,
@@ -1782,34 +1866,6 @@ static int dense_group_m(int M, int K) {
   int gm = static_cast<int>((static_cast<size_t>(24) << 20) / (static_cast<size_t>(BM) * K));
   gm = gm < 8 ? 8 : (gm > 64 ? 64 : gm);
   return cdiv(M, BM) >= 2 * gm ? gm : 0;
-}
-
-// Decode sizes on the tiled kernel (block scales only: the per-token tiles are 256 wide and lose to the decode
-// kernel on such shapes). Its narrow tiles take 0.2-0.25 us a K block, and with split-K few tiles fill the GPU as
-// well. The decode kernel stays where it is faster: few weight tiles and a middling K, and more tiles at K of about
-// 2600 to 4900, where the two are within 10 % of one another on the grid and the decode kernel's plans are the steadier
-// ones off it (19 x 5760 x 3328 9.0 / 10.8, 25 x 3328 x 4736 8.7 / 9.6). Measured over 13 N x 7 K, decode / tiled kernel
-// (us, graph replay, cold weights):
-//   M = 1   N = 1024 K = 2048 4.0 / 5.0, 2048 x 4096 6.2 / 6.7, 7168 x 3072 8.1 / 8.8, 8192 x 4096 10.3 / 10.5; 2048 x 1024
-//           4.0 / 3.6, 7168 x 2048 6.8 / 6.4, 7168 x 7168 14.8 / 13.0, 16384 x 4096 18.2 / 13.6
-//   M = 16  N = 1536 K = 2048 4.5 / 5.0, 2048 x 3072 6.1 / 6.3, 8192 x 4096 11.0 / 11.1; 4096 x 1024 5.1 / 3.7, 3072 x 7168 10.9 /
-//           9.1, 7168 x 2048 7.3 / 6.6
-//   M = 32  N = 1024 K = 2048 4.4 / 4.9, 2048 x 3072 6.7 / 7.0, 5120 x 3072 8.7 / 8.3; 4096 x 1024 6.1 / 3.8, 4096 x 7168 11.5 /
-//           10.1, 6144 x 2048 8.3 / 6.8
-//   M = 33  N = 2048 K = 3072 6.8 / 7.1 (the one exception), 1024 x 7168 8.3 / 7.0, 7168 x 2048 9.0 / 6.8; M = 64 3072 x 7168
-//           14.1 / 10.1, 10240 x 3072 14.4 / 10.4, 12288 x 4096 28.6 / 13.5
-// Beyond the tile counts of the first condition of each line the older rule stands (3 n_tiles <= 2 sms: the decode
-// kernel's plan has three CTAs per tile at two per SM, fewer beyond): decode 55 tiles and up K = 4096 up to 32 tokens, 64
-// to 95 tiles K >= 4096 up to 64 tokens, 96 tiles and up K < 5120 up to 16, though the tiled kernel has become as fast
-// or faster there too (up to 16 tokens by 0 to 15 %, 8192 x 4096 at 64 tokens 14.6 / 11.2).
-static bool tiled_beats_decode(int M, int N, int K, int sms) {
-  const int n_tiles = cdiv(N, 128);
-  if (M > 32) return n_tiles < 64 || n_tiles >= 96 || K < 4096;
-  if (M > 16)
-    return (n_tiles < 55 && !(n_tiles <= 20 && K >= 2048 && K <= 4096) && !(K > 2560 && K <= 4864)) || n_tiles >= 96 ||
-           (n_tiles >= 56 && K <= 2048) || (n_tiles >= 66 && K <= 4096 && (2 * n_tiles <= sms || K > 3584));
-  return (n_tiles < 96 && !(n_tiles <= 20 && K >= 1536 && K <= 4096) && !(n_tiles <= 64 && K > 2560 && K <= 4864)) ||
-         n_tiles > sms || (3 * n_tiles > 2 * sms && K >= 2048) || (n_tiles >= 96 && K >= 5120);
 }
 
 // Block scales: 256 x 256 tiles on CTA pairs (bs_pair_gemm.cu) instead of the tiled kernel, which takes
@@ -1860,11 +1916,17 @@ static DensePlan plan_dense(bool pertoken, int M, int N, int K, const flyb200_ge
   const int path = cfg ? cfg->path : 0, block_n = cfg ? cfg->block_n : 0;
   const int max_ctas = cfg ? cfg->max_ctas : 0, split_k = cfg ? cfg->split_k : 0;
   DensePlan plan{1, 0, 1, K / BK, 0};
+  const int m_blocks = cdiv(M, BM);
+  SplitPlan split{0, 1, K / BK};
+  // Block scales and nothing asked for: what is estimated to be fastest. (The per-token tiles are 256 wide and lose
+  // to the decode kernel wherever it runs in one wave.)
+  const bool any = !pertoken && path == 0 && !block_n && !max_ctas && !split_k;
+  double us = 0.0;
+  if (any) split = fastest_tiles(M, N, K, sms, live, us);
   // Decode-size M: the swap-AB split-K kernel (decode_gemm.cu; per-token: the token's scale on every K
-  // block, the channel's once), unless a tile width or the tiled path was asked for, or the shape is
-  // wide and nothing was asked for that the tiled kernel would not honour.
-  const bool wide = !pertoken && !split_k && !max_ctas && tiled_beats_decode(M, N, K, sms);
-  if (path == 2 || (path == 0 && M <= 64 && !block_n && !wide && decode_path_pays_off(M, N, K, sms))) {
+  // block, the channel's once). It is the one that a cluster size or a limit on the CTAs is meant for.
+  if (path == 2 || (path == 0 && M <= 64 && !block_n &&
+                    (any ? decode_us(M, N, K, sms) < us : decode_path_pays_off(M, N, K, sms)))) {
     plan.kernel = 2;
     return plan;
   }
@@ -1874,28 +1936,30 @@ static DensePlan plan_dense(bool pertoken, int M, int N, int K, const flyb200_ge
     plan.kernel = 3;
     return plan;
   }
-  const int m_blocks = cdiv(M, BM);
-  SplitPlan split{0, 1, K / BK};
   if (path == 1 && split_k > 1 && block_n != 32) {
     split = pick_split(M, N, K, sms, live, pertoken, pertoken ? 256 : block_n, split_k);
     // a limit on the CTAs comes before the split: its clusters have no persistent loop
     if (max_ctas > 0 && static_cast<long>(m_blocks) * cdiv(N, split.bn ? split.bn : 256) * split.splits > max_ctas)
       split = SplitPlan{0, 1, K / BK};
-  } else if (path == 0 && !block_n && !max_ctas && !split_k) {
-    split = pick_split(M, N, K, sms, live, pertoken, pertoken ? 256 : 0, 0);
+  } else if (pertoken && path == 0 && !block_n && !max_ctas && !split_k) {
+    split = pick_split(M, N, K, sms, live, true, 256, 0);
   }
   plan.splits = split.splits;
   plan.kbps = split.kbps;
-  plan.bn = pertoken ? 256 : block_n ? block_n : split.splits > 1 ? split.bn : pick_block_n(m_blocks, N, sms, false);
+  const int wide = pertoken || block_n ? 0 : pick_block_n(m_blocks, N, sms, false);   // of many tiles
+  plan.bn = pertoken ? 256 : block_n ? block_n : any || split.splits > 1 ? split.bn : wide;
   const long tiles = static_cast<long>(m_blocks) * cdiv(N, plan.bn);
   plan.grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
-  if (!pertoken && path == 0 && !block_n && !split_k && split.splits == 1 && plan.grid >= 2 &&
-      pair_beats_tiled(M, N, K / BK, plan.grid, ((tiles + plan.grid - 1) / plan.grid) * tile_kb_ns(plan.bn))) {
-    const long pairs = static_cast<long>(cdiv(M, 256)) * cdiv(N, 256);
-    plan.kernel = 3;
-    plan.bn = 256;
-    plan.grid = 2 * static_cast<int>(pairs < plan.grid / 2 ? pairs : plan.grid / 2);
-    return plan;
+  if (!pertoken && path == 0 && !block_n && !split_k && plan.grid >= 2) {
+    const long wide_tiles = static_cast<long>(m_blocks) * cdiv(N, wide);
+    if (pair_beats_tiled(M, N, K / BK, plan.grid, ((wide_tiles + plan.grid - 1) / plan.grid) * tile_kb_ns(wide)) &&
+        !(any && in_fitted_range(M, N, sms) && us < pair_us(M, N, K, plan.grid))) {
+      const long pairs = static_cast<long>(cdiv(M, 256)) * cdiv(N, 256);
+      plan.kernel = 3;
+      plan.bn = 256;
+      plan.grid = 2 * static_cast<int>(pairs < plan.grid / 2 ? pairs : plan.grid / 2);
+      return plan;
+    }
   }
   if (split.splits > 1) plan.grid = static_cast<int>(tiles * split.splits);
   else if (tiles < plan.grid) plan.grid = static_cast<int>(tiles);

@@ -430,16 +430,33 @@ static int launch_decode(const CUtensorMap& tmap, const DecodeParams& p, int n_t
   return FLYB200_OK;
 }
 
-// Whether the automatic dispatch should take the decode kernel (measured on B200): it wins when all
-// of its CTAs are resident at once (one wave) -- with more than 32 tokens only if K is deep enough
-// (>= 32 blocks) for split-K to matter; wide-N shapes that need several waves run faster on the
-// persistent tiled kernel.
+// Per-token scales, and calls with a request: whether to take the decode kernel (measured on B200). It wins when
+// all of its CTAs are resident at once (one wave) -- with more than 32 tokens only if K is deep enough (>= 32
+// blocks) for split-K to matter; wide-N shapes that need several waves run faster on the persistent tiled kernel.
 bool decode_path_pays_off(int M, int N, int K, int sms) {
   if (M > 64) return false;
   const DecodePlan plan = plan_decode(M, N, K, sms, 0);
   if (plan.splits < 1 || plan.rounds != 1) return false;
   if (M > 32 && K / 128 < 32) return false;
   return true;
+}
+
+// Estimated time (us) of a block-scale call on this kernel, where its CTAs are resident at once: the counterpart of
+// the tiled kernel's estimates in blockscale_gemm.cu, fitted to the same shapes (2700 of them where this kernel is
+// within a quarter of the fastest; 4 % off on average, 15 % at most).
+double decode_us(int M, int N, int K, int sms) {
+  if (M > 64) return 1e30;
+  const DecodePlan plan = plan_decode(M, N, K, sms, 0);
+  if (plan.splits < 1 || plan.rounds != 1) return 1e30;
+  const double ctas = static_cast<double>((N + 127) / 128) * plan.splits;
+  const double weights = static_cast<double>(N) * K / 6.5e6;   // their time at 6.5 TB/s
+  const double full = static_cast<double>(M) / plan.nt;
+  const double wide = plan.splits > 6 ? 1.0 : 0.0;             // fewer clusters of seven and eight fit the GPU
+  switch (plan.nt) {
+    case 16: return 2.51 + 0.436 * plan.kbps + 0.33 * full + 0.71 * weights + 0.58 * ctas / sms + 0.19 * wide;
+    case 32: return 2.46 + 0.455 * plan.kbps + 0.64 * full + 0.73 * weights + 0.79 * ctas / sms + 0.15 * wide;
+    default: return 2.54 + 0.463 * plan.kbps + 1.52 * full + 0.91 * weights + 0.86 * ctas / sms + 0.09 * wide;
+  }
 }
 
 // Entry used by flyb200_blockscale_gemm for M <= 64.

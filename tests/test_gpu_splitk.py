@@ -78,11 +78,12 @@ def test_split_k_pertoken(M, N, K):
 
 
 # Decode-size M on both sides of the lines between the decode and the tiled kernel
-@pytest.mark.parametrize("M,N,K,kernel", [(1, 12288, 256, DECODE), (16, 12688, 2048, TILED), (16, 12544, 2048, DECODE),
-                                          (16, 12688, 1920, DECODE), (8, 12288, 5120, TILED), (1, 19072, 256, TILED),
-                                          (17, 7168, 512, TILED), (32, 7056, 512, TILED), (17, 7040, 512, DECODE),
-                                          (32, 7168, 4224, DECODE), (32, 8448, 2304, TILED), (20, 8320, 2304, DECODE),
-                                          (24, 9600, 2304, DECODE), (33, 12288, 4096, TILED), (33, 12160, 4096, DECODE)])
+@pytest.mark.parametrize("M,N,K,kernel", [(1, 1152, 1024, DECODE), (1, 1536, 1024, TILED), (1, 12288, 256, TILED),
+                                          (1, 19072, 256, DECODE), (8, 12288, 5120, TILED), (16, 2688, 2048, DECODE),
+                                          (16, 3216, 2048, TILED), (16, 12688, 1920, TILED), (17, 1040, 3072, DECODE),
+                                          (17, 7040, 512, TILED), (32, 1552, 2048, DECODE), (32, 2192, 2048, TILED),
+                                          (32, 7168, 4224, TILED), (24, 9600, 2304, TILED), (33, 768, 2048, DECODE),
+                                          (33, 1536, 2048, TILED), (33, 12160, 4096, TILED)])
 def test_decode_or_tiled(M, N, K, kernel):
     from flydsl_b200 import _lib
     from flydsl_b200.kernels import compile_blockscale_preshuffle_gemm

@@ -33,7 +33,7 @@ def test_tiled_counters(M, N, K, max_ctas, block_n):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 1024), (8, 7168, 2048), (16, 2688, 1408), (16, 8192, 5120), (17, 6912, 2560),
-                                   (32, 1024, 1920), (32, 2560, 4992), (33, 7168, 7168), (64, 10240, 3968),
+                                   (32, 2192, 1920), (32, 2560, 4992), (33, 7168, 7168), (64, 10240, 3968),
                                    (64, 1040, 7168)])
 def test_decode_sizes_on_the_tiled_kernel_equal_the_decode_kernel(M, N, K):
     """Both edges of each token range of the dispatch rule; the two kernels differ in the order of sums over K."""
