@@ -488,12 +488,12 @@ const int* max_clusters();   // blockscale_gemm.cu
 // tokens 0.45 us for a group of each; a wave costs 3 us (4 with more than 16 tokens), a larger cluster a little.
 // Clusters that are not all resident make another wave (2048 x 2048, 64 tokens, 16 clusters of 8: 11.6 us, of 4:
 // 6.1). The plan is within 1 % of the best cluster size on average (worst 14 %).
-static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits) {
+static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits, bool live) {
   I4Plan best{0, 0, 0, 0};
   const int nt = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
   const int n_tiles = N / 128;
   const int KBt = K / 128;
-  const int* clusters = max_clusters();
+  const int* clusters = live ? max_clusters() : nullptr;   // otherwise estimated
   double best_cost = 1e30;
   for (int s = 1; s <= 8; ++s) {
     if (force_splits > 0 && s != force_splits) continue;
@@ -502,7 +502,7 @@ static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits) {
     if (s_eff != s && force_splits <= 0) continue;
     const int slots = nt == 16 ? i4_slots<16>(kbps) : nt == 32 ? i4_slots<32>(kbps) : i4_slots<64>(kbps);
     if (!slots) continue;
-    int alone = s == 1 ? sms : clusters[s];   // clusters at one CTA per SM
+    int alone = s > 1 && clusters ? clusters[s] : sms / s;   // clusters at one CTA per SM
     if (alone < 1) alone = 1;
     const int resident = nt <= 32 ? 2 * alone : alone;
     const int full = n_tiles / resident, rest = n_tiles % resident;
@@ -586,6 +586,22 @@ extern "C" int flyb200_int4_repack(const int8_t* q, const void* scales, int32_t 
   return FLYB200_OK;
 }
 
+extern "C" int flyb200_int4_tensor_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t sms,
+                                        int32_t* plan) {
+  if (!plan || M < 1 || M > 64 || N < 128 || N % 128 || K < 128 || K % 128)
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_tensor_plan: bad arguments (M=%d N=%d K=%d)", M, N, K);
+  const bool live = sms <= 0;
+  if (live && (sms = sm_count()) <= 0) return FLYB200_ERR_CUDA;
+  const I4Plan p = plan_int4(M, N, K, sms, split_k, live);
+  plan[0] = p.splits < 1 || stream_beats_tensor(M, N, K) ? 1 : 2;
+  plan[1] = p.nt; plan[2] = p.splits; plan[3] = p.kbps; plan[4] = p.slots;
+  plan[5] = p.splits < 1 ? 0 : p.nt == 16 ? I4Cfg<16>::smem_bytes(p.slots, p.kbps)
+                           : p.nt == 32 ? I4Cfg<32>::smem_bytes(p.slots, p.kbps)
+                                        : I4Cfg<64>::smem_bytes(p.slots, p.kbps);
+  plan[6] = p.splits < 1 ? 0 : p.nt == 64 ? I4Cfg<64>::kTmemCols : I4Cfg<16>::kTmemCols;
+  return FLYB200_OK;
+}
+
 extern "C" int flyb200_int4_gemm(void* c, const void* a, const void* wq, const void* scales_t, int32_t M,
                                  int32_t N, int32_t K, const flyb200_gemm_cfg* cfg, void* stream) {
   if (!c || !a || !wq || !scales_t) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_gemm: NULL buffer");
@@ -602,7 +618,7 @@ extern "C" int flyb200_int4_gemm(void* c, const void* a, const void* wq, const v
   if (sms <= 0) return FLYB200_ERR_CUDA;
   I4Plan plan{0, 0, 0, 0};
   if (path == 2 || (path == 0 && !stream_beats_tensor(M, N, K)))
-    plan = plan_int4(M, N, K, sms, cfg ? cfg->split_k : 0);
+    plan = plan_int4(M, N, K, sms, cfg ? cfg->split_k : 0, true);
   if (path == 2 && plan.splits < 1)
     return set_error(FLYB200_ERR_INVALID_ARGUMENT, "int4_gemm: no plan for M=%d N=%d K=%d", M, N, K);
   if (plan.splits < 1)   // (also K ranges whose group scales leave no room for this kernel's ring)

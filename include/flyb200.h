@@ -381,6 +381,11 @@ int flyb200_int4_gemm(void* c, const void* a, const void* wq, const void* scales
  * Host only; split_k as in the cfg. */
 int flyb200_int4_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t sms, int32_t* plan);
 
+/* The same for the tcgen05 kernel (path 2): plan[0] the kernel that path 0 takes (1 or 2), [1] token columns, [2] CTAs
+ * per cluster (0: no plan), [3] K groups per CTA, [4] ring slots (two sets of dequantisers take every other group),
+ * [5] bytes of shared memory and [6] tensor memory columns of a CTA. */
+int flyb200_int4_tensor_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t sms, int32_t* plan);
+
 /* Masked top-k reduce of the local experts' route rows (the arithmetic of flyb200_moe_reduce with a
  * valid_mask) whose result rows go straight into the owners' memory: row i of routes' [W*T, k, H]
  * belongs to source rank i / T, slot i % T and is stored at row rank*T + slot of that rank's back area

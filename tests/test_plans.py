@@ -50,6 +50,42 @@ def test_int4_two_sets_only_where_every_cta_has_an_sm(M):
     assert seen == ({1, 2} if M <= 32 else {1})
 
 
+def _int4_tensor_plan(M, N, K, split_k=0, sms=SMS):
+    from flydsl_b200 import _lib
+
+    plan = (ctypes.c_int32 * 7)()
+    _lib.check(_lib.load().flyb200_int4_tensor_plan(M, N, K, split_k, sms, plan))
+    return dict(zip(("kernel", "cols", "splits", "groups", "slots", "smem", "tmem"), plan))
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("split_k", [0, 1, 3, 8])
+def test_int4_tensor_rings(M, split_k):
+    """The tcgen05 kernel's plans. A ring that wraps is even, so that a slot's groups all belong to one of the two sets
+    of dequantisers (see test_int4_ring_slots_belong_to_one_set); it fits the SM, or half of it where two CTAs are to
+    share one; the groups of a cluster cover K; and every size has a plan for one of the two kernels."""
+    wrapped, kernels = 0, set()
+    for N in range(128, 16385, 768):
+        for K in list(range(128, 16385, 128)) + list(range(16512, 131072, 3200)):
+            plan = _int4_tensor_plan(M, N, K, split_k)
+            if plan["splits"] == 0:
+                assert plan["kernel"] == 1
+            else:
+                groups, slots = plan["groups"], plan["slots"]
+                assert plan["cols"] == (16 if M <= 16 else 32 if M <= 32 else 64)
+                assert min(2, groups) <= slots <= min(16, groups) and (slots == groups or slots % 2 == 0)
+                assert (plan["splits"] - 1) * groups < K // 128 <= plan["splits"] * groups
+                assert plan["smem"] <= 232448
+                if M <= 32 and groups <= 64:
+                    assert 2 * (plan["smem"] + 1024) <= 233472
+                wrapped += groups > slots
+                assert M <= 32 or plan["kernel"] == 2
+            if plan["kernel"] == 1 and split_k == 0:
+                assert _int4_plan(M, N, K, 0)[2] > 0
+            kernels.add(plan["kernel"])
+    assert wrapped > 100 and 2 in kernels and (M > 32 or 1 in kernels)
+
+
 def _kernel_source(name):
     import os
     import re
