@@ -487,7 +487,9 @@ const int* max_clusters();   // blockscale_gemm.cu
 // all cluster sizes (graph replay, cold weights): a CTA alone on an SM takes about 0.25 us a group, two of up to 32
 // tokens 0.45 us for a group of each; a wave costs 3 us (4 with more than 16 tokens), a larger cluster a little.
 // Clusters that are not all resident make another wave (2048 x 2048, 64 tokens, 16 clusters of 8: 11.6 us, of 4:
-// 6.1). The plan is within 1 % of the best cluster size on average (worst 14 %).
+// 6.1). Over 2600 drawn shapes the plan is within 1.4 % of the best cluster size on average, more than 10 % off in 74.
+// A term for the cluster size of 0.2 instead of 0.05 at 64 tokens left small problems in too few CTAs (57 x 256 x 768
+// in clusters of three 5.6 us, of six 4.6).
 static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits, bool live) {
   I4Plan best{0, 0, 0, 0};
   const int nt = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
@@ -507,7 +509,7 @@ static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits, bool liv
     const int resident = nt <= 32 ? 2 * alone : alone;
     const int full = n_tiles / resident, rest = n_tiles % resident;
     const double wave = nt == 16 ? 3.0 : 4.0;
-    double cost = full * (wave + kbps * (nt <= 32 ? 0.45 : 0.25)) + (nt == 64 ? 0.2 : 0.1) * s;
+    double cost = full * (wave + kbps * (nt <= 32 ? 0.45 : 0.25)) + (nt == 64 ? 0.05 : 0.1) * s;
     if (rest) cost += wave + kbps * (rest <= alone ? 0.25 : 0.45);
     if (cost < best_cost - 1e-9) {
       best_cost = cost;
@@ -525,10 +527,14 @@ static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits, bool liv
 //           2048 5.07 / 4.71, 8192 x 8192 19.2 / 12.4
 //   M = 32  3072 x 1024 4.25 / 4.52, 5120 x 1024 5.29 / 5.47; 1536 x 1536 4.76 / 4.62, 8192 x 8192 23.4 / 13.3
 //   M = 64  1024 x 1024 6.03 / 5.25, 8192 x 8192 35.1 / 18.6
+// The limits were drawn again from 2280 shapes of up to 32 tokens: with them the choice is 1 % slower than the faster
+// kernel on average, and of calls that used to take the mma.sync kernel two in a thousand lose more than 5 % (8 x 6656 x
+// 1280 4.7 / 5.4, 12 x 27904 x 384 5.2 / 5.7, 2 x 1664 x 5120 4.7 / 5.0, 32 x 17664 x 384 5.4 / 5.9 had). Beyond K = 5120
+// the tcgen05 kernel is never slower (5 to 13 % faster, whatever N).
 static bool stream_beats_tensor(int M, int N, int K) {
   const double weights = static_cast<double>(N) * K;
-  if (M <= 16) return weights < (K <= 1024 ? 1e7 : 8e6);
-  return M <= 32 && K <= 1024 && weights < 6e6;
+  if (M <= 16) return K <= 5120 && weights < (K <= 1280 ? 1.1e7 : 8.7e6);
+  return M <= 32 && K <= 1024 && weights < (K <= 384 ? 7e6 : 5e6);
 }
 
 template <int NT>
