@@ -92,6 +92,7 @@ SIGNATURES = {
     "flyb200_int4_gemm": (c_int, [c_void_p] * 4 + [c_int32] * 3 + [POINTER(GemmCfg), c_void_p]),
     "flyb200_gemm_plan": (c_int, [c_int32] * 4 + [POINTER(GemmCfg), c_int32, POINTER(c_int32)]),
     "flyb200_int4_plan": (c_int, [c_int32] * 5 + [POINTER(c_int32)]),
+    "flyb200_decode_plan": (c_int, [c_int32] * 5 + [POINTER(c_int32)]),
     "flyb200_int4_tensor_plan": (c_int, [c_int32] * 5 + [POINTER(c_int32)]),
     "flyb200_query_device_error": (c_int, [c_void_p, POINTER(c_int32)]),
     "flyb200_last_error_string": (c_char_p, []),

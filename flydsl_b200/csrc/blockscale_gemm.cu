@@ -128,6 +128,7 @@ struct Cfg {
   static constexpr int kRingBytes = SPLIT ? kAvail : kStages * kStageBytes;
   static constexpr int kSmemBytes = kRingBytes + kCBytes + kMiscBytes + 1024;
   static_assert(kStages >= 3, "pipeline too shallow");
+  static_assert(!SPLIT || kSmemBytes >= tmem_share_bytes(kTmemCols), "tensor memory beside another cluster kernel");
 };
 
 template <typename OutT>

@@ -54,7 +54,7 @@ constexpr int kBufs = 2;                         // accumulator buffers per colu
 // producer has seen its previous phase
 constexpr int kDone = kStages + kBufs;
 constexpr int kHalfWarps = 4;                    // epilogue warps per column half
-static_assert(kSmem <= 232448, "shared memory");
+static_assert(kSmem <= 232448 && kSmem >= tmem_share_bytes(512), "shared memory");
 
 struct Params {
   const uint8_t* b;

@@ -224,6 +224,12 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // ---- tcgen05 -----------------------------------------------------------------------------------
+// The least dynamic shared memory of a CTA that holds `cols` of an SM's 512 columns of tensor memory: the same
+// share of its 228 KB (1 KB of which goes to the system per CTA). An allocation waits until enough columns are free,
+// without a limit, and only shared memory, registers and threads keep CTAs off an SM. Two clusters of two streams
+// could so hold columns on one SM each and wait for those on the other's. With every cluster kernel's CTAs at this
+// size or above, whatever is resident together finds its columns.
+constexpr int tmem_share_bytes(int cols) { return 233472 / 512 * cols - 1024; }
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t cols) {
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem),
                "r"(cols)

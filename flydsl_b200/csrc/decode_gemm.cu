@@ -63,7 +63,8 @@ struct DecCfg {
   static constexpr int kScaleBytes = kDecMaxStages * 2 * (NT + 1) * 4 + 64;  // generous
   static constexpr int kMiscBytes = 1024;
   static int smem_bytes(int stages, int kbps) {
-    return ring_bytes(stages) + (kbps * (NT + 1) * 4 + 64) + kMiscBytes + 1024;
+    const int bytes = ring_bytes(stages) + (kbps * (NT + 1) * 4 + 64) + kMiscBytes + 1024;
+    return bytes > tmem_share_bytes(kTmemCols) ? bytes : tmem_share_bytes(kTmemCols);
   }
 };
 
@@ -458,6 +459,24 @@ double decode_us(int M, int N, int K, int sms) {
     default: return 2.54 + 0.463 * plan.kbps + 1.52 * full + 0.91 * weights + 0.86 * ctas / sms + 0.09 * wide;
   }
 }
+
+}  // namespace flyb200
+
+extern "C" int flyb200_decode_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t sms, int32_t* out) {
+  using namespace flyb200;
+  if (!out || M < 1 || M > 64 || N < 16 || N % 16 || K < 128 || K % 128)
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "decode_plan: bad arguments (M=%d N=%d K=%d)", M, N, K);
+  if (sms <= 0 && (sms = sm_count()) <= 0) return FLYB200_ERR_CUDA;
+  const DecodePlan p = plan_decode(M, N, K, sms, split_k);
+  out[0] = p.nt; out[1] = p.splits; out[2] = p.kbps; out[3] = p.stages;
+  out[4] = p.splits < 1 ? 0 : p.nt == 16 ? DecCfg<16>::smem_bytes(p.stages, p.kbps)
+                          : p.nt == 32 ? DecCfg<32>::smem_bytes(p.stages, p.kbps)
+                                       : DecCfg<64>::smem_bytes(p.stages, p.kbps);
+  out[5] = p.splits < 1 ? 0 : p.nt == 16 ? DecCfg<16>::kTmemCols : p.nt == 32 ? DecCfg<32>::kTmemCols : DecCfg<64>::kTmemCols;
+  return FLYB200_OK;
+}
+
+namespace flyb200 {
 
 // Entry used by flyb200_blockscale_gemm for M <= 64.
 int launch_decode_gemm(void* c, const void* a, const void* b_repacked, const float* scale_a_t,

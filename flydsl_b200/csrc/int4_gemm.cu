@@ -114,7 +114,10 @@ struct I4Cfg {
   }
   // + the group scales of the CTA's K range: [kbps][128] bf16
   static int fixed_bytes(int kbps) { return kRecvBytes + kbps * 256 + kMiscBytes + 1024; }
-  static int smem_bytes(int slots, int kbps) { return ring_bytes(slots) + fixed_bytes(kbps); }
+  static int smem_bytes(int slots, int kbps) {
+    const int bytes = ring_bytes(slots) + fixed_bytes(kbps);
+    return bytes > tmem_share_bytes(kTmemCols) ? bytes : tmem_share_bytes(kTmemCols);
+  }
 };
 
 template <int NT>
@@ -468,7 +471,7 @@ static int i4_slots(int kbps) {
   using C = I4Cfg<NT>;
   const int least = kbps < 2 ? kbps : 2;
   // half of an SM's shared memory where two CTAs are to share it, all of it where that does not do
-  for (int limit : {C::kHalfSm ? 233472 / 2 - 1024 : 232448, 232448}) {
+  for (int limit : {tmem_share_bytes(C::kTmemCols), 232448}) {
     int slots = (limit - C::fixed_bytes(kbps)) / C::kSlotBytes;
     slots = slots < kbps ? slots : kbps;
     if (slots > kI4MaxSlots) slots = kI4MaxSlots;

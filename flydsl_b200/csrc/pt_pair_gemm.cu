@@ -36,6 +36,7 @@ constexpr int kPRegionBytes = 128 * 128;        // 128 rows x 64 bf16
 constexpr int kPStagingBytes = 2 * kPRegionBytes;   // half a tile: 128 rows x 128 columns
 constexpr int kPMisc = 2048;
 constexpr int kPSmem = kPStages * kPStageBytes + kPStagingBytes + kPMisc + 1024;
+static_assert(kPSmem >= tmem_share_bytes(512), "tensor memory beside another cluster kernel");
 constexpr int kPAccBufs = 2;
 constexpr int kPEpiWarps = 8;
 

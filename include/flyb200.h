@@ -386,6 +386,11 @@ int flyb200_int4_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t 
  * [5] bytes of shared memory and [6] tensor memory columns of a CTA. */
 int flyb200_int4_tensor_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t sms, int32_t* plan);
 
+/* What the decode kernel of the dense GEMMs (cfg.path 2, M <= 64) plans: plan[0] token columns, [1] CTAs per cluster
+ * (0: no plan), [2] K blocks per CTA, [3] pipeline stages, [4] bytes of shared memory and [5] tensor memory columns of a
+ * CTA. Host only. */
+int flyb200_decode_plan(int32_t M, int32_t N, int32_t K, int32_t split_k, int32_t sms, int32_t* plan);
+
 /* Masked top-k reduce of the local experts' route rows (the arithmetic of flyb200_moe_reduce with a
  * valid_mask) whose result rows go straight into the owners' memory: row i of routes' [W*T, k, H]
  * belongs to source rank i / T, slot i % T and is stored at row rank*T + slot of that rank's back area

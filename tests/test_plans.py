@@ -86,6 +86,32 @@ def test_int4_tensor_rings(M, split_k):
     assert wrapped > 100 and 2 in kernels and (M > 32 or 1 in kernels)
 
 
+def _decode_plan(M, N, K, split_k=0, sms=SMS):
+    from flydsl_b200 import _lib
+
+    plan = (ctypes.c_int32 * 6)()
+    _lib.check(_lib.load().flyb200_decode_plan(M, N, K, split_k, sms, plan))
+    return dict(zip(("cols", "splits", "groups", "stages", "smem", "tmem"), plan))
+
+
+@pytest.mark.parametrize("plan_of", [_int4_tensor_plan, _decode_plan])
+@pytest.mark.parametrize("split_k", [0, 1, 8])
+def test_resident_ctas_of_cluster_kernels_find_their_tensor_memory(plan_of, split_k):
+    """A CTA takes its columns of tensor memory by an instruction that waits without a limit, and then meets its cluster.
+    Two streams could wait for one another's columns in a circle unless shared memory (228 KB an SM, 1 KB of it taken by
+    every CTA) keeps CTAs apart that ask for more than the 512 columns together: registers do so by chance only."""
+    seen = set()
+    for M in (1, 16, 17, 32, 33, 64):
+        for N in (128, 1024, 8192, 24576):
+            for K in (128, 256, 512, 1024, 2048, 4096, 8192, 32768):
+                plan = plan_of(M, N, K, split_k)
+                if plan["splits"]:
+                    assert (plan["smem"] + 1024) * 512 >= 233472 * plan["tmem"], (M, N, K, plan)
+                    assert plan["smem"] <= 232448
+                    seen.add(plan["tmem"])
+    assert seen == ({64, 128, 256} if plan_of is _decode_plan else {256, 512})
+
+
 # M, N, K; time (us) of the mma.sync kernel, of the tcgen05 one (graph replays, cold weights)
 INT4_SIZES = [
     (11, 20480, 256, 4.2, 4.8), (14, 4096, 3328, 6.9, 5.5), (13, 7552, 2048, 6.7, 5.7), (2, 2688, 4608, 6.1, 5.2),
