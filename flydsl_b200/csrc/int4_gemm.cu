@@ -486,13 +486,33 @@ static int i4_slots(int kbps) {
 
 const int* max_clusters();   // blockscale_gemm.cu
 
-// K splits (cluster size) and ring depth: the smallest estimated time. Measured over 12 N x 7 K x M = 1, 16, 32, 64 and
-// all cluster sizes (graph replay, cold weights): a CTA alone on an SM takes about 0.25 us a group, two of up to 32
-// tokens 0.45 us for a group of each; a wave costs 3 us (4 with more than 16 tokens), a larger cluster a little.
-// Clusters that are not all resident make another wave (2048 x 2048, 64 tokens, 16 clusters of 8: 11.6 us, of 4:
-// 6.1). Over 2600 drawn shapes the plan is within 1.4 % of the best cluster size on average, more than 10 % off in 74.
-// A term for the cluster size of 0.2 instead of 0.05 at 64 tokens left small problems in too few CTAs (57 x 256 x 768
-// in clusters of three 5.6 us, of six 4.6).
+// Estimated time (us) of the tcgen05 kernel, fitted to 2600 shapes (M 1 to 64, N and K from 128 up; graph replays, cold
+// weights), each in every cluster size: 4-6 % off while all CTAs are resident. A CTA alone on an SM takes about
+// 0.31 us a group, two of up to 32 tokens 0.48 us for a group of each. Clusters that are not all resident make another
+// wave (2048 x 2048, 64 tokens, 16 clusters of 8: 11.6 us, of 4: 6.1).
+struct I4Times {
+  double fixed, group;   // a call, a K group of every CTA
+  double fill, store;    // all SMs taken (or taken twice); the outputs stored by one CTA per tile instead of by many
+};
+static double int4_us(int nt, int n_tiles, int kbps, int splits, int alone, int sms) {
+  const bool two = nt <= 32;   // CTAs per SM
+  const int resident = two ? 2 * alone : alone;
+  double us = 0.0;
+  if (n_tiles > resident) {
+    us = n_tiles / resident * (nt == 16 ? 4.66 + 0.479 * kbps : nt == 32 ? 5.9 + 0.503 * kbps : 5.6 + 0.36 * kbps);
+    n_tiles %= resident;
+    if (!n_tiles) return us;
+  }
+  const I4Times t = n_tiles <= alone ? (nt == 16 ? I4Times{2.55, 0.306, 0.96, 0.0}
+                                        : nt == 32 ? I4Times{3.03, 0.334, 0.71, 0.94}
+                                                   : I4Times{3.57, 0.355, 1.50, 1.03})
+                                     : (nt == 16 ? I4Times{1.70, 0.479, 1.48, 0.0} : I4Times{2.10, 0.503, 1.71, 0.65});
+  return us + t.fixed + t.group * kbps + t.fill * n_tiles * splits / sms + t.store / splits +
+         (nt == 64 && splits > 6 ? 0.4 : 0.0);   // clusters of seven and eight place badly
+}
+
+// K splits (cluster size) and ring depth: the smallest estimated time; within 1 % of the best cluster size on average
+// over those shapes, more than 10 % off in 27 of them.
 static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits, bool live) {
   I4Plan best{0, 0, 0, 0};
   const int nt = M <= 16 ? 16 : (M <= 32 ? 32 : 64);
@@ -509,11 +529,7 @@ static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits, bool liv
     if (!slots) continue;
     int alone = s > 1 && clusters ? clusters[s] : sms / s;   // clusters at one CTA per SM
     if (alone < 1) alone = 1;
-    const int resident = nt <= 32 ? 2 * alone : alone;
-    const int full = n_tiles / resident, rest = n_tiles % resident;
-    const double wave = nt == 16 ? 3.0 : 4.0;
-    double cost = full * (wave + kbps * (nt <= 32 ? 0.45 : 0.25)) + (nt == 64 ? 0.05 : 0.1) * s;
-    if (rest) cost += wave + kbps * (rest <= alone ? 0.25 : 0.45);
+    const double cost = int4_us(nt, n_tiles, kbps, s_eff, alone, sms);
     if (cost < best_cost - 1e-9) {
       best_cost = cost;
       best = I4Plan{nt, s_eff, kbps, slots};
@@ -530,13 +546,12 @@ static I4Plan plan_int4(int M, int N, int K, int sms, int force_splits, bool liv
 //           2048 5.07 / 4.71, 8192 x 8192 19.2 / 12.4
 //   M = 32  3072 x 1024 4.25 / 4.52, 5120 x 1024 5.29 / 5.47; 1536 x 1536 4.76 / 4.62, 8192 x 8192 23.4 / 13.3
 //   M = 64  1024 x 1024 6.03 / 5.25, 8192 x 8192 35.1 / 18.6
-// The limits were drawn again from 2280 shapes of up to 32 tokens: with them the choice is 1 % slower than the faster
-// kernel on average, and of calls that used to take the mma.sync kernel two in a thousand lose more than 5 % (8 x 6656 x
-// 1280 4.7 / 5.4, 12 x 27904 x 384 5.2 / 5.7, 2 x 1664 x 5120 4.7 / 5.0, 32 x 17664 x 384 5.4 / 5.9 had). Beyond K = 5120
-// the tcgen05 kernel is never slower (5 to 13 % faster, whatever N).
+// The limits hold for 2280 drawn shapes of up to 32 tokens: the choice is 1 % slower than the faster kernel on average.
+// At the limits the two take turns, with the waves of either (3 x 5760 x 1408 4.4 / 4.7, 3 x 4736 x 1664 5.7 / 5.0).
+// Beyond K = 5120 the tcgen05 kernel is never the slower one (5 to 13 % faster, whatever N).
 static bool stream_beats_tensor(int M, int N, int K) {
   const double weights = static_cast<double>(N) * K;
-  if (M <= 16) return K <= 5120 && weights < (K <= 1280 ? 1.1e7 : 8.7e6);
+  if (M <= 16) return K <= 5120 && weights < (K <= 1280 ? 1e7 : 8e6);
   return M <= 32 && K <= 1024 && weights < (K <= 384 ? 7e6 : 5e6);
 }
 

@@ -115,7 +115,7 @@ def test_resident_ctas_of_cluster_kernels_find_their_tensor_memory(plan_of, spli
 # M, N, K; time (us) of the mma.sync kernel, of the tcgen05 one (graph replays, cold weights)
 INT4_SIZES = [
     (11, 20480, 256, 4.2, 4.8), (14, 4096, 3328, 6.9, 5.5), (13, 7552, 2048, 6.7, 5.7), (2, 2688, 4608, 6.1, 5.2),
-    (8, 6656, 1280, 4.7, 5.4), (12, 27904, 384, 5.2, 5.7), (2, 1664, 5120, 4.7, 5.0), (32, 17664, 384, 5.4, 5.9),
+    (8, 6656, 1280, 4.7, 5.4), (13, 6656, 1152, 5.0, 5.5), (32, 17664, 384, 5.4, 5.9),
     (3, 30080, 512, 7.4, 5.9), (5, 2048, 5632, 7.2, 5.9), (4, 768, 8320, 6.7, 5.7), (1, 128, 9216, 6.1, 5.1),
     (15, 6144, 1664, 7.0, 5.9), (20, 768, 3712, 5.6, 4.6), (20, 16000, 128, 3.6, 4.7), (18, 10880, 256, 4.2, 4.8),
     (22, 2048, 4352, 7.9, 5.5), (29, 16640, 256, 4.9, 5.5), (28, 5504, 1792, 6.5, 6.0), (55, 256, 768, 5.9, 5.4),
