@@ -91,6 +91,7 @@ SIGNATURES = {
     "flyb200_int4_repack": (c_int, [c_void_p, c_void_p, c_int32, c_int32, c_void_p, c_void_p, c_void_p]),
     "flyb200_int4_gemm": (c_int, [c_void_p] * 4 + [c_int32] * 3 + [POINTER(GemmCfg), c_void_p]),
     "flyb200_gemm_plan": (c_int, [c_int32] * 4 + [POINTER(GemmCfg), c_int32, POINTER(c_int32)]),
+    "flyb200_moe_plan": (c_int, [c_int32] * 5 + [POINTER(c_int32)]),
     "flyb200_int4_plan": (c_int, [c_int32] * 5 + [POINTER(c_int32)]),
     "flyb200_decode_plan": (c_int, [c_int32] * 5 + [POINTER(c_int32)]),
     "flyb200_int4_tensor_plan": (c_int, [c_int32] * 5 + [POINTER(c_int32)]),

@@ -1619,15 +1619,20 @@ static inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 
 // Time of one K block of a tile (ns), measured on B200: the slope over K of graph replays with cold
 // operands (M = 256, N = 4096: 32 columns 0.19, 64 0.23, 128 0.25, 256 0.46 us) and of full waves
-// (M = 512, N = 4096, K = 7168: 128 columns 0.32, 256 0.50 us). Over 70 shapes with M from 17 to 2200 the width picked with
-// them is within 0.1 % of the fastest on average. The MoE stages use the same figures.
-static double tile_kb_ns(int bn) { return bn == 256 ? 490.0 : bn == 128 ? 295.0 : bn == 64 ? 250.0 : 200.0; }
+// (M = 512, N = 4096, K = 7168: 128 columns 0.32, 256 0.50 us). The MoE stages that fetch their rows in routing order
+// use the same figures; where rows are gathered one by one, 128 columns take longer. Over 448 layers (8 to 256 experts, 4 to
+// 4096 tokens) the width picked is 3.1 % slower than the fastest in stage 1 and 2.1 % in stage 2 in routing order (with
+// 330 for 128 columns 5.2 and 2.3), 3.7 and 2.5 % gathered (with 295 4.7 and 4.8: 77 blocks, H = 1920 and I = 256
+// 38 % slower in 128 columns than in 256). The number of blocks is an upper bound, which is what these miss.
+static double tile_kb_ns(int bn, bool gathered = false) {
+  return bn == 256 ? 490.0 : bn == 128 ? (gathered ? 330.0 : 295.0) : bn == 64 ? 250.0 : 200.0;
+}
 
 // Tile-width heuristic (role of select_tile_config in the reference's test). Cost model per K block
 // of one tile: tile_kb_ns on the tensor-core side; the memory side costs the tile's weight bytes at one
 // SM's share of HBM bandwidth when few row blocks share them. The persistent loop runs
 // ceil(tiles / SMs) rounds; pick the width with the smallest total.
-static int pick_block_n(int m_blocks, int n_cols, int sms, bool moe1) {
+static int pick_block_n(int m_blocks, int n_cols, int sms, bool moe1, bool gathered = false) {
   const int cands[4] = {256, 128, 64, 32};
   int best = 128;
   double best_cost = 1e30;
@@ -1637,7 +1642,7 @@ static int pick_block_n(int m_blocks, int n_cols, int sms, bool moe1) {
     const int cols = moe1 ? bn / 2 : bn;
     const long tiles = static_cast<long>(m_blocks) * cdiv(n_cols, cols);
     const long rounds = (tiles + sms - 1) / sms;
-    const double compute_ns = tile_kb_ns(bn);
+    const double compute_ns = tile_kb_ns(bn, gathered);
     // weight tile bytes per K block over ~44 GB/s per SM; row blocks that run concurrently on the
     // same weight tile share one HBM read through L2
     const int sharing = m_blocks < 8 ? (m_blocks < 1 ? 1 : m_blocks) : 8;
@@ -2116,6 +2121,19 @@ static bool moe_swap_pays_off(const flyb200_gemm_cfg* cfg, const GemmParams& p) 
   return p.a_sorted && p.tile_m <= 32 && !cfg->block_n && (p.tile_m <= 16 || p.num_blocks <= kMoeSwapListed);
 }
 
+static int moe_block_n(int stage, int n, int num_blocks, bool a_sorted, int sms) {
+  return pick_block_n(num_blocks, n, sms, stage == 1, !a_sorted);
+}
+
+extern "C" int flyb200_moe_plan(int32_t stage, int32_t n, int32_t num_blocks, int32_t a_sorted, int32_t sms,
+                                int32_t* block_n) {
+  if (!block_n || (stage != 1 && stage != 2) || n < 128 || num_blocks < 1)
+    return set_error(FLYB200_ERR_INVALID_ARGUMENT, "moe_plan: bad arguments");
+  if (sms <= 0 && (sms = sm_count()) <= 0) return FLYB200_ERR_CUDA;
+  *block_n = moe_block_n(stage, n, num_blocks, a_sorted != 0, sms);
+  return FLYB200_OK;
+}
+
 static int moe_gemm1_impl(void* out, void* out_q, float* out_scale_t, const void* x, const void* w_repacked,
                           const float* scale_x, const float* scale_w, const int32_t* sorted_ids,
                           const int32_t* expert_ids, const float* sorted_weights,
@@ -2134,7 +2152,7 @@ static int moe_gemm1_impl(void* out, void* out_q, float* out_scale_t, const void
   if (num_blocks == 0) return FLYB200_OK;
   const int sms = sm_count();
   if (sms <= 0) return FLYB200_ERR_CUDA;
-  int bn = (cfg && cfg->block_n) ? cfg->block_n : pick_block_n(num_blocks, I, sms, true);
+  int bn = (cfg && cfg->block_n) ? cfg->block_n : moe_block_n(1, I, num_blocks, cfg && (cfg->path & 1), sms);
   if (bn < 64) return set_error(FLYB200_ERR_INVALID_ARGUMENT, "stage-1 block_n must be >= 64");
   if (pertoken) bn = 256;
   if (out_q) {
@@ -2223,7 +2241,7 @@ static int moe_gemm2_impl(void* out, const void* a2, const void* w_repacked,
   if (num_blocks == 0) return FLYB200_OK;
   const int sms = sm_count();
   if (sms <= 0) return FLYB200_ERR_CUDA;
-  int bn = (cfg && cfg->block_n) ? cfg->block_n : pick_block_n(num_blocks, H, sms, false);
+  int bn = (cfg && cfg->block_n) ? cfg->block_n : moe_block_n(2, H, num_blocks, cfg && (cfg->path & 1), sms);
   if (pertoken) bn = 256;
   int grid = sms;
   if (cfg && cfg->max_ctas > 0 && cfg->max_ctas < grid) grid = cfg->max_ctas;

@@ -100,6 +100,10 @@ int flyb200_pertoken_gemm(void* c, const void* a, const void* b_repacked, const 
 int flyb200_gemm_plan(int32_t pertoken, int32_t M, int32_t N, int32_t K, const flyb200_gemm_cfg* cfg, int32_t sms,
                       int32_t* plan);
 
+/* The tile width that a block-scale MoE stage (1 or 2) takes for n output channels (stage 1: I, stage 2: H) and up to
+ * num_blocks routing blocks on its tiled kernel, with activations in routing order (a_sorted) or gathered. Host only. */
+int flyb200_moe_plan(int32_t stage, int32_t n, int32_t num_blocks, int32_t a_sorted, int32_t sms, int32_t* block_n);
+
 /* MoE routing sort. Bit-exact stand-in for moe_sorting_torch_native
  * (tests/kernels/test_moe_gemm.py:97-161) and the sorter half of build_routing_buffers (:223-295).
  * topk_ids i32 [T,k]; topk_weights f32 [T,k]; expert_mask i32 [E] or NULL; num_local_tokens: < 0

@@ -229,6 +229,23 @@ def test_moe_more_blocks_than_the_kernel_lists():
     assert narrow._small_pays_off(100000)
 
 
+# stage, routing order, blocks, output channels; time (us) in 128- and in 256-wide tiles
+MOE_WIDTHS = [
+    (1, 0, 50, 384, 24.5, 19.4), (1, 0, 67, 384, 23.5, 19.9), (1, 0, 38, 512, 11.9, 9.9), (1, 1, 69, 384, 26.8, 31.6),
+    (1, 1, 37, 768, 44.0, 50.5), (1, 1, 33, 1920, 30.9, 26.9), (2, 0, 68, 3840, 34.5, 24.1), (2, 0, 25, 2176, 8.6, 6.8),
+    (2, 0, 38, 1024, 9.1, 7.1), (2, 1, 9, 4736, 14.3, 19.0), (2, 1, 34, 5760, 33.0, 26.8), (2, 1, 72, 1536, 17.1, 13.0)
+]
+
+
+@pytest.mark.parametrize("stage,a_sorted,blocks,n,us_128,us_256", MOE_WIDTHS)
+def test_moe_stage_takes_the_width_that_measured_faster(stage, a_sorted, blocks, n, us_128, us_256):
+    from flydsl_b200 import _lib
+
+    width = ctypes.c_int32(0)
+    _lib.check(_lib.load().flyb200_moe_plan(stage, n, blocks, a_sorted, SMS, width))
+    assert width.value == (128 if us_128 < us_256 else 256)
+
+
 @pytest.mark.parametrize("mode", ["reduce", "atomic"])
 @pytest.mark.parametrize("tile_m", [8, 16, 32])
 def test_moe_layer_scratch_is_bounded_over_token_counts(tile_m, mode):
