@@ -325,18 +325,33 @@ def dense_check(w, c, world):
             "against": "CPU oracle, every rank its column shard; worst over ranks"}
 
 
-def profile_traffic(name):
+def dense_kernel(M, N, K, sms=0):
+    """Name of the kernel that the dense block-scale GEMM launches for a problem (on this GPU, or one of ``sms`` SMs)."""
+    import ctypes
+
+    from flydsl_b200 import _lib
+
+    plan = (ctypes.c_int32 * 5)()
+    _lib.check(_lib.load().flyb200_gemm_plan(0, M, N, K, ctypes.byref(_lib.GemmCfg(0, 0, 0, 0)), sms, plan))
+    return {1: "bs_gemm_kernel", 2: "bs_gemm_decode_kernel", 3: "bs_pair_kernel"}[plan[0]]
+
+
+def profile_traffic(name, kernel):
     """`traffic_bytes_per_launch` recorded in a committed ncu summary under profiles/ (dram bytes read
-    + written by one launch of the kernel), or None. The number is a property of the kernel and the
+    + written by one launch), or None if there is none for ``kernel``. The number is a property of the kernel and the
     shape, captured once under ncu; it is not measured by this run."""
     path = os.path.join(ROOT, "profiles", name)
+    found = {}
     try:
         for line in open(path):
-            if line.strip().startswith("traffic_bytes_per_launch:"):
-                return float(line.split(":", 1)[1].split()[0])
+            key, _, value = line.strip().partition(":")
+            if key in ("traffic_kernel", "traffic_bytes_per_launch"):
+                found[key] = value.split()[0]
     except OSError:
         pass
-    return None
+    if found.get("traffic_kernel") != kernel or "traffic_bytes_per_launch" not in found:
+        return None
+    return float(found["traffic_bytes_per_launch"])
 
 
 def dense_sweep(dev, peaks, quick=False):
@@ -925,6 +940,8 @@ def run_ours(args):
 
     fp8_peak = 2.0 * peaks["bf16_tflops"]
     per_gpu_tflops = value / world
+    profile = f"bs_gemm_dense_M{M}_N{N}_K{K}.md"
+    traffic = profile_traffic(profile, dense_kernel(M, N, K)) if world == 1 else None
     out = {
         "metric": METRIC, "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "strong",
@@ -946,10 +963,10 @@ def run_ours(args):
         "gpu_launches": args.steps,
         "roofline": {"bound": "tensor", "achieved": per_gpu_tflops, "peak": fp8_peak, "unit": "TFLOP/s",
                      "frac": per_gpu_tflops / fp8_peak,
-                     # dram__bytes_read.sum + dram__bytes_write.sum of one launch of this kernel at N=1,
-                     # read from the committed ncu summary (not measured by this run)
-                     "traffic": profile_traffic(f"bs_gemm_dense_M{M}_N{N}_K{K}.md") if world == 1 else None,
-                     "traffic_source": f"profiles/bs_gemm_dense_M{M}_N{N}_K{K}.md" if world == 1 else None,
+                     # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the kernel that this call takes at
+                     # N=1, read from the committed ncu summary (not measured by this run)
+                     "traffic": traffic,
+                     "traffic_source": f"profiles/{profile}" if traffic is not None else None,
                      "peak_source": f"2 x bf16_tflops ({peaks['source']}); dense FP8 rate is twice bf16",
                      "frac_of_nominal_4500": per_gpu_tflops / 4500.0},
         "clocks": clk.summary(),
