@@ -4,7 +4,8 @@ Plays the part of the reference's autotuner (python/flydsl/autotune.py:91-268: b
 configurations per key, keep the best, persist it as JSON) and of ``select_tile_config`` in its
 dense test. A configuration here is what the C ABI's ``flyb200_gemm_cfg`` exposes: MMA width
 ``block_n``, kernel ``path`` (tiled / decode) and ``split_k``. The key is the shape with M rounded
-up to a power-of-two bucket, the output type and the device name.
+up to a power-of-two bucket, the output type, the device name and the library (a choice among the kernels of
+one build says nothing about those of another).
 
     tuner = GemmAutotuner()                       # cache: $FLYB200_AUTOTUNE_CACHE_DIR or ~/.flyb200
     fn = tuner.tuned_gemm(M=4096, N=7168, K=2048) # benchmarks once per key, then reads the cache
@@ -12,6 +13,8 @@ up to a power-of-two bucket, the output type and the device name.
 """
 from __future__ import annotations
 
+import functools
+import hashlib
 import json
 import os
 from pathlib import Path
@@ -62,6 +65,22 @@ def do_bench(fn: Callable[[], None], warmup: int = 5, rep: int = 25, flush=None)
     return times[len(times) // 2]
 
 
+@functools.lru_cache(maxsize=8)
+def _file_hash(path: str) -> str:
+    with open(path, "rb") as f:
+        return hashlib.file_digest(f, "sha256").hexdigest()[:12]
+
+
+def library_id() -> str:
+    """Which build of the CUDA library a timing belongs to: a hash of the file that is loaded."""
+    from . import _lib
+
+    try:
+        return _file_hash(_lib.LIB_PATH)
+    except OSError:
+        return "nolibrary"
+
+
 def m_bucket(m: int) -> int:
     """Power-of-two bucket of the row count (1, 2, 4, ... ): shapes in a bucket share a configuration."""
     b = 1
@@ -101,6 +120,8 @@ class GemmAutotuner:
         except (OSError, ValueError):
             return
         for key, d in raw.items():
+            if key.count("|") < 5:
+                continue                      # an entry from before keys named the library
             try:
                 self.cache[key] = Config.from_dict(d)
             except (TypeError, AttributeError):
@@ -122,7 +143,7 @@ class GemmAutotuner:
 
             name = torch.cuda.get_device_name() if torch.cuda.is_available() else "nodevice"
             self._device_name = name
-        return f"{name}|m{m_bucket(M)}|n{N}|k{K}|{out_dtype}"
+        return f"{name}|{library_id()}|m{m_bucket(M)}|n{N}|k{K}|{out_dtype}"
 
     # ---- tuning ----
     def tune(self, M: int, N: int, K: int, out_dtype: str = "bf16",

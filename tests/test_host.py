@@ -111,6 +111,28 @@ def test_autotuner_keys_cache_and_persistence(tmp_path):
     assert all(c.path != "decode" for c in default_configs(4096, 7168, 2048))
 
 
+def test_autotuner_tunes_again_for_another_library(tmp_path, monkeypatch):
+    """A choice among the kernels of one build is not taken over by another one, nor one that names no build."""
+    import json
+
+    from flydsl_b200 import autotune
+
+    def tune(shape=(4096, 7168, 2048)):
+        timed = []
+        t = autotune.GemmAutotuner(cache_dir=str(tmp_path), device_name="fake",
+                                   do_bench_fn=lambda call, warmup, rep: call())
+        t.tune(*shape, make_call=lambda cfg: timed.append(cfg) or (lambda: 1.0 + len(timed)))
+        return len(timed)
+
+    old = {"fake|m4096|n7168|k2048|bf16": {"block_n": 256, "path": "tiled", "split_k": None}}
+    (tmp_path / "blockscale_gemm.json").write_text(json.dumps(old))
+    assert tune() > 1 and tune() == 0            # timed although an entry without a library is there; then cached
+    monkeypatch.setattr(autotune, "library_id", lambda: "another")
+    assert tune() > 1 and tune() == 0
+    monkeypatch.undo()
+    assert tune() == 0                           # the first build's entry is still its own
+
+
 def test_c_abi_refuses_bad_sizes_before_any_launch():
     """Argument checks that protect vector accesses run on the host before anything is launched, so
     they can be exercised without a GPU: a non-NULL dummy pointer is enough."""
