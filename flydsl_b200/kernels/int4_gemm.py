@@ -36,7 +36,7 @@ def pack_int4_weight(q: torch.Tensor, scales: torch.Tensor) -> Tuple[torch.Tenso
     """int8 values ``[N, K]`` in [-8, 7] + bf16 scales ``[N, K/128]`` -> the kernel's layout:
     packed uint8 ``[K/128, N/8, 4, 8, 16]`` (per group and block of 8 rows: four 16-byte chunks, each
     holding its 8 rows back to back) and scales bf16 ``[K/128, N]`` (CUDA). ``N % 8 == 0``."""
-    if not q.is_cuda:
+    if not (q.is_cuda and scales.is_cuda):
         raise ValueError("pack_int4_weight needs CUDA tensors (this library has no CPU path)")
     N, K = q.shape
     if q.dtype != torch.int8 or K % GROUP or N % 8 or tuple(scales.shape) != (N, K // GROUP):
@@ -58,8 +58,9 @@ class Int4GemmLauncher:
     def __init__(self, N: int, K: int, split_k: Optional[int], path: str = "auto"):
         if path not in ("auto", "stream", "tensor"):
             raise ValueError("path must be 'auto', 'stream' (mma.sync, weights unpacked in registers) or "
-                             "'tensor' (tcgen05, weights unpacked through shared memory)")
+                             "'tensor' (tcgen05, weights unpacked into tensor memory)")
         self.N, self.K = int(N), int(K)
+        self._wq_bytes, self._scales = self.K // GROUP * self.N * (GROUP // 2), self.K // GROUP * self.N
         self._cfg = _lib.GemmCfg(0, 0, {"auto": 0, "stream": 1, "tensor": 2}[path], int(split_k or 0))
         self._fn = _lib.load().flyb200_int4_gemm
 
@@ -70,8 +71,14 @@ class Int4GemmLauncher:
             raise ValueError("int4 GEMM takes bf16 activations and writes bf16")
         if tuple(a.shape) != (int(m), self.K) or tuple(c.shape) != (int(m), self.N):
             raise ValueError(f"expected a [{m}, {self.K}] and c [{m}, {self.N}]")
+        if wq.element_size() * wq.numel() < self._wq_bytes or not wq.is_contiguous():
+            raise ValueError(f"wq must be the {self._wq_bytes} packed bytes of pack_int4_weight, contiguous")
+        if scales_t.dtype != torch.bfloat16 or scales_t.numel() < self._scales or not scales_t.is_contiguous():
+            raise ValueError(f"scales_t must be bf16 [{self.K // GROUP}, {self.N}] of pack_int4_weight, contiguous")
         if not (a.is_contiguous() and c.is_contiguous()):
             raise ValueError("a and c must be contiguous")
+        if not (a.is_cuda and c.is_cuda and wq.is_cuda and scales_t.is_cuda):
+            raise ValueError("int4 GEMM takes CUDA tensors (this library has no CPU path)")
         _lib.check(self._fn(c.data_ptr(), a.data_ptr(), wq.data_ptr(), scales_t.data_ptr(), int(m), self.N,
                             self.K, ctypes.byref(self._cfg), _lib.stream_handle(stream)))
 
