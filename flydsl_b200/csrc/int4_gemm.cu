@@ -9,9 +9,9 @@
 //   * two sets of four dequantiser warps, each taking every other group. A thread owns a weight row (= TMEM lane):
 //     it reads the row's 64 packed bytes, turns them into EXACT bf16 values q / 4 and writes them with tcgen05.st
 //     where tcgen05.mma takes its A operand from: tensor memory. The weights never go back to shared memory
-//     (the image there is four times the packed bytes, written and read again). The integer pipe bounds
-//     this, so it gets 2.25 instructions per two weights, one of them on the FMA pipe: nibble n = q + 8 in the low
-//     bits, (n | 0x4300) is bf16 128 + n, times 1/4 minus 34 gives q / 4; n in bits 4-7 is the bf16 number n 2^-129
+//     (the image there is four times the packed bytes, written and read again). The unpacking takes 2.25
+//     instructions per two weights, one of them on the FMA pipe (with 3.25 the integer pipe was 59 % busy and bound the
+//     kernel, 14.6 us at N = K = 8192 and 16 tokens; now 33 % and 12.4 us): nibble n = q + 8 in the low bits, (n | 0x4300) is bf16 128 + n, times 1/4 minus 34 gives q / 4; n in bits 4-7 is the bf16 number n 2^-129
 //     (bits up to 255 are subnormals or have the same spacing), times 2^127 minus 2 gives q / 4 without a shift.
 //   * tcgen05.mma kind::f16 (bf16 x bf16 -> f32), 128 x NT x 16, eight per K group, each group into a
 //     fresh accumulator buffer; the issuing warp stays converged (one elected lane issues).
@@ -21,8 +21,10 @@
 //     in fp32 before scaling.
 //   * split-K over a thread-block cluster with the partials exchanged by bulk copies through
 //     distributed shared memory and summed in rank order (deterministic), as in decode_gemm.cu.
-//   * up to 32 tokens a CTA takes half an SM (448 threads of at most 72 registers, 256 TMEM columns, 113 KB), so
-//     that two share one and hide each other's chain dequantise -> MMA -> completion -> dequantise.
+//   * up to 32 tokens a CTA takes half an SM (448 threads of 64 registers, 256 TMEM columns, 113 KB), so
+//     that two share one and hide each other's chain dequantise -> MMA -> completion -> dequantise. Each set owns one
+//     operand buffer there, and that chain is what a group takes (0.31 us alone, 0.24 with two CTAs): ncu shows no unit
+//     more than half busy (issue slots 44 %, integer pipe 33 %, DRAM 24 %, tensor pipe 7 %).
 //
 // The reference has no kernel for this exact format (its nearest code is the W4A16 path of
 // kernels/moe_gemm_2stage.py:607-630 and the int4 unpack of kernels/mfma_preshuffle_pipeline.py:

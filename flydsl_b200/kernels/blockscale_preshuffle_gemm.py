@@ -59,9 +59,10 @@ def compile_blockscale_preshuffle_gemm(
 
     ``tile_m/tile_n/tile_k`` are validated like the reference does but do not pick the B200 tile
     (the MMA tile is 128 x block_n x 128; ``block_n`` in {32,64,128,256} overrides the built-in
-    heuristic; ``path`` = "auto" | "tiled" | "decode" picks the kernel: M <= 64 defaults to the
-    swap-AB split-K decode kernel, ``split_k`` its cluster size; with ``path="tiled"`` the CTAs that
-    share a tile's K range). ``use_cshuffle_epilog``, ``waves_per_eu`` and ``use_async_copy`` are AMD tuning
+    heuristic; ``path`` = "auto" | "tiled" | "decode" picks the kernel: "auto" takes what is estimated
+    to be fastest for the shape, "decode" is the swap-AB split-K kernel for M <= 64; ``split_k`` is its
+    cluster size, with ``path="tiled"`` the CTAs that share a tile's K range, and with "auto" and M <= 64 it asks for
+    the decode kernel where that runs in one wave). ``use_cshuffle_epilog``, ``waves_per_eu`` and ``use_async_copy`` are AMD tuning
     switches, accepted and ignored.
     """
     if out_dtype not in ("fp16", "bf16"):

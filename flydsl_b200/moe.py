@@ -139,16 +139,21 @@ class BlockscaleMoE:
     def _small_pays_off(self, T: int) -> bool:
         """Whether T tokens in blocks of at most 32 rows take routing-order layouts. The stages gain from
         blocks that follow one another in the same expert (one pass over its weights for two) and, in a
-        steady stream of calls, from the tensor work that is not done for padding; the permute and the
-        re-quantiser of padded rows cost 10 to 30 us. Measured in steady streams, routing order / gathered
-        (us a layer; uniform routing, and with every 16th expert hot):
-          blocks of 16  256 experts of 7168 x 2048, top 8, 32 tokens 1089 / 1105 and 536 / 548, 128 x 4096 x 1536, 64
-                        tokens 394 / 411 and 336 / 363, 8 tokens 182 / 183 and 137 / 124, 256 x 3072 x 1024, top 4, 128
-                        tokens 356 / 350 and 157 / 174, 32 tokens 180 / 174 and 90 / 81, 64 x 2048 x 1024, top 6, 200
-                        tokens 117 / 135 and 125 / 136, 64 tokens 105 / 96 and 102 / 95
-          blocks of 32  256 x 7168 x 2048, 256 tokens 1769 / 1861 and 1658 / 1846, 128 x 4096 x 1536, 256 tokens 443 /
-                        426 and 459 / 507, 512 tokens 463 / 602 and 538 / 611, 256 x 3072 x 1024, 384 tokens 485 /
-                        419 and 357 / 354, 64 x 2048 x 1024, 384 tokens 129 / 144 and 136 / 142
+        steady stream of calls, from the tensor work that is not done for padding; the permute costs 5 to 20 us.
+        Measured in steady streams, routing order / gathered (us a layer; uniform routing, and with every 16th expert
+        hot):
+          blocks of 16  256 experts of 7168 x 2048, top 8, 12 tokens 582 / 708 and 331 / 349, 32 tokens 1087 / 1330 and 543 /
+                        605, 128 x 4096 x 1536, 64 tokens 389 / 424 and 357 / 427, 8 tokens 187 / 187 and 141 / 131, 256 x
+                        3072 x 1024, top 4, 128 tokens 343 / 370 and 158 / 164, 32 tokens 184 / 185 and 93 / 84, 64 x 2048 x
+                        1024, top 6, 200 tokens 116 / 133 and 128 / 134, 128 tokens 109 / 100 and 107 / 115, 64 tokens 124 /
+                        100 and 101 / 99
+          blocks of 32  256 x 7168 x 2048, 64 tokens 1522 / 1818 and 871 / 1014, 256 tokens 1744 / 2078 and 1725 / 2177, 128 x
+                        4096 x 1536, 256 tokens 440 / 454 and 469 / 547, 128 tokens 428 / 442 and 429 / 483, 512 tokens 486 /
+                        683 and 532 / 664, 256 x 3072 x 1024, 384 tokens 441 / 455 and 317 / 341, 64 x 2048 x 1024, 256 tokens
+                        123 / 104 and 123 / 120, 384 tokens 129 / 142 and 145 / 141
+        Over 120 drawn layers the choice is 0.7 % slower than the faster side on average (two of them by more than
+        10 %). Graph replays of the same layers leave the clock higher and move the crossings up: there blocks of 32 with
+        less than a tenth of a block per expert are up to 15 % faster gathered;
         and with more blocks than the kernel lists: see moe_swap_pays_off in blockscale_gemm.cu."""
         routes, rows = T * self.topk, self.E * self.tile_m
         if self.tile_m > 16 and routes + rows - self.topk > 4096 * self.tile_m:

@@ -138,7 +138,7 @@ def _kernel_source(name):
     return re.sub(r"//[^\n]*", "", text)
 
 
-@pytest.mark.parametrize("name", ["blockscale_gemm.cu", "moe_swap.cu", "pt_pair_gemm.cu"])
+@pytest.mark.parametrize("name", ["blockscale_gemm.cu", "moe_swap.cu", "pt_pair_gemm.cu", "bs_pair_gemm.cu"])
 def test_roles_that_may_give_up_meet_at_bounded_barriers_only(name):
     """In these kernels a warp whose bounded wait runs out leaves its loop at once, so nobody may wait for
     it at a named hardware barrier, which has no limit (decode_gemm.cu, int4_gemm.cu and int4_stream.cu send
