@@ -77,13 +77,12 @@ def test_split_k_pertoken(M, N, K):
     assert torch.equal(out[1], out[2])
 
 
-# Decode-size M on both sides of the lines between the decode and the tiled kernel
-@pytest.mark.parametrize("M,N,K,kernel", [(1, 1152, 1024, DECODE), (1, 1536, 1024, TILED), (1, 12288, 256, TILED),
-                                          (1, 19072, 256, DECODE), (8, 12288, 5120, TILED), (16, 2688, 2048, DECODE),
-                                          (16, 3216, 2048, TILED), (16, 12688, 1920, TILED), (17, 1040, 3072, DECODE),
-                                          (17, 7040, 512, TILED), (32, 1552, 2048, DECODE), (32, 2192, 2048, TILED),
-                                          (32, 7168, 4224, TILED), (24, 9600, 2304, TILED), (33, 768, 2048, DECODE),
-                                          (33, 1536, 2048, TILED), (33, 12160, 4096, TILED)])
+# Decode-size M on both sides of the choice between the decode and the tiled kernel
+@pytest.mark.parametrize("M,N,K,kernel", [(1, 528, 1536, DECODE), (1, 2064, 3072, DECODE), (1, 7056, 7168, TILED),
+                                          (8, 2064, 2048, DECODE), (8, 12288, 5120, TILED), (16, 1552, 2048, DECODE),
+                                          (16, 12688, 1920, TILED), (17, 1040, 3072, DECODE), (17, 1552, 2560, DECODE),
+                                          (17, 7040, 512, TILED), (32, 2192, 2048, TILED), (32, 7168, 4224, TILED),
+                                          (24, 9600, 2304, TILED), (33, 1536, 2048, TILED), (33, 12160, 4096, TILED)])
 def test_decode_or_tiled(M, N, K, kernel):
     from flydsl_b200 import _lib
     from flydsl_b200.kernels import compile_blockscale_preshuffle_gemm
