@@ -8,6 +8,7 @@ here is this library's own, produced by :func:`pack_int4_weight`.
 """
 from __future__ import annotations
 
+import ctypes
 import functools
 from typing import Optional, Tuple
 
@@ -62,16 +63,27 @@ class Int4GemmLauncher:
         self.N, self.K = int(N), int(K)
         self._wq_bytes, self._scales = self.K // GROUP * self.N * (GROUP // 2), self.K // GROUP * self.N
         self._cfg = _lib.GemmCfg(0, 0, {"auto": 0, "stream": 1, "tensor": 2}[path], int(split_k or 0))
+        self._cfg_ref = ctypes.byref(self._cfg)
         self._fn = _lib.load().flyb200_int4_gemm
 
     def __call__(self, c, a, wq, scales_t, m, stream=None):
-        import ctypes
+        # Small calls wait for the host: one pass over the attributes, the reasons only where something is wrong.
+        if not (a.dtype is c.dtype is scales_t.dtype is torch.bfloat16 and a.shape == (m, self.K)
+                and c.shape == (m, self.N) and wq.nbytes >= self._wq_bytes and scales_t.numel() >= self._scales
+                and a.is_contiguous() and c.is_contiguous() and wq.is_contiguous() and scales_t.is_contiguous()
+                and a.is_cuda and c.is_cuda and wq.is_cuda and scales_t.is_cuda):
+            self._refuse(c, a, wq, scales_t, int(m))
+        rc = self._fn(c.data_ptr(), a.data_ptr(), wq.data_ptr(), scales_t.data_ptr(), int(m), self.N, self.K,
+                      self._cfg_ref, _lib.stream_handle(stream))
+        if rc:
+            _lib.check(rc)
 
+    def _refuse(self, c, a, wq, scales_t, m):
         if a.dtype != torch.bfloat16 or c.dtype != torch.bfloat16:
             raise ValueError("int4 GEMM takes bf16 activations and writes bf16")
-        if tuple(a.shape) != (int(m), self.K) or tuple(c.shape) != (int(m), self.N):
+        if tuple(a.shape) != (m, self.K) or tuple(c.shape) != (m, self.N):
             raise ValueError(f"expected a [{m}, {self.K}] and c [{m}, {self.N}]")
-        if wq.element_size() * wq.numel() < self._wq_bytes or not wq.is_contiguous():
+        if wq.nbytes < self._wq_bytes or not wq.is_contiguous():
             raise ValueError(f"wq must be the {self._wq_bytes} packed bytes of pack_int4_weight, contiguous")
         if scales_t.dtype != torch.bfloat16 or scales_t.numel() < self._scales or not scales_t.is_contiguous():
             raise ValueError(f"scales_t must be bf16 [{self.K // GROUP}, {self.N}] of pack_int4_weight, contiguous")
@@ -79,8 +91,6 @@ class Int4GemmLauncher:
             raise ValueError("a and c must be contiguous")
         if not (a.is_cuda and c.is_cuda and wq.is_cuda and scales_t.is_cuda):
             raise ValueError("int4 GEMM takes CUDA tensors (this library has no CPU path)")
-        _lib.check(self._fn(c.data_ptr(), a.data_ptr(), wq.data_ptr(), scales_t.data_ptr(), int(m), self.N,
-                            self.K, ctypes.byref(self._cfg), _lib.stream_handle(stream)))
 
 
 @functools.lru_cache(maxsize=256)
