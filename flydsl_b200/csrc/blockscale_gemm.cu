@@ -1760,32 +1760,41 @@ struct TileTimes {
   double bytes;          // the weights, as a multiple of their time at 6.5 TB/s
   double round, busy;    // each further round of tiles; a K block with every SM at work
 };
-static double unsplit_us(int M, int N, int K, int bn, int sms) {
+// What the estimates of a call share. A call evaluates about twenty of them on the host: no divisions in the loops.
+struct TileCall {
+  int m_blocks, rows, kbt, sms;   // row blocks, rows of the first one, K blocks
+  double weights, per_sm;         // the weights' time at 6.5 TB/s; 1 / sms
+  TileCall(int M, int N, int K, int sms_)
+      : m_blocks(cdiv(M, BM)), rows(M < BM ? M : BM), kbt(K / BK), sms(sms_),
+        weights(static_cast<double>(N) * K * (1.0 / 6.5e6)), per_sm(1.0 / sms_) {}
+};
+static double unsplit_us(const TileCall& c, int N, int bn) {
   const TileTimes t = bn == 256 ? TileTimes{3.50, 0.407, 1.12, 0.30, 0.96, 0.060}
                       : bn == 128 ? TileTimes{3.56, 0.197, 0.54, 0.225, 0.97, 0.059}
                       : bn == 64 ? TileTimes{2.78, 0.166, 0.32, 0.185, 0.55, 0.040}
                                  : TileTimes{2.16, 0.163, 0.35, 0.216, 0.37, 0.032};
-  const long tiles = static_cast<long>(cdiv(M, BM)) * cdiv(N, bn);
-  const long rounds = (tiles + sms - 1) / sms;
-  const double fill = tiles < sms ? static_cast<double>(tiles) / sms : 1.0;
-  return t.fixed + (t.block * rounds + t.busy * fill) * (K / BK) + t.rows * (M < BM ? M : BM) / BM +
-         t.bytes * (static_cast<double>(N) * K / 6.5e6) + t.round * (rounds - 1);
+  const int n_tiles = bn == 256 ? (N + 255) >> 8 : bn == 128 ? (N + 127) >> 7 : bn == 64 ? (N + 63) >> 6 : (N + 31) >> 5;
+  const long tiles = static_cast<long>(c.m_blocks) * n_tiles;
+  const long rounds = tiles <= c.sms ? 1 : (tiles + c.sms - 1) / c.sms;
+  const double fill = tiles < c.sms ? tiles * c.per_sm : 1.0;
+  return t.fixed + (t.block * rounds + t.busy * fill) * c.kbt + t.rows * c.rows * (1.0 / BM) + t.bytes * c.weights +
+         t.round * (rounds - 1);
 }
 struct SplitTimes {
   double fixed, block;   // a call with its exchange; a K block
   double kb;             // 1000 bytes that leave a CTA
   double bytes, fill;    // the weights, as above; all SMs taken
 };
-static double split_us(int M, int N, int K, int bn, int splits, int sms) {
-  const SplitTimes t = bn == 256 ? SplitTimes{3.34, 0.382, 0.0561, 0.244, 3.31}
-                       : bn == 128 ? SplitTimes{3.59, 0.2255, 0.0497, 0.245, 2.06}
-                                   : SplitTimes{3.17, 0.2045, 0.0496, 0.102, 1.675};
-  const long ctas = static_cast<long>(cdiv(M, BM)) * cdiv(N, bn) * splits;
-  const double sent = (M < BM ? M : BM) * bn * 4.0 * (splits - 1) / splits / 1000.0;
-  return t.fixed + t.block * cdiv(K / BK, splits) + t.kb * sent + t.bytes * (static_cast<double>(N) * K / 6.5e6) +
-         t.fill * ctas / sms;
+static SplitTimes split_times(int bn) {
+  return bn == 256 ? SplitTimes{3.34, 0.382, 0.0561, 0.244, 3.31}
+         : bn == 128 ? SplitTimes{3.59, 0.2255, 0.0497, 0.245, 2.06}
+                     : SplitTimes{3.17, 0.2045, 0.0496, 0.102, 1.675};
 }
-
+static double split_us(const TileCall& c, const SplitTimes& t, int bn, int tiles, int splits, int kbps) {
+  constexpr double kLeaving[9] = {0.0, 0.0, 1.0 / 2, 2.0 / 3, 3.0 / 4, 4.0 / 5, 5.0 / 6, 6.0 / 7, 7.0 / 8};   // of a partial tile
+  return t.fixed + t.block * kbps + t.kb * (c.rows * bn * 0.004) * kLeaving[splits] + t.bytes * c.weights +
+         t.fill * (tiles * splits) * c.per_sm;
+}
 static double pair_us(int M, int N, int K, int ctas) {   // CTA pairs (bs_pair_gemm.cu)
   const long tiles = static_cast<long>(cdiv(M, 256)) * cdiv(N, 256), pairs = ctas / 2;
   const long rounds = (tiles + pairs - 1) / pairs;
@@ -1800,32 +1809,39 @@ static bool in_fitted_range(int M, int N, int sms) {
 // The tiles of a block-scale call that asked for nothing, and their estimated time. Clusters have to be resident
 // all at once.
 static SplitPlan fastest_tiles(int M, int N, int K, int sms, bool live, double& us) {
-  const int m_blocks = cdiv(M, BM), kbt = K / BK;
+  constexpr double kPer[9] = {0.0, 1.0, 1.0 / 2, 1.0 / 3, 1.0 / 4, 1.0 / 5, 1.0 / 6, 1.0 / 7, 1.0 / 8};
+  const TileCall c(M, N, K, sms);
   if (!in_fitted_range(M, N, sms)) {
-    const int bn = pick_block_n(m_blocks, N, sms, false);
-    us = unsplit_us(M, N, K, bn, sms);
-    return SplitPlan{bn, 1, kbt};
+    const int bn = pick_block_n(c.m_blocks, N, sms, false);
+    us = unsplit_us(c, N, bn);
+    return SplitPlan{bn, 1, c.kbt};
   }
-  SplitPlan best{0, 1, kbt};
+  SplitPlan best{0, 1, c.kbt};
   us = 1e30;
   for (int bn = 32; bn <= 256; bn *= 2) {
-    const double t = unsplit_us(M, N, K, bn, sms);
+    const double t = unsplit_us(c, N, bn);
     if (t < us) {
       us = t;
       best.bn = bn;
     }
   }
-  if (us <= 3.4) return best;   // no split is estimated below that
-  const int* clusters = live ? max_clusters() : nullptr;
+  const int* clusters = nullptr;   // asked for where it matters: 50 ns of a call
   for (int bn = 64; bn <= 256; bn *= 2) {
-    const long tiles = static_cast<long>(m_blocks) * cdiv(N, bn);
-    for (int sp = 2; sp <= (bn == 256 ? 4 : 8) && tiles * sp <= sms; ++sp) {
-      const int kbps = cdiv(kbt, sp);
-      if (cdiv(kbt, kbps) != sp) continue;   // some CTA would have no K block
-      if (tiles > (clusters ? clusters[sp] : sms / sp)) continue;
-      const double t = split_us(M, N, K, bn, sp, sms);
-      if (t < us) {
-        us = t;
+    const int tiles = c.m_blocks * (bn == 256 ? (N + 255) >> 8 : bn == 128 ? (N + 127) >> 7 : (N + 63) >> 6);
+    const int most = bn == 256 ? 4 : 8;
+    const SplitTimes t = split_times(bn);
+    // no cluster size of this width can win: the fewest K blocks, the least exchanged, two CTAs per tile
+    if (t.fixed + t.block * (bn == 256 ? (c.kbt + 3) >> 2 : (c.kbt + 7) >> 3) + t.kb * (c.rows * bn * 0.002) +
+            t.bytes * c.weights + t.fill * (2 * tiles) * c.per_sm >= us)
+      continue;
+    for (int sp = 2; sp <= most && tiles * sp <= sms; ++sp) {
+      const int kbps = static_cast<int>((c.kbt + sp - 1) * kPer[sp] + 1e-6);   // cdiv(kbt, sp)
+      if ((sp - 1) * kbps >= c.kbt) continue;   // some CTA would have no K block
+      const double s = split_us(c, t, bn, tiles, sp, kbps);
+      if (s < us) {
+        if (live && !clusters) clusters = max_clusters();
+        if (clusters && tiles > clusters[sp]) continue;   // (not live: tiles * sp <= sms)
+        us = s;
         best = SplitPlan{bn, sp, kbps};
       }
     }
@@ -1845,7 +1861,7 @@ int launch_decode_gemm(void* c, const void* a, const void* b_repacked, const flo
                        const float* scale_b, int M, int N, int K, int out_dtype, int force_splits,
                        cudaStream_t stream, bool pertoken);
 bool decode_path_pays_off(int M, int N, int K, int sms);
-double decode_us(int M, int N, int K, int sms);
+double decode_us(int M, int N, int K, int sms, double limit);
 // moe_swap.cu
 int launch_moe_swap(int stage, bool pertoken, void* out, const void* act, const void* w_repacked,
                     const float* scale_x, const float* scale_w, const int32_t* sorted_ids, const int32_t* expert_ids,
@@ -1934,7 +1950,7 @@ static DensePlan plan_dense(bool pertoken, int M, int N, int K, const flyb200_ge
   // Decode-size M: the swap-AB split-K kernel (decode_gemm.cu; per-token: the token's scale on every K
   // block, the channel's once). It is the one that a cluster size or a limit on the CTAs is meant for.
   if (path == 2 || (path == 0 && M <= 64 && !block_n &&
-                    (any ? decode_us(M, N, K, sms) < us : decode_path_pays_off(M, N, K, sms)))) {
+                    (any ? decode_us(M, N, K, sms, us) < us : decode_path_pays_off(M, N, K, sms)))) {
     plan.kernel = 2;
     return plan;
   }
@@ -1954,11 +1970,12 @@ static DensePlan plan_dense(bool pertoken, int M, int N, int K, const flyb200_ge
   }
   plan.splits = split.splits;
   plan.kbps = split.kbps;
-  const int wide = pertoken || block_n ? 0 : pick_block_n(m_blocks, N, sms, false);   // of many tiles
+  // the width for many tiles (a row block on its own is never one for pairs, see pair_beats_tiled)
+  const int wide = pertoken || block_n || (any && m_blocks == 1) ? 0 : pick_block_n(m_blocks, N, sms, false);
   plan.bn = pertoken ? 256 : block_n ? block_n : any || split.splits > 1 ? split.bn : wide;
   const long tiles = static_cast<long>(m_blocks) * cdiv(N, plan.bn);
   plan.grid = max_ctas > 0 && max_ctas < sms ? max_ctas : sms;
-  if (!pertoken && path == 0 && !block_n && !split_k && plan.grid >= 2) {
+  if (wide && path == 0 && !split_k && plan.grid >= 2) {
     const long wide_tiles = static_cast<long>(m_blocks) * cdiv(N, wide);
     if (pair_beats_tiled(M, N, K / BK, plan.grid, ((wide_tiles + plan.grid - 1) / plan.grid) * tile_kb_ns(wide)) &&
         !(any && in_fitted_range(M, N, sms) && us < pair_us(M, N, K, plan.grid))) {

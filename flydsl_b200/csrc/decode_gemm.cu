@@ -360,12 +360,13 @@ static DecodePlan plan_decode(int M, int N, int K, int sms, int force_splits) {
   const int n_tiles = (N + 127) / 128;
   const int KBt = K / 128;
   const int stage_bytes = kWTileBytes + nt * 128;
+  constexpr double kPer[9] = {0.0, 1.0, 1.0 / 2, 1.0 / 3, 1.0 / 4, 1.0 / 5, 1.0 / 6, 1.0 / 7, 1.0 / 8};
   double best_cost = 1e30;
   for (int s = 1; s <= 8; ++s) {
     if (force_splits > 0 && s != force_splits) continue;
-    const int kbps = (KBt + s - 1) / s;
-    const int s_eff = (KBt + kbps - 1) / kbps;
-    if (s_eff != s && force_splits <= 0) continue;  // same plan as a smaller s
+    const int kbps = static_cast<int>((KBt + s - 1) * kPer[s] + 1e-6);   // ceil(KBt / s); a division takes longer
+    if ((s - 1) * kbps >= KBt && force_splits <= 0) continue;   // same plan as a smaller s
+    const int s_eff = force_splits > 0 ? (KBt + kbps - 1) / kbps : s;
     int stages = kbps < kDecMaxStages ? kbps : kDecMaxStages;
     if (stages < 2) stages = 2;  // the stage area doubles as the send buffer of the exchange
     const int fixed = kbps * (nt + 1) * 4 + 64 + 2048;
@@ -376,17 +377,14 @@ static DecodePlan plan_decode(int M, int N, int K, int sms, int force_splits) {
     while (stages > 2 && stages * stage_bytes + fixed > 232448) --stages;
     const int ring = stages * stage_bytes > exchange ? stages * stage_bytes : exchange;
     const int smem = ring + fixed;
-    if (smem > 232448) continue;
-    int cps = 232448 / (smem + 1024);
-    const int tmem_cols = nt * 4 < 32 ? 32 : nt * 4;
-    if (cps > 512 / tmem_cols) cps = 512 / tmem_cols;
-    if (cps > 4) cps = 4;
-    if (cps < 1) continue;
+    if (smem + 1024 > 232448) continue;
+    int cps = 4 * (smem + 1024) <= 232448 ? 4 : 3 * (smem + 1024) <= 232448 ? 3 : 2 * (smem + 1024) <= 232448 ? 2 : 1;
+    if (cps > 128 / nt) cps = 128 / nt;   // 4 nt of the 512 columns of tensor memory each
     const long ctas = static_cast<long>(n_tiles) * s_eff;
     // the K split is chosen as if two CTAs shared an SM (more splits only lengthen the exchange);
     // the rest of the SM is left to the next launch
     const long slots = static_cast<long>(sms) * (cps > 2 ? 2 : cps);
-    const long rounds = (ctas + slots - 1) / slots;
+    const long rounds = ctas <= slots ? 1 : (ctas + slots - 1) / slots;
     // a round costs the MMA-issue time of its K blocks (~0.2 us each; two co-resident CTAs share
     // the SM) plus a fixed ~1 us (fill latency, reduction, store)
     const double cost = rounds * (kbps * 0.2 * (cps > 1 && ctas > sms ? 1.5 : 1.0) + 1.0);
@@ -445,19 +443,24 @@ bool decode_path_pays_off(int M, int N, int K, int sms) {
 // Estimated time (us) of a block-scale call on this kernel, where its CTAs are resident at once: the counterpart of
 // the tiled kernel's estimates in blockscale_gemm.cu, fitted to the same shapes (2700 of them where this kernel is
 // within a quarter of the fastest; 4 % off on average, 15 % at most).
-double decode_us(int M, int N, int K, int sms) {
+// At least `limit` where it cannot be below that: then there is no plan to look for.
+double decode_us(int M, int N, int K, int sms, double limit) {
+  struct Times {
+    double fixed, block, rows, bytes, fill, wide;   // rows: all token columns used; wide: clusters of seven and eight
+  };
   if (M > 64) return 1e30;
+  const Times t = M <= 16 ? Times{2.51, 0.436, 0.33, 0.71, 0.58, 0.19}
+                  : M <= 32 ? Times{2.46, 0.455, 0.64, 0.73, 0.79, 0.15}
+                            : Times{2.54, 0.463, 1.52, 0.91, 0.86, 0.09};
+  const double weights = static_cast<double>(N) * K * (1.0 / 6.5e6);   // their time at 6.5 TB/s
+  const int n_tiles = (N + 127) / 128, kbt = K / 128;
+  const double least = t.fixed + t.rows * M * (M <= 16 ? 1.0 / 16 : M <= 32 ? 1.0 / 32 : 1.0 / 64) + t.bytes * weights;
+  const double per_sm = t.fill / sms;
+  if (least + t.block * ((kbt + 7) >> 3) + per_sm * n_tiles >= limit) return limit;
   const DecodePlan plan = plan_decode(M, N, K, sms, 0);
   if (plan.splits < 1 || plan.rounds != 1) return 1e30;
-  const double ctas = static_cast<double>((N + 127) / 128) * plan.splits;
-  const double weights = static_cast<double>(N) * K / 6.5e6;   // their time at 6.5 TB/s
-  const double full = static_cast<double>(M) / plan.nt;
-  const double wide = plan.splits > 6 ? 1.0 : 0.0;             // fewer clusters of seven and eight fit the GPU
-  switch (plan.nt) {
-    case 16: return 2.51 + 0.436 * plan.kbps + 0.33 * full + 0.71 * weights + 0.58 * ctas / sms + 0.19 * wide;
-    case 32: return 2.46 + 0.455 * plan.kbps + 0.64 * full + 0.73 * weights + 0.79 * ctas / sms + 0.15 * wide;
-    default: return 2.54 + 0.463 * plan.kbps + 1.52 * full + 0.91 * weights + 0.86 * ctas / sms + 0.09 * wide;
-  }
+  return least + t.block * plan.kbps + per_sm * (static_cast<double>(n_tiles) * plan.splits) +
+         (plan.splits > 6 ? t.wide : 0.0);   // fewer clusters of seven and eight fit the GPU
 }
 
 }  // namespace flyb200
